@@ -331,6 +331,25 @@ gr_status NbSystem::upload(const gr_topology* t) {
     std::vector<int> atom_cg(N);
     for (int c = 0; c < NCG; ++c)
         for (int a = h_cg_off[c]; a < h_cg_off[c + 1]; ++a) atom_cg[a] = c;
+    // solute CG pairs that share an excluded or 1-4 atom pair, both directions
+    std::vector<std::pair<int, int>> xp;
+    for (int a = 0; a < NSA; ++a) {
+        auto link = [&](int b) {
+            if (b < 0 || b >= NSA || atom_cg[b] == atom_cg[a]) return;
+            xp.push_back({atom_cg[a], atom_cg[b]});
+            xp.push_back({atom_cg[b], atom_cg[a]});
+        };
+        for (int k = h_excl_off[a]; k < h_excl_off[a + 1]; ++k) link(h_excl[k]);
+        for (int k = h_o14_off[a]; k < h_o14_off[a + 1]; ++k) link(h_o14[k]);
+    }
+    std::sort(xp.begin(), xp.end());
+    xp.erase(std::unique(xp.begin(), xp.end()), xp.end());
+    std::vector<int> cgx_off(size_t(NSCG) + 1, 0), cgx;
+    for (const auto& p : xp) {
+        ++cgx_off[size_t(p.first) + 1];
+        cgx.push_back(p.second);
+    }
+    for (int c = 0; c < NSCG; ++c) cgx_off[size_t(c) + 1] += cgx_off[size_t(c)];
     // perturbation
     std::vector<int> pidx(N, -1), piac, pp;
     std::vector<double> pq, palpha;
@@ -368,7 +387,7 @@ gr_status NbSystem::upload(const gr_topology* t) {
     double* lj64 = nullptr;
     float2* lj32d = nullptr;
     int *excl_off = nullptr, *excl = nullptr, *o14_off = nullptr, *o14 = nullptr, *eg = nullptr, *acg = nullptr;
-    int *pidx_d = nullptr, *piac_d = nullptr, *pp_d = nullptr;
+    int *pidx_d = nullptr, *piac_d = nullptr, *pp_d = nullptr, *cgxo_d = nullptr, *cgx_d = nullptr;
     double *pq_d = nullptr, *pa_d = nullptr;
     if ((st = upload_array(&cg_off, h_cg_off.data(), h_cg_off.size()))) return st;
     if ((st = upload_array(&charge, t->charge, size_t(N)))) return st;
@@ -386,6 +405,8 @@ gr_status NbSystem::upload(const gr_topology* t) {
     if ((st = upload_array(&pq_d, pq.data(), pq.size()))) return st;
     if ((st = upload_array(&pa_d, palpha.data(), palpha.size()))) return st;
     if ((st = upload_array(&pp_d, pp.data(), pp.size()))) return st;
+    if ((st = upload_array(&cgxo_d, cgx_off.data(), cgx_off.size()))) return st;
+    if ((st = upload_array(&cgx_d, cgx.data(), cgx.size()))) return st;
     h.cg_off = cg_off;
     h.charge = charge;
     h.iac = iac;
@@ -402,6 +423,8 @@ gr_status NbSystem::upload(const gr_topology* t) {
     h.pert_q = pq_d;
     h.pert_alpha = pa_d;
     h.pp = pp_d;
+    h.cgx_off = cgxo_d;
+    h.cgx = cgx_d;
     // solvent exclusions exactly the other atoms of the molecule and no 1-4
     // pairs (Topology::solvate, topology.rs:1240-1262): then the energy-only
     // solvent excluded terms are computed with the per-step water data
@@ -847,7 +870,7 @@ gr_status NbSystem::build_pairlist(cudaStream_t s, bool sync) {
                 GR_WATER_SEARCH(8, true);
 #undef GR_WATER_SEARCH
         }
-        if (NSCG > 0) (++launches, k_solute_search<<<blocks_for(NSCG, 4), 128, 0, s>>>(d_sys));
+        if (NSCG > 0) (++launches, k_solute_search<<<NSCG, kSoluteSearchWarps * 32, 0, s>>>(d_sys));
         if (n_pert > 0 && NSCG > 0) {
             GR_CUDA(cudaMemsetAsync(h.n_pert_pairs, 0, sizeof(int), s));
             (++launches, k_pert_pairs<<<blocks_for((long long)NSCG * h.scap, 256), 256, 0, s>>>(d_sys));

@@ -92,6 +92,8 @@ struct SysDev {
     const double* pert_q;      // [n_pert*2] a, b
     const double* pert_alpha;  // [n_pert*2] lj, crf
     const int* pp;             // [n_pp*4] i, j, a_type, b_type
+    const int* cgx_off;        // n_solute_cg+1: per solute CG, the other solute CGs that share an excluded
+    const int* cgx;            // or 1-4 atom pair with it
     int n_pert, n_pp;
     // ---- state
     double* pos;               // n_atoms*3

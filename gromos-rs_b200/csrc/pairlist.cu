@@ -29,8 +29,9 @@ __device__ __forceinline__ int imod(int a, int m) {
 }
 
 // Cell of stencil lane l (0..26, offsets in z-y-x order, -1..1 per axis;
-// grids of 1 or 2 cells along an axis use the de-duplicated offsets of
-// axis_offsets), -1 for a lane a small grid does not use.  The stencil is
+// grids of 1 or 2 cells along an axis use each cell once: the reference
+// de-duplicates with a HashSet, pairlist.rs:675-692), -1 for a lane a small
+// grid does not use.  The stencil is
 // symmetric: c is in the stencil of c' iff c' is in the stencil of c.
 __device__ __forceinline__ int stencil_cell(int cell, int l, int gx, int gy, int gz) {
     const int ix = l % 3, iy = (l / 3) % 3, iz = l / 9;
@@ -436,24 +437,6 @@ __global__ void __launch_bounds__(256) k_cell_candidates(const SysDev* __restric
             cext[v] = e[u];
         }
     }
-}
-
-// Neighbour cell offsets along one axis, de-duplicated for grids of 1 or 2
-// cells (the reference de-duplicates with a HashSet, pairlist.rs:675-692).
-__device__ __forceinline__ int axis_offsets(int g, int* off) {
-    if (g >= 3) {
-        off[0] = -1;
-        off[1] = 0;
-        off[2] = 1;
-        return 3;
-    }
-    if (g == 2) {
-        off[0] = 0;
-        off[1] = 1;
-        return 2;
-    }
-    off[0] = 0;
-    return 1;
 }
 
 // Water-water search, one warp per i-cluster (clusters handed out by a
@@ -870,67 +853,92 @@ __device__ unsigned long long excl_mask(const SysDev& s, int ci, int cj) {
     return m;
 }
 
+// excl_mask of one CG pair by a whole warp: two of the 64 (a, b) places per
+// lane, gathered with two ballots.  Every lane returns the mask.
+__device__ __forceinline__ unsigned long long excl_mask_warp(const SysDev& s, int ci, int cj, int lane) {
+    const int i0 = s.cg_off[ci], ni = s.cg_off[ci + 1] - i0;
+    const int j0 = s.cg_off[cj], nj = s.cg_off[cj + 1] - j0;
+    unsigned half[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int a = (lane >> 3) + 4 * h, b = lane & 7;
+        const bool ex = a < ni && b < nj && ((ci == cj && b <= a) || excluded_or_14(s, i0 + a, j0 + b));
+        half[h] = __ballot_sync(0xffffffffu, ex);
+    }
+    return (static_cast<unsigned long long>(half[1]) << 32) | half[0];
+}
+
 // Solute CG i against every CG in the neighbour cells: solute j > i
 // (COG-COG, with exclusions for the short range) and every solvent CG
-// (COG-first atom, no exclusion check), pairlist.rs:237-350.  One warp per
-// solute CG.  Entry = (j << 1 | long); the first entry is the CG itself
-// (intra-CG pairs, pairlist.rs:239-249).
-__global__ void k_solute_search(const SysDev* __restrict__ sys) {
-    // Candidates are swept 32 at a time through the neighbour cells in z-y-x
-    // order; positions come from the sorted copy of the reference positions
-    // (sref: the same FP64 values, stored at the sorted position) and the next
-    // round's candidate is loaded while this round's is tested, so a round
-    // waits for one memory latency instead of two chained ones.
+// (COG-first atom, no exclusion check), pairlist.rs:237-350.  Entry =
+// (j << 1 | long); the first entry is the CG itself (intra-CG pairs,
+// pairlist.rs:239-249).
+//
+// One block per solute CG.  A system has few solute CGs and each has every CG
+// of its 27 cells to look at, so one warp per CG left nearly all of the chip
+// idle and its time was the length of that warp's sweep.  Here the
+// neighbour cells' sorted runs are one concatenated candidate range swept 256
+// at a time (positions from the sorted copy, the next round loaded while this
+// one is tested); the hits are compacted in candidate order with the warps'
+// counts, one barrier per round, so the lists are those of a serial sweep.
+// Exclusion masks are only looked up for the CGs that share an excluded or
+// 1-4 pair with this one (cgx, from the topology), after the sweep, one
+// warp per mask.
+constexpr int kSoluteSearchWarps = 8;
+constexpr int kMaskQueue = 64;
+
+__global__ void __launch_bounds__(kSoluteSearchWarps * 32) k_solute_search(const SysDev* __restrict__ sys) {
     const SysDev& s = sys[blockIdx.y];
-    const int lane = threadIdx.x & 31;
-    const int ci = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (ci >= s.n_solute_cg) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int ci = blockIdx.x;
     if (s.cg_off[ci + 1] - s.cg_off[ci] > kMaxCGAtoms) {
-        if (lane == 0) atomicOr(&s.err[0], ERR_CG_TOO_LARGE);
+        if (threadIdx.x == 0) atomicOr(&s.err[0], ERR_CG_TOO_LARGE);
         return;
     }
-    int* out = s.sl + static_cast<size_t>(ci) * s.scap;
-    unsigned long long* outx = s.sl_excl + static_cast<size_t>(ci) * s.scap;
-    int cnt = 0;
-    if (lane == 0) {
-        out[0] = ci << 1;
-        outx[0] = excl_mask(s, ci, ci);
-    }
-    cnt = 1;
-    const double xi = s.ref[3 * ci], yi = s.ref[3 * ci + 1], zi = s.ref[3 * ci + 2];
-    const int cell = s.cg_cell[ci];
-    const int gx = s.gdim[0], gy = s.gdim[1], gz = s.gdim[2];
-    const int cx = cell % gx, cy = (cell / gx) % gy, cz = cell / (gx * gy);
-    int ox[3], oy[3], oz[3];
-    const int nx = axis_offsets(gx, ox), ny = axis_offsets(gy, oy), nz = axis_offsets(gz, oz);
-    int ncl[27];
-    int nn = 0;
-    for (int iz = 0; iz < nz; ++iz)
-        for (int iy = 0; iy < ny; ++iy)
-            for (int ix = 0; ix < nx; ++ix)
-                ncl[nn++] = imod(cx + ox[ix], gx) + gx * (imod(cy + oy[iy], gy) + gy * imod(cz + oz[iz], gz));
-    const int stride = s.n_cg + 2;
-    const int* __restrict__ cell_start = s.cell_start;
+    __shared__ int seg_lo[27], seg_pre[28];
+    __shared__ int wcnt[2][kSoluteSearchWarps];
+    __shared__ int q_p[kMaskQueue], q_cj[kMaskQueue], qn;
+    int* __restrict__ out = s.sl + static_cast<size_t>(ci) * s.scap;
+    unsigned long long* __restrict__ outx = s.sl_excl + static_cast<size_t>(ci) * s.scap;
     const int* __restrict__ sorted_cg = s.sorted_cg;
     const double* __restrict__ sref = s.sref;
-    // sweep state: neighbour k, round start base within [cell_start[ncl[k]], cell_start[ncl[k] + 1])
-    int k = 0, base = 0, end = 0;
-    auto seek = [&]() {  // first non-empty cell at or after k
-        while (k < nn) {
-            base = cell_start[ncl[k]];
-            end = cell_start[ncl[k] + 1];
-            if (base < end) return;
-            ++k;
+    const int* __restrict__ cgx = s.cgx;
+    const int stride = s.n_cg + 2, nscg = s.n_solute_cg, scap = s.scap;
+    const int x0 = s.cgx_off[ci], x1 = s.cgx_off[ci + 1];
+    const double xi = s.ref[3 * ci], yi = s.ref[3 * ci + 1], zi = s.ref[3 * ci + 2];
+    if (w == 0) {
+        const int nc = lane < 27 ? stencil_cell(s.cg_cell[ci], lane, s.gdim[0], s.gdim[1], s.gdim[2]) : -1;
+        const int lo = nc >= 0 ? s.cell_start[nc] : 0;
+        const int len = nc >= 0 ? s.cell_start[nc + 1] - lo : 0;
+        int incl = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
         }
-    };
+        if (lane < 27) {
+            seg_lo[lane] = lo;
+            seg_pre[lane + 1] = incl;
+        }
+        if (lane == 0) {
+            seg_pre[0] = 0;
+            qn = 0;
+        }
+    }
+    __syncthreads();
+    const int total = seg_pre[27];
     struct Cand {
         int cj;
         double x, y, z;
     };
-    auto load = [&](int b, int e) {
+    auto load = [&](int v) {
         Cand c{-1, 0.0, 0.0, 0.0};
-        const int sp = b + lane;
-        if (sp < e) {
+        if (v < total) {
+            int lo = 0;  // run of v: the last one that starts at or before it
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1)
+                if (lo + step < 27 && seg_pre[lo + step] <= v) lo += step;
+            const int sp = seg_lo[lo] + v - seg_pre[lo];
             c.cj = sorted_cg[sp];
             c.x = sref[sp];
             c.y = sref[stride + sp];
@@ -938,55 +946,71 @@ __global__ void k_solute_search(const SysDev* __restrict__ sys) {
         }
         return c;
     };
-    seek();
-    Cand cur = k < nn ? load(base, end) : Cand{-1, 0.0, 0.0, 0.0};
-    while (k < nn) {
-        // the next round: advance, then load it before this round is tested
-        int nb = base + 32, ne = end;
-        if (nb >= end) {
-            ++k;
-            seek();
-            nb = base;
-            ne = end;
-        }
-        const bool more = k < nn;
-        const Cand nxt = more ? load(nb, ne) : Cand{-1, 0.0, 0.0, 0.0};
+    int cnt = 1;  // the CG's own entry is written last
+    Cand cur = load(threadIdx.x);
+    for (int v0 = 0, par = 0; v0 < total; v0 += blockDim.x, par ^= 1) {
+        const Cand nxt = load(v0 + int(blockDim.x) + int(threadIdx.x));
         int entry = -1;
-        unsigned long long xm = 0;
+        bool masked = false;
         const int cj = cur.cj;
-        if (cj >= 0) {
-            const bool solute_j = cj < s.n_solute_cg;
-            if (!solute_j || cj > ci) {
-                double rx, ry, rz;
-                nearest_image_exact(s, xi, yi, zi, cur.x, cur.y, cur.z, rx, ry, rz);
-                const double d2 = len2_exact(rx, ry, rz);
-                if (!(d2 > s.c2l)) {
-                    const int lr = d2 > s.c2s ? 1 : 0;
-                    if (solute_j && s.cg_off[cj + 1] - s.cg_off[cj] > kMaxCGAtoms) {
-                        atomicOr(&s.err[0], ERR_CG_TOO_LARGE);
-                    } else {
-                        entry = (cj << 1) | lr;
-                        if (solute_j && !lr) xm = excl_mask(s, ci, cj);
-                    }
+        if (cj >= nscg || cj > ci) {
+            double rx, ry, rz;
+            nearest_image_exact(s, xi, yi, zi, cur.x, cur.y, cur.z, rx, ry, rz);
+            const double d2 = len2_exact(rx, ry, rz);
+            if (!(d2 > s.c2l)) {
+                const int lr = d2 > s.c2s ? 1 : 0;
+                if (cj < nscg && s.cg_off[cj + 1] - s.cg_off[cj] > kMaxCGAtoms) {
+                    atomicOr(&s.err[0], ERR_CG_TOO_LARGE);
+                } else {
+                    entry = (cj << 1) | lr;
+                    if (cj < nscg && !lr)
+                        for (int k = x0; k < x1; ++k) masked |= cgx[k] == cj;
                 }
             }
         }
         const unsigned bal = __ballot_sync(0xffffffffu, entry >= 0);
+        if (lane == 0) wcnt[par][w] = __popc(bal);
+        __syncthreads();
+        int before = 0, round = 0;
+#pragma unroll
+        for (int k = 0; k < kSoluteSearchWarps; ++k) {
+            const int c = wcnt[par][k];
+            if (k < w) before += c;
+            round += c;
+        }
         if (entry >= 0) {
-            const int p = cnt + __popc(bal & ((1u << lane) - 1u));
-            if (p < s.scap) {
+            const int p = cnt + before + __popc(bal & ((1u << lane) - 1u));
+            if (p < scap) {
                 out[p] = entry;
+                unsigned long long xm = 0ull;
+                if (masked) {
+                    const int q = atomicAdd(&qn, 1);
+                    if (q < kMaskQueue) {
+                        q_p[q] = p;
+                        q_cj[q] = cj;
+                    } else {
+                        xm = excl_mask(s, ci, cj);
+                    }
+                }
                 outx[p] = xm;
             }
         }
-        cnt += __popc(bal);
+        cnt += round;
         cur = nxt;
-        base = nb;
-        end = ne;
     }
-    if (lane == 0) {
-        if (cnt > s.scap) atomicOr(&s.err[0], ERR_SLIST_OVERFLOW);
-        s.sn[ci] = min(cnt, s.scap);
+    __syncthreads();  // the queue, and the zero masks of its entries
+    const int nq = min(qn, kMaskQueue);
+    for (int q = w; q <= nq; q += kSoluteSearchWarps) {
+        const int cj = q < nq ? q_cj[q] : ci, p = q < nq ? q_p[q] : 0;  // the last one: the CG itself
+        const unsigned long long xm = excl_mask_warp(s, ci, cj, lane);
+        if (lane == 0) {
+            outx[p] = xm;
+            if (q == nq) out[0] = ci << 1;
+        }
+    }
+    if (threadIdx.x == 0) {
+        if (cnt > scap) atomicOr(&s.err[0], ERR_SLIST_OVERFLOW);
+        s.sn[ci] = min(cnt, scap);
     }
 }
 

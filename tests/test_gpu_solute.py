@@ -1,0 +1,48 @@
+"""GPU: the solute pairlist search and the solute force kernels at their edges, against the FP64 oracle."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from gromos_nb import generators
+from gromos_nb.system import csr_from_lists
+from test_gpu_parity import check_pairlist, compare_eval
+
+pytestmark = pytest.mark.gpu
+
+
+def linked_solute(n_waters, n_solute, seed, links, o14=0, hub=0, rcutp=0.8, rcutl=1.4, single=False):
+    """A solvated solute whose charge groups share `links` random excluded atom pairs and `o14` 1-4
+    pairs; `hub` charge groups exclude the first atom."""
+    s = generators.solvated_solute_system(n_waters, n_solute, seed=seed, single_atom_cgs=single)
+    t = s.topo
+    rng = np.random.default_rng(seed + 1)
+    cg = t.atom_to_cg()
+    excl = [set(t.excl[t.excl_off[a]:t.excl_off[a + 1]].tolist()) for a in range(t.n_atoms)]
+    f14 = [set() for _ in range(t.n_atoms)]
+    pairs = [tuple(sorted(p)) for p in rng.integers(0, t.n_solute_atoms, (links + o14, 2)).tolist()]
+    pairs = [p for p in pairs if cg[p[0]] != cg[p[1]]]
+    first = t.cg_offsets[1:1 + hub]
+    for a, b in pairs[:links] + [(0, int(b)) for b in first]:
+        excl[a].add(b)
+        excl[b].add(a)
+    for a, b in pairs[links:]:
+        if b not in excl[a]:
+            f14[a].add(b)
+    eo, ef = csr_from_lists([sorted(x) for x in excl], t.n_atoms)
+    fo, ff = csr_from_lists([sorted(x) for x in f14], t.n_atoms)
+    s.topo = dataclasses.replace(t, excl_off=eo, excl=ef, o14_off=fo, o14=ff)
+    s.params.rcutp, s.params.rcutl = rcutp, rcutl
+    return s
+
+
+# candidate counts around the 256 of one sweep round (80: below one, 256: one exactly with the
+# solute's groups, 700: several); 300 links over few groups; one group with more than the 64 masks
+# that a block queues
+@pytest.mark.parametrize("waters,solute,links,o14,hub,single", [
+    (80, 12, 4, 3, 0, False), (226, 30, 0, 0, 0, True), (700, 60, 300, 20, 0, False),
+    (900, 120, 30, 10, 80, True), (1500, 6, 0, 0, 0, False)])
+def test_solute_lists_with_exclusions_between_groups(waters, solute, links, o14, hub, single):
+    s = linked_solute(waters, solute, 31 + waters, links, o14, hub, single=single)
+    check_pairlist(s)
+    compare_eval(s, steps=2, move=0.001)
