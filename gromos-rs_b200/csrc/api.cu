@@ -443,6 +443,19 @@ gr_status NbSystem::upload(const gr_topology* t) {
             if (k != h_excl_off[a + 1] || h_o14_off[a + 1] != h_o14_off[a]) solvent_excl_intra = false;
         }
     h.excl_atoms = solvent_excl_intra ? NSA : N;
+    // the excluded and 1-4 pairs (i < j) that k_excluded_14 evaluates
+    std::vector<int2> terms;
+    for (int a = 0; a < h.excl_atoms; ++a)
+        for (int k = h_excl_off[a]; k < h_excl_off[a + 1]; ++k)
+            if (h_excl[k] > a) terms.push_back(make_int2(a, h_excl[k]));
+    h.n_ex_pairs = int(terms.size());
+    for (int a = 0; a < h.excl_atoms; ++a)
+        for (int k = h_o14_off[a]; k < h_o14_off[a + 1]; ++k)
+            if (h_o14[k] > a) terms.push_back(make_int2(a, h_o14[k]));
+    h.n_14_pairs = int(terms.size()) - h.n_ex_pairs;
+    int2* terms_d = nullptr;
+    if ((st = upload_array(&terms_d, terms.data(), terms.size()))) return st;
+    h.term_pairs = terms_d;
     // solvent parameter table from the first solvent molecule (innerloops.rs:241-255)
     h.water_lj00_only = 1;
     if (NSA < N) {
@@ -1027,7 +1040,12 @@ gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events) {
     }
     if (stage) GR_CUDA(record_event(ev[3], s));
     const size_t sha = size_t(NA) * sizeof(unsigned long long);
-    if (h.excl_atoms > 0) (++launches, k_excluded_14<<<blocks_for(h.excl_atoms, 128), 128, sha, s>>>(d_sys));
+    // one thread per term, in small blocks: the few terms of a solute spread over SMs
+    const int nterm = NSA + h.n_ex_pairs + h.n_14_pairs;
+    if (nterm > 0) {
+        const int bt = nterm <= 64 * sm ? 64 : 128;
+        (++launches, k_excluded_14<<<blocks_for(nterm, bt), bt, sha, s>>>(d_sys));
+    }
     if (n_pert > 0) {
         if (NSCG > 0)
             (++launches, k_pert_pairs_force<<<blocks_for((std::max(pcap_alloc, 1) + kPertRun - 1) / kPertRun, 128), 128, sha,

@@ -94,6 +94,8 @@ struct SysDev {
     const int* pp;             // [n_pp*4] i, j, a_type, b_type
     const int* cgx_off;        // n_solute_cg+1: per solute CG, the other solute CGs that share an excluded
     const int* cgx;            // or 1-4 atom pair with it
+    const int2* term_pairs;    // excluded pairs (i < j, i < excl_atoms), then 1-4 pairs
+    int n_ex_pairs, n_14_pairs;
     int n_pert, n_pp;
     // ---- state
     double* pos;               // n_atoms*3
