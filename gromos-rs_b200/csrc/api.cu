@@ -119,23 +119,107 @@ cudaError_t device_pool(cudaMemPool_t* pool) {
     return cudaSuccess;
 }
 
+// Small page-locked host buffers (error flags, energies read back): cudaMallocHost
+// and cudaFreeHost take a millisecond or two each beside a busy process's
+// mappings, and a context needs four such buffers, which was most of the time
+// to create and release one.  Blocks of 256 B, 1 KB and 8 KB come from slabs of
+// 256 KB; a slab whose blocks are all back is freed, except the last of its size.
+// A block is returned only when no copy into it is under way (its context's
+// stream is synchronised first).
+struct PinnedSlabs {
+    static constexpr size_t kClass[3] = {256, 1024, 8192}, kSlab = 256 << 10;
+    struct Slab {
+        char* base;
+        size_t live;
+    };
+    std::mutex mu;
+    std::vector<Slab> slabs[3];
+    std::vector<char*> free_blocks[3];
+};
+
+static PinnedSlabs& pinned_slabs() {
+    static PinnedSlabs* p = new PinnedSlabs;  // never destroyed: contexts may be released at exit
+    return *p;
+}
+
+cudaError_t pinned_alloc(void** out, size_t n) {
+    *out = nullptr;
+    int k = 0;
+    while (k < 3 && PinnedSlabs::kClass[k] < n) ++k;
+    if (k == 3) return cudaHostAlloc(out, n, cudaHostAllocPortable);
+    PinnedSlabs& P = pinned_slabs();
+    std::lock_guard<std::mutex> lock(P.mu);
+    if (P.free_blocks[k].empty()) {
+        void* base = nullptr;
+        const cudaError_t e = cudaHostAlloc(&base, PinnedSlabs::kSlab, cudaHostAllocPortable);
+        if (e != cudaSuccess) return e;
+        P.slabs[k].push_back({static_cast<char*>(base), 0});
+        for (size_t o = PinnedSlabs::kSlab; o > 0; o -= PinnedSlabs::kClass[k])
+            P.free_blocks[k].push_back(static_cast<char*>(base) + o - PinnedSlabs::kClass[k]);
+    }
+    char* b = P.free_blocks[k].back();
+    P.free_blocks[k].pop_back();
+    for (auto& s : P.slabs[k])
+        if (b >= s.base && b < s.base + PinnedSlabs::kSlab) ++s.live;
+    *out = b;
+    return cudaSuccess;
+}
+
+void pinned_free(void* p, size_t n) {
+    if (!p) return;
+    int k = 0;
+    while (k < 3 && PinnedSlabs::kClass[k] < n) ++k;
+    if (k == 3) {
+        cudaFreeHost(p);
+        return;
+    }
+    PinnedSlabs& P = pinned_slabs();
+    std::lock_guard<std::mutex> lock(P.mu);
+    char* b = static_cast<char*>(p);
+    P.free_blocks[k].push_back(b);
+    for (size_t i = 0; i < P.slabs[k].size(); ++i) {
+        PinnedSlabs::Slab& s = P.slabs[k][i];
+        if (b < s.base || b >= s.base + PinnedSlabs::kSlab) continue;
+        if (--s.live > 0 || P.slabs[k].size() == 1) return;
+        char* base = s.base;
+        auto& f = P.free_blocks[k];
+        f.erase(std::remove_if(f.begin(), f.end(),
+                               [&](char* q) { return q >= base && q < base + PinnedSlabs::kSlab; }),
+                f.end());
+        P.slabs[k].erase(P.slabs[k].begin() + long(i));
+        cudaFreeHost(base);
+        return;
+    }
+}
+
+template <class T>
+static cudaError_t pinned_alloc(T** out, size_t n) {
+    void* p = nullptr;
+    const cudaError_t e = pinned_alloc(&p, n * sizeof(T));
+    *out = static_cast<T*>(p);
+    return e;
+}
+
 // A pool allocation, complete before it returns (so any stream and synchronous
 // copies may use it at once), and its release after the work on this
 // context's stream.  Buffers are reallocated or released only when no other
 // stream has work on them (batch steps synchronise before members change).
-cudaError_t NbSystem::dev_malloc(void** p, size_t n) {
+cudaError_t pool_malloc(void** p, size_t n, cudaStream_t s) {
     cudaMemPool_t pool = nullptr;
     cudaError_t e = device_pool(&pool);
-    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(p, n, pool, mem_stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(mem_stream);
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(p, n, pool, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     return e;
 }
 
-void NbSystem::dev_free(void* p) {
+void pool_free(void* p, cudaStream_t s) {
     if (!p) return;
-    cudaStreamSynchronize(mem_stream);
-    cudaFreeAsync(p, mem_stream);
+    cudaStreamSynchronize(s);
+    cudaFreeAsync(p, s);
 }
+
+cudaError_t NbSystem::dev_malloc(void** p, size_t n) { return pool_malloc(p, n, mem_stream); }
+void NbSystem::dev_free(void* p) { pool_free(p, mem_stream); }
 
 NbSystem::~NbSystem() { release(); }
 
@@ -156,15 +240,15 @@ void NbSystem::release() {
     for (auto& e : evk) e = nullptr;
     if (ev_err) cudaEventDestroy(ev_err);
     ev_err = nullptr;
-    if (err_host) cudaFreeHost(err_host);
+    pinned_free(err_host, 4 * sizeof(int));
     err_host = nullptr;
     pending_check = false;
     drop_graphs();
-    if (err_step_host) cudaFreeHost(err_step_host);
+    pinned_free(err_step_host, 4 * sizeof(int));
     err_step_host = nullptr;
-    if (err_dl_host) cudaFreeHost(err_dl_host);
+    pinned_free(err_dl_host, 4 * sizeof(int));
     err_dl_host = nullptr;
-    if (e_dl_host) cudaFreeHost(e_dl_host);
+    pinned_free(e_dl_host, size_t(e_dl_n) * sizeof(double));
     e_dl_host = nullptr;
     e_dl_n = 0;
     if (ev_step) cudaEventDestroy(ev_step);
@@ -179,7 +263,7 @@ void NbSystem::release() {
     md_psnap_ke = nullptr;
     md_psnap_valid = false;
     md_fail = nullptr;
-    if (md_err_host) cudaFreeHost(md_err_host);
+    pinned_free(md_err_host, 8 * sizeof(long long));
     md_err_host = nullptr;
     if (ev_md) cudaEventDestroy(ev_md);
     ev_md = nullptr;
@@ -510,7 +594,7 @@ gr_status NbSystem::upload(const gr_topology* t) {
     for (auto& e : ev) GR_CUDA(cudaEventCreate(&e));
     for (auto& e : evk) GR_CUDA(cudaEventCreate(&e));
     GR_CUDA(cudaEventCreateWithFlags(&ev_err, cudaEventDisableTiming));
-    if (!err_host) GR_CUDA(cudaMallocHost(reinterpret_cast<void**>(&err_host), 4 * sizeof(int)));
+    if (!err_host) GR_CUDA(pinned_alloc(&err_host, 4));
     err_host[0] = 0;
     pending_check = false;
     ever_built = false;
@@ -1080,7 +1164,7 @@ void NbSystem::drop_graphs() {
 // an overflow) run through eval().
 gr_status NbSystem::eval_graph(cudaStream_t s, int flags) {
     gr_status st;
-    if (!err_step_host) GR_CUDA(cudaMallocHost(&err_step_host, 4 * sizeof(int)));
+    if (!err_step_host) GR_CUDA(pinned_alloc(&err_step_host, 4));
     if (!ev_step) GR_CUDA(cudaEventCreateWithFlags(&ev_step, cudaEventDisableTiming));
     if (step_check) {  // flags of the previous graph step (deferred-pair overflow)
         GR_CUDA(cudaEventSynchronize(ev_step));
@@ -1380,20 +1464,27 @@ gr_status NbSystem::pair_counts(cudaStream_t s, long long* n_short, long long* n
     return GR_OK;
 }
 
+// The page-locked buffer of the energies (and, for md_stats, two more words).
+gr_status NbSystem::energy_buffer() {
+    const int n = acc_size(G) + 2;
+    if (e_dl_n >= n) return GR_OK;
+    pinned_free(e_dl_host, size_t(e_dl_n) * sizeof(double));
+    e_dl_host = nullptr;
+    e_dl_n = 0;
+    GR_CUDA(pinned_alloc(&e_dl_host, size_t(n)));
+    e_dl_n = n;
+    return GR_OK;
+}
+
 // Energies, the error flags and (if requested) the forces are copied in
 // stream order -- the flags and energies into pinned buffers -- and read
 // after one synchronisation.
 gr_status NbSystem::download(cudaStream_t s, gr_result* out) {
     if (!out) return GR_OK;
     const int NA = acc_size(G);
-    if (e_dl_n < NA) {
-        if (e_dl_host) cudaFreeHost(e_dl_host);
-        e_dl_host = nullptr;
-        e_dl_n = 0;
-        GR_CUDA(cudaMallocHost(&e_dl_host, size_t(NA) * sizeof(double)));
-        e_dl_n = NA;
-    }
-    if (!err_dl_host) GR_CUDA(cudaMallocHost(&err_dl_host, 4 * sizeof(int)));
+    gr_status st = energy_buffer();
+    if (st) return st;
+    if (!err_dl_host) GR_CUDA(pinned_alloc(&err_dl_host, 4));
     const double* e = e_dl_host;
     GR_CUDA(cudaMemcpyAsync(e_dl_host, h.e_out, NA * sizeof(double), cudaMemcpyDeviceToHost, s));
     GR_CUDA(cudaMemcpyAsync(err_dl_host, h.err, 4 * sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1727,6 +1818,30 @@ gr_status gr_forces_eval(gr_ctx* ctx, int32_t flags, gr_result* out) {
     return GR_OK;
 }
 
+// Page-locked host memory for result buffers: a download into it is one DMA
+// transfer, where one into pageable memory is staged by the driver and faults
+// in every fresh page on the way.
+gr_status gr_host_alloc(size_t bytes, void** out) {
+    if (!out || bytes == 0) {
+        set_error("gr_host_alloc: null out or no bytes");
+        return GR_ERR_INVALID;
+    }
+    *out = nullptr;
+    const cudaError_t e = cudaHostAlloc(out, bytes, cudaHostAllocPortable);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        *out = nullptr;
+        set_error(std::string("gr_host_alloc: ") + cudaGetErrorString(e));
+        return e == cudaErrorMemoryAllocation ? GR_ERR_OOM : GR_ERR_CUDA;
+    }
+    return GR_OK;
+}
+
+gr_status gr_host_free(void* p) {
+    if (p) GR_CUDA(cudaFreeHost(p));
+    return GR_OK;
+}
+
 gr_status gr_forces_device(gr_ctx* ctx, const double** dev_forces) {
     CTX_GUARD(ctx);
     if (!dev_forces) return GR_ERR_INVALID;
@@ -1849,16 +1964,17 @@ extern "C" gr_status gr_lj_crf_innerloop(const float* positions, const float* ch
         set_error("gr_lj_crf_innerloop: null input");
         return GR_ERR_INVALID;
     }
-    for (uint32_t p = 0; p < 2 * n_pairs; ++p)
-        if (pairlist[p] >= n_atoms) {
-            set_error("gr_lj_crf_innerloop: pair index out of range");
-            return GR_ERR_INVALID;
-        }
-    for (uint32_t a = 0; a < n_atoms; ++a)
-        if (iac[a] >= n_types) {
-            set_error("gr_lj_crf_innerloop: iac out of range");
-            return GR_ERR_INVALID;
-        }
+    uint32_t most_i = 0, most_t = 0;  // the largest index and type: plain maxima, which vectorise
+    for (size_t p = 0; p < 2 * size_t(n_pairs); ++p) most_i = std::max(most_i, pairlist[p]);
+    for (uint32_t a = 0; a < n_atoms; ++a) most_t = std::max(most_t, iac[a]);
+    if (most_i >= n_atoms) {
+        set_error("gr_lj_crf_innerloop: pair index out of range");
+        return GR_ERR_INVALID;
+    }
+    if (most_t >= n_types) {
+        set_error("gr_lj_crf_innerloop: iac out of range");
+        return GR_ERR_INVALID;
+    }
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
         set_error("gr_lj_crf_innerloop: no CUDA device");
@@ -1866,27 +1982,44 @@ extern "C" gr_status gr_lj_crf_innerloop(const float* positions, const float* ch
     }
     std::vector<float2> lj(size_t(n_types) * n_types);
     for (size_t k = 0; k < lj.size(); ++k) lj[k] = make_float2(float(lj_params[2 * k]), float(lj_params[2 * k + 1]));
-    float *dpos = nullptr, *dq = nullptr, *dF = nullptr;
-    uint32_t *diac = nullptr, *dpairs = nullptr;
-    float2* dlj = nullptr;
-    double* dE = nullptr;
+    // one block of the library's pool holds every buffer (seven allocations and
+    // releases of their own, each a device synchronisation, took about a millisecond)
+    size_t total = 0;
+    auto place = [&](size_t n) {
+        const size_t at = total;
+        total += (n + 255) / 256 * 256;
+        return at;
+    };
+    const size_t o_pairs = place(sizeof(uint32_t) * 2 * size_t(n_pairs)), o_pos = place(sizeof(float) * 3 * size_t(n_atoms));
+    const size_t o_q = place(sizeof(float) * size_t(n_atoms)), o_iac = place(sizeof(uint32_t) * size_t(n_atoms));
+    const size_t o_lj = place(sizeof(float2) * lj.size());
+    const size_t o_F = place(sizeof(float) * 3 * size_t(n_atoms)), o_E = place(sizeof(double) * 11);
+    char* block = nullptr;
     gr_status st = GR_OK;
     auto fail = [&](cudaError_t e) {
         set_error(std::string("gr_lj_crf_innerloop: ") + cudaGetErrorString(e));
         st = GR_ERR_CUDA;
     };
-    cudaError_t e;
-    if ((e = cudaMalloc(&dpos, sizeof(float) * 3 * n_atoms)) || (e = cudaMalloc(&dq, sizeof(float) * n_atoms)) ||
-        (e = cudaMalloc(&dF, sizeof(float) * 3 * n_atoms)) || (e = cudaMalloc(&diac, sizeof(uint32_t) * n_atoms)) ||
-        (e = cudaMalloc(&dpairs, sizeof(uint32_t) * 2 * n_pairs)) || (e = cudaMalloc(&dlj, sizeof(float2) * lj.size())) ||
-        (e = cudaMalloc(&dE, sizeof(double) * 11))) {
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = device_pool(&pool);
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&block), total, pool, 0);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
         fail(e);
-    } else if ((e = cudaMemcpy(dpos, positions, sizeof(float) * 3 * n_atoms, cudaMemcpyHostToDevice)) ||
-               (e = cudaMemcpy(dq, charges, sizeof(float) * n_atoms, cudaMemcpyHostToDevice)) ||
-               (e = cudaMemcpy(diac, iac, sizeof(uint32_t) * n_atoms, cudaMemcpyHostToDevice)) ||
-               (e = cudaMemcpy(dpairs, pairlist, sizeof(uint32_t) * 2 * n_pairs, cudaMemcpyHostToDevice)) ||
-               (e = cudaMemcpy(dlj, lj.data(), sizeof(float2) * lj.size(), cudaMemcpyHostToDevice)) ||
-               (e = cudaMemset(dF, 0, sizeof(float) * 3 * n_atoms)) || (e = cudaMemset(dE, 0, sizeof(double) * 11))) {
+        return st;
+    }
+    uint32_t* dpairs = reinterpret_cast<uint32_t*>(block + o_pairs);
+    uint32_t* diac = reinterpret_cast<uint32_t*>(block + o_iac);
+    float *dpos = reinterpret_cast<float*>(block + o_pos), *dq = reinterpret_cast<float*>(block + o_q);
+    float* dF = reinterpret_cast<float*>(block + o_F);
+    float2* dlj = reinterpret_cast<float2*>(block + o_lj);
+    double* dE = reinterpret_cast<double*>(block + o_E);
+    if ((e = cudaMemcpyAsync(dpairs, pairlist, sizeof(uint32_t) * 2 * size_t(n_pairs), cudaMemcpyHostToDevice, 0)) ||
+        (e = cudaMemcpyAsync(dpos, positions, sizeof(float) * 3 * size_t(n_atoms), cudaMemcpyHostToDevice, 0)) ||
+        (e = cudaMemcpyAsync(dq, charges, sizeof(float) * size_t(n_atoms), cudaMemcpyHostToDevice, 0)) ||
+        (e = cudaMemcpyAsync(diac, iac, sizeof(uint32_t) * size_t(n_atoms), cudaMemcpyHostToDevice, 0)) ||
+        (e = cudaMemcpyAsync(dlj, lj.data(), sizeof(float2) * lj.size(), cudaMemcpyHostToDevice, 0)) ||
+        (e = cudaMemsetAsync(block + o_F, 0, total - o_F, 0))) {
         fail(e);
     } else {
         float bx = boundary_type ? float(box_data[0]) : 1.f, by = boundary_type ? float(box_data[1]) : 1.f;
@@ -1905,13 +2038,8 @@ extern "C" gr_status gr_lj_crf_innerloop(const float* positions, const float* ch
             for (int k = 0; k < 9; ++k) virial[k] = h[2 + k];
         }
     }
-    cudaFree(dpos);
-    cudaFree(dq);
-    cudaFree(dF);
-    cudaFree(diac);
-    cudaFree(dpairs);
-    cudaFree(dlj);
-    cudaFree(dE);
+    cudaStreamSynchronize(0);  // also after an error: nothing may still read the caller's arrays
+    cudaFreeAsync(block, 0);
     return st;
 }
 

@@ -85,15 +85,16 @@ gr_status batch_capacity(gr_batch* b) {
     const int n = int(b->m.size());
     if (n <= b->cap) return GR_OK;
     const int c = std::max(n, 2 * b->cap + 8);
-    if (b->d_errp) cudaFree(b->d_errp);
-    if (b->d_flags) cudaFree(b->d_flags);
-    if (b->h_flags) cudaFreeHost(b->h_flags);
+    gnb::pool_free(b->d_errp, b->s0);
+    gnb::pool_free(b->d_flags, b->s0);
+    gnb::pinned_free(b->h_flags, sizeof(int) * size_t(b->cap));
     b->d_errp = nullptr;
     b->d_flags = nullptr;
     b->h_flags = nullptr;
-    GR_CUDA(cudaMalloc(&b->d_errp, sizeof(int*) * c));
-    GR_CUDA(cudaMalloc(&b->d_flags, sizeof(int) * c));
-    GR_CUDA(cudaMallocHost(&b->h_flags, sizeof(int) * c));
+    b->cap = 0;
+    GR_CUDA(gnb::pool_malloc(reinterpret_cast<void**>(&b->d_errp), sizeof(int*) * c, b->s0));
+    GR_CUDA(gnb::pool_malloc(reinterpret_cast<void**>(&b->d_flags), sizeof(int) * c, b->s0));
+    GR_CUDA(gnb::pinned_alloc(&b->h_flags, size_t(c)));
     b->cap = c;
     return GR_OK;
 }
@@ -326,9 +327,9 @@ gr_status gr_batch_destroy(gr_batch* b) {
         if (mb.join) cudaEventDestroy(mb.join);
         mb.ctx->sys.batch_member = false;
     }
-    if (b->d_errp) cudaFree(b->d_errp);
-    if (b->d_flags) cudaFree(b->d_flags);
-    if (b->h_flags) cudaFreeHost(b->h_flags);
+    gnb::pool_free(b->d_errp, b->s0);
+    gnb::pool_free(b->d_flags, b->s0);
+    gnb::pinned_free(b->h_flags, sizeof(int) * size_t(b->cap));
     for (cudaEvent_t e : {b->fork, b->done, b->t0, b->t1})
         if (e) cudaEventDestroy(e);
     cudaStreamDestroy(b->s0);

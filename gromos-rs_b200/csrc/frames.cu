@@ -37,18 +37,18 @@ extern "C" gr_status gr_energy_frames(gr_ctx* ctx, int32_t n_frames, const doubl
     cudaEvent_t ev[2] = {nullptr, nullptr};
     gr_status r = GR_OK;
     auto cleanup = [&]() {
-        if (dE) cudaFree(dE);
-        if (pin_err) cudaFreeHost(pin_err);
+        if (dE) S.dev_free(dE);
+        gnb::pinned_free(pin_err, 8 * sizeof(int));
         for (auto& e : ev)
             if (e) cudaEventDestroy(e);
     };
-    if (cudaMalloc(&dE, size_t(n_frames) * NA * sizeof(double)) != cudaSuccess) {
+    if (S.dev_malloc(reinterpret_cast<void**>(&dE), size_t(n_frames) * NA * sizeof(double)) != cudaSuccess) {
         cudaGetLastError();
         dE = nullptr;
         set_error("gr_energy_frames: device allocation of the per-frame energies failed");
         return GR_ERR_OOM;
     }
-    if (cudaMallocHost(&pin_err, 8 * sizeof(int)) != cudaSuccess ||
+    if (gnb::pinned_alloc(&pin_err, 8) != cudaSuccess ||
         cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming) != cudaSuccess) {
         cudaGetLastError();

@@ -267,7 +267,7 @@ gr_status NbSystem::md_init(const double* mass, const double* vel, const gr_md_p
     // an MD run starts a pairlist period with a build at its first step
     built = false;
     lr_computed = false;
-    if (!md_err_host) GR_CUDA(cudaMallocHost(&md_err_host, 8 * sizeof(long long)));
+    if (!md_err_host) GR_CUDA(pinned_alloc(&md_err_host, 8));
     if (!ev_md) GR_CUDA(cudaEventCreateWithFlags(&ev_md, cudaEventDisableTiming));
     mdp = *p;
     md_settle = settle;
@@ -316,13 +316,18 @@ gr_status NbSystem::md_step_launch(cudaStream_t s, bool fuse_prep) {
 }
 
 gr_status NbSystem::md_stats(cudaStream_t s, gr_md_stats* out) {
-    long long ke = 0;
-    int fails = 0;
-    std::vector<double> e(acc_size(G));
-    GR_CUDA(cudaMemcpyAsync(&ke, md_ke, sizeof(ke), cudaMemcpyDeviceToHost, s));
-    GR_CUDA(cudaMemcpyAsync(&fails, md_fail, sizeof(int), cudaMemcpyDeviceToHost, s));
-    GR_CUDA(cudaMemcpyAsync(e.data(), h.e_out, e.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
+    const int NA = acc_size(G);
+    gr_status st = energy_buffer();
+    if (st) return st;
+    const double* e = e_dl_host;
+    long long* ke_host = reinterpret_cast<long long*>(e_dl_host + NA);
+    int* fails_host = reinterpret_cast<int*>(e_dl_host + NA + 1);
+    GR_CUDA(cudaMemcpyAsync(ke_host, md_ke, sizeof(long long), cudaMemcpyDeviceToHost, s));
+    GR_CUDA(cudaMemcpyAsync(fails_host, md_fail, sizeof(int), cudaMemcpyDeviceToHost, s));
+    GR_CUDA(cudaMemcpyAsync(e_dl_host, h.e_out, size_t(NA) * sizeof(double), cudaMemcpyDeviceToHost, s));
     GR_CUDA(cudaStreamSynchronize(s));
+    const long long ke = *ke_host;
+    const int fails = *fails_host;
     double elj = 0.0, ecrf = 0.0;
     for (int g = 0; g < G * G; ++g) {
         elj += e[g];
@@ -525,9 +530,12 @@ gr_status gr_md_download(gr_ctx* ctx, double* pos, double* vel) {
         return GR_ERR_STATE;
     }
     const size_t bytes3 = size_t(S.N) * 3 * sizeof(double);
-    if (pos) GR_CUDA(cudaMemcpyAsync(pos, S.h.pos, bytes3, cudaMemcpyDeviceToHost, ctx->stream));
-    if (vel) GR_CUDA(cudaMemcpyAsync(vel, S.md_vel, bytes3, cudaMemcpyDeviceToHost, ctx->stream));
-    GR_CUDA(cudaStreamSynchronize(ctx->stream));
+    cudaError_t e = cudaSuccess;
+    if (pos) e = cudaMemcpyAsync(pos, S.h.pos, bytes3, cudaMemcpyDeviceToHost, ctx->stream);
+    if (vel && e == cudaSuccess) e = cudaMemcpyAsync(vel, S.md_vel, bytes3, cudaMemcpyDeviceToHost, ctx->stream);
+    // also after an error: no copy may still be under way into the caller's buffers
+    const cudaError_t e2 = cudaStreamSynchronize(ctx->stream);
+    GR_CUDA(e != cudaSuccess ? e : e2);
     return GR_OK;
 }
 

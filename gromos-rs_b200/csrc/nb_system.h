@@ -15,6 +15,10 @@ namespace gnb {
 struct WaterParams;
 struct WaterScaled;
 void set_error(const std::string& m);
+cudaError_t pinned_alloc(void** out, size_t n);
+void pinned_free(void* p, size_t n);
+cudaError_t pool_malloc(void** p, size_t n, cudaStream_t s);
+void pool_free(void* p, cudaStream_t s);
 void crf_params(double cutoff, double epsilon, double rf_epsilon, double rf_kappa, double out[4]);
 void lambda_params(double lam, int n, double lp[17]);
 
@@ -32,6 +36,7 @@ class NbSystem {
     gr_status eval_graph(cudaStream_t s, int flags);
     void drop_graphs();
     gr_status download(cudaStream_t s, gr_result* out);
+    gr_status energy_buffer();
     gr_status pair_counts(cudaStream_t s, long long* n_short, long long* n_long);
     gr_status push_descriptor(cudaStream_t s);
     cudaError_t dev_malloc(void** p, size_t n);

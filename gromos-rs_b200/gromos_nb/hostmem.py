@@ -1,0 +1,113 @@
+"""Result arrays in recycled page-locked memory.
+
+A download into ordinary memory is staged by the driver, and a result array
+of a few MB is fresh memory from the operating system on every call, so each of
+its pages is faulted in on the way: reading 90,000 positions and velocities
+took 1.4 ms, of which the transfer is 0.1.  :func:`empty` returns arrays whose
+memory is page-locked and goes back to a pool when the array (and every view
+of it) is gone.  Live and pooled blocks together stay within
+:data:`LIMIT` bytes; beyond that, and for small arrays, it returns ordinary
+arrays.  Safe with several threads: a block has one owner at a time.
+"""
+from __future__ import annotations
+
+import ctypes as C
+import threading
+from collections import deque
+from typing import Dict, List
+
+import numpy as np
+
+from . import _lib
+
+LIMIT = 512 << 20          # bytes of page-locked memory held at most, in use or pooled
+SMALLEST = 8 << 10        # smaller arrays gain nothing
+
+ARENA = 8 << 20            # blocks of one size are cut from arenas of about this many bytes
+
+_lock = threading.Lock()
+_free: Dict[int, List[tuple]] = {}  # block size -> (address, arena)
+_held = 0                           # bytes of all arenas
+_returned: deque = deque()          # (block size, (address, arena)) of arrays that are gone
+
+
+class _Arena:
+    """One page-locked allocation cut into blocks of one size."""
+
+    def __init__(self, address: int, size: int, blocks: int):
+        self.address, self.size, self.blocks, self.idle = address, size, blocks, 0
+
+
+class _Block:
+    """One page-locked block, the base of the array over it."""
+
+    def __init__(self, place: tuple, size: int, shape):
+        self._place, self._size = place, size
+        self.__array_interface__ = {"data": (place[0], False), "shape": tuple(shape), "typestr": "<f8", "version": 3}
+
+    def __del__(self):
+        _returned.append((self._size, self._place))  # no lock: this may run inside any allocation
+
+
+def _drain() -> None:
+    while _returned:
+        size, place = _returned.popleft()
+        _free.setdefault(size, []).append(place)
+        place[1].idle += 1
+
+
+def _pop(size: int):
+    place = _free[size].pop()
+    place[1].idle -= 1
+    return place
+
+
+def _take(size: int):
+    """A block of `size` bytes, or None when the limit is reached."""
+    global _held
+    n = max(1, min(ARENA // size, 64))
+    with _lock:
+        _drain()
+        if _free.get(size):
+            return _pop(size)
+        full = _held + n * size > LIMIT
+    if full:
+        release()          # idle arenas of other sizes make room
+    with _lock:
+        if _held + n * size > LIMIT:
+            return None
+        _held += n * size
+    p = C.c_void_p()
+    if _lib.lib().gr_host_alloc(n * size, C.byref(p)) != _lib.GR_OK:
+        with _lock:
+            _held -= n * size
+        return None
+    arena = _Arena(int(p.value), n * size, n)
+    with _lock:
+        arena.idle += n
+        _free.setdefault(size, []).extend((arena.address + k * size, arena) for k in range(n))
+        return _pop(size)
+
+
+def empty(shape) -> np.ndarray:
+    """An uninitialised C-contiguous float64 array for a download to fill."""
+    n = 8 * int(np.prod(shape))
+    if n >= SMALLEST:
+        size = -(-n // 4096) * 4096
+        place = _take(size)
+        if place is not None:
+            return np.asarray(_Block(place, size, shape))
+    return np.empty(shape)
+
+
+def release() -> None:
+    """Give back the arenas that no array uses."""
+    global _held
+    with _lock:
+        _drain()
+        idle = {p[1] for places in _free.values() for p in places if p[1].idle == p[1].blocks}
+        for size in list(_free):
+            _free[size] = [p for p in _free[size] if p[1] not in idle]
+        _held -= sum(a.size for a in idle)
+    for a in idle:
+        _lib.lib().gr_host_free(a.address)

@@ -20,11 +20,12 @@ from __future__ import annotations
 
 import ctypes as C
 import dataclasses
+import weakref
 from typing import Dict, List, Optional, Tuple
 
 import numpy as np
 
-from . import _lib
+from . import _lib, hostmem
 from ._lib import GromosNbError, check  # noqa: F401  (re-exported)
 from .system import NonbondedParams, System, Topology
 
@@ -177,7 +178,7 @@ class Forcefield:
                 raise ValueError("out must be a C-contiguous float64 (n_atoms, 3) array")
             f = out
         else:
-            f = np.zeros((self.n_atoms, 3)) if download_forces else None
+            f = hostmem.empty((self.n_atoms, 3)) if download_forces else None
         glj = np.zeros((self.G, self.G))
         gcrf = np.zeros((self.G, self.G))
         r = _lib.GrResult()
@@ -281,7 +282,7 @@ class Forcefield:
 
     def result(self) -> Dict:
         """Results of the last evaluation (e.g. after a batch evaluation), without evaluating."""
-        f = np.zeros((self.n_atoms, 3))
+        f = hostmem.empty((self.n_atoms, 3))
         glj = np.zeros((self.G, self.G))
         gcrf = np.zeros((self.G, self.G))
         r = _lib.GrResult()
@@ -318,8 +319,8 @@ class Forcefield:
         return self._h
 
     def md_state(self):
-        x = np.zeros((self.n_atoms, 3))
-        v = np.zeros((self.n_atoms, 3))
+        x = hostmem.empty((self.n_atoms, 3))
+        v = hostmem.empty((self.n_atoms, 3))
         check(self._L.gr_md_download(self._h, _p(x, C.c_double), _p(v, C.c_double)))
         return x, v
 
@@ -346,6 +347,7 @@ class Forcefield:
     def close(self) -> None:
         if getattr(self, "_h", None):
             batch = getattr(self, "_batch", None)
+            batch = batch() if batch is not None else None
             if batch is not None:  # a batch member leaves its batch first
                 batch.remove(self)
             check(self._L.gr_ctx_destroy(self._h))
@@ -383,7 +385,7 @@ class Batch:
     def add(self, ff: "Forcefield") -> None:
         check(self._L.gr_batch_add(self._h, ff.handle))
         self.members.append(ff)
-        ff._batch = self
+        ff._batch = weakref.ref(self)  # no cycle: a dropped batch and its members go at once
 
     def remove(self, ff: "Forcefield") -> None:
         check(self._L.gr_batch_remove(self._h, ff.handle))

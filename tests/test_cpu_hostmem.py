@@ -1,0 +1,91 @@
+"""CPU: the pool of page-locked result arrays, over a fake of the library's allocation calls."""
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+
+from gromos_nb import hostmem
+
+
+class FakeLib:
+    def __init__(self):
+        self.live = {}
+
+    def gr_host_alloc(self, n, out):
+        buf = C.create_string_buffer(int(n))
+        p = C.addressof(buf)
+        self.live[p] = (buf, int(n))
+        C.cast(out, C.POINTER(C.c_void_p))[0] = p
+        return 0
+
+    def gr_host_free(self, p):
+        del self.live[p]
+        return 0
+
+    def bytes(self):
+        return sum(n for _, n in self.live.values())
+
+
+@pytest.fixture
+def lib(monkeypatch):
+    fake = FakeLib()
+    monkeypatch.setattr(hostmem._lib, "lib", lambda: fake)
+    hostmem._free.clear()
+    hostmem._returned.clear()
+    hostmem._held = 0
+    yield fake
+    hostmem._free.clear()
+    hostmem._returned.clear()
+    hostmem._held = 0
+
+
+def test_memory_is_reused_after_every_view_is_gone(lib):
+    a = hostmem.empty((5000, 3))
+    a[:] = 7.0
+    at, view = a.ctypes.data, a[10:]
+    del a
+    b = hostmem.empty((5000, 3))
+    assert b.ctypes.data != at and (view == 7.0).all()   # the view still owns the block
+    del view
+    c = hostmem.empty((5000, 3))
+    assert c.ctypes.data == at and c.flags.c_contiguous and c.flags.writeable and c.dtype == np.float64
+    assert len(lib.live) == 1                             # one arena for the three
+
+
+def test_limit_and_release(lib, monkeypatch):
+    monkeypatch.setattr(hostmem, "LIMIT", 20 << 20)
+    keep = [hostmem.empty((1 << 20,)) for _ in range(4)]  # 8 MB each: the first two fit
+    assert lib.bytes() <= 20 << 20 and hostmem._held == lib.bytes()
+    for k, x in enumerate(keep):
+        x[:] = k                                          # the others are ordinary arrays
+    assert [x[0] for x in keep] == [0, 1, 2, 3]
+    del keep, x
+    y = hostmem.empty((1000, 3))                          # another size: idle arenas make room
+    assert lib.bytes() <= 20 << 20
+    hostmem.release()
+    assert len(lib.live) == 1                             # the arena of y stays
+    del y
+    hostmem.release()
+    assert not lib.live and hostmem._held == 0
+
+
+def test_small_arrays_are_ordinary(lib):
+    hostmem.empty((10, 3))[:] = 1.0
+    assert not lib.live
+
+
+def test_threads_never_share_a_block(lib):
+    bad = []
+
+    def work(tag):
+        for _ in range(300):
+            a, b = hostmem.empty((2000, 3)), hostmem.empty((2000, 3))
+            a[:], b[:] = tag, -tag
+            if (a != tag).any() or (b != -tag).any():
+                bad.append(tag)
+
+    ts = [threading.Thread(target=work, args=(k + 1,)) for k in range(6)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    assert not bad
