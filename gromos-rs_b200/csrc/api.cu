@@ -1018,8 +1018,21 @@ gr_status NbSystem::expand_cg_pairs(cudaStream_t s) {
     return GR_OK;
 }
 
+// Water records that the last MD step wrote for an evaluation that does not
+// use them (new positions, a rebuild, a recorded graph): their excluded
+// energies leave the accumulators.
+gr_status NbSystem::drop_prep(cudaStream_t s) {
+    if (!prep_in_acc) return GR_OK;
+    prep_in_acc = false;
+    GR_CUDA(cudaMemsetAsync(h.acc_short, 0, size_t(acc_size(G)) * sizeof(long long), s));
+    GR_CUDA(cudaMemsetAsync(h.max_delta, 0, sizeof(float), s));
+    return GR_OK;
+}
+
 // One Forcefield::apply, nonbonded part.
-gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events) {
+// Without `finalize` the caller's MD step kernel does k_finalize's work
+// (the fixed-point kernel only).
+gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events, bool finalize) {
     if (!uploaded || !params_set || !box_set || !pos_set) {
         set_error("gr_forces_eval before topology, parameters, box and positions are set");
         return GR_ERR_STATE;
@@ -1033,6 +1046,10 @@ gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events) {
     // lists, and so the slots, are kept); a recorded graph always holds the prep
     const bool prepped = prepped_next && !rebuild && !in_capture;
     prepped_next = false;
+    if (prepped)
+        prep_in_acc = false;
+    else if (!in_capture && (st = drop_prep(s)))
+        return st;
     // stage timing events are recorded kernel by kernel only: inside a recorded
     // graph each event node adds its own latency to the step, so a graph holds
     // just the first and last (the step's total device time)
@@ -1136,8 +1153,10 @@ gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events) {
                                               s>>>(d_sys));
         (++launches, k_pert_terms<<<blocks_for(std::max(N, h.n_pp), 128), 128, sha, s>>>(d_sys));
     }
-    (++launches, k_finalize<<<blocks_for(std::max<long long>(3LL * N, NA), 256), 256, 0, s>>>(d_sys, prm.kernel == GR_KERNEL_PLAIN));
-    acc_clean = true;  // k_finalize leaves the short-range accumulators zero
+    if (finalize) {
+        (++launches, k_finalize<<<blocks_for(std::max<long long>(3LL * N, NA), 256), 256, 0, s>>>(d_sys, prm.kernel == GR_KERNEL_PLAIN));
+        acc_clean = true;  // k_finalize leaves the short-range accumulators zero
+    }
     if (prm.kernel == GR_KERNEL_PLAIN) (++launches, k_finalize_plain_energies<<<1, 32, 0, s>>>(d_sys));
     if (record_events) GR_CUDA(record_event(ev[4], s));
     GR_CUDA(cudaGetLastError());
@@ -1242,6 +1261,7 @@ gr_status NbSystem::eval_graph(cudaStream_t s, int flags) {
         g_gen = alloc_gen;
     }
     prepped_next = false;  // the graphs hold their own prep
+    if ((st = drop_prep(s))) return st;
     GR_CUDA(cudaGraphLaunch(g_step[rebuild ? 1 : 0], s));
     last_staged = false;
     GR_CUDA(cudaEventRecord(ev_step, s));

@@ -191,7 +191,7 @@ gr_status batch_capture_graphs(gr_batch* b) {
             S.built = true;
             S.lr_computed = true;
             S.pending_check = false;
-            st = S.eval(si, 0, false);
+            st = S.eval(si, 0, false, false);
             if (!st) st = S.md_step_launch(si);
             if (!st) e = cudaEventRecord(mb.join, si);
             if (!st && e == cudaSuccess) e = cudaStreamWaitEvent(b->s0, mb.join, 0);
@@ -261,6 +261,7 @@ gr_status batch_recover(gr_batch* b, gr_batch::Member& mb, int flags, int steps)
     gr_status st = S.md_run(si, steps, nullptr);
     S.prepped_next = false;  // the batch's step graphs write their own water records
     if (st) return st;
+    if ((st = S.drop_prep(si))) return st;
     S.md_steps_total -= steps;  // counted once, by the batch step that failed
     S.md_rollbacks += 1;
     GR_CUDA(cudaStreamSynchronize(si));
@@ -413,6 +414,12 @@ gr_status gr_batch_md_run(gr_batch* b, int32_t n_steps) {
     if (b->m.empty() || n_steps == 0) return GR_OK;
     gr_status st;
     if ((st = batch_prepare(b, true))) return st;
+    for (auto& mb : b->m) {  // the graphs write their own water records
+        NbSystem& S = mb.ctx->sys;
+        if (!S.prep_in_acc) continue;
+        if ((st = S.drop_prep(mb.ctx->stream))) return st;
+        GR_CUDA(cudaStreamSynchronize(mb.ctx->stream));
+    }
     float total_ms = 0.f;
     for (int k = 0; k < n_steps; ++k) {
         // a member reallocated since the graphs were recorded (parameters,

@@ -47,7 +47,7 @@ __device__ __forceinline__ void water_record(const SysDev& s, int slot, const do
     // descriptor fields first: the stores below go through pointers the
     // compiler cannot tell apart from the descriptor
     WaterRec* __restrict__ wrec = s.wrec;
-    long long* __restrict__ fs_short = s.fs_short;
+    long long* fs_short = s.fs_short;  // the MD step kernel reads the slot's sums before they are cleared here
     const uint32_t* __restrict__ wl_s = s.wl_s;
     const int W = s.W, wcap = s.wcap;
     const bool rect = s.boundary == 1;
@@ -881,8 +881,10 @@ __global__ void k_finalize(const SysDev* __restrict__ sys, int plain) {
             const int w = (a - nsa) / 3;
             const int slot = cg_slot[nscg + w];
             const int k = i - 3 * (nsa + 3 * w);
-            fx += fs_short[slot * 9 + k];
-            if (twin) fx += fs_long[slot * 9 + k];
+            if (slot >= 0) {  // (no slot: the build failed on this molecule's cell and reported it)
+                fx += fs_short[slot * 9 + k];
+                if (twin) fx += fs_long[slot * 9 + k];
+            }
         }
         double v = double(fx) * inv;
         if (plain) {

@@ -25,8 +25,9 @@ struct MdDev {
     double dt, dt_i;
     int settle;               // SETTLE every solvent molecule
     double m_o, m_h, ra, rb, rc;  // canonical SETTLE triangle (constraints.rs:836-840)
-    long long* ke;            // [3]: [0] kinetic energy of the velocities entering the step, [1] accumulator
-                              // of the velocities leaving it (fixed point 2^24), [2] blocks finished
+    long long* ke;            // [5]: [0] kinetic energy of the velocities entering the step, [1] accumulator
+                              // of the velocities leaving it (fixed point 2^24), [2] blocks finished,
+                              // [3] excluded energies and [4] largest extent of the next step's records
     int* failures;            // [1] molecules SETTLE could not solve
     const double* t0;         // [1] Berendsen bath temperature (device memory: a replica exchange changes it
                               // without touching recorded graphs)
@@ -123,81 +124,183 @@ __device__ bool settle_molecule(const D3 old[3], D3 nw[3], D3 v[3], const MdDev&
 }
 
 // One thread per unit: a solute atom (leap-frog only) or a solvent molecule
-// (leap-frog of its atoms, then SETTLE).  Forces are the finalized FP64
-// forces of this step's evaluation.  With prep_next the kernel also does the
-// next evaluation's k_water_prep for each molecule from its new coordinates
-// (same record, same cleared force sums, same excluded energies and extent;
-// the slots are those of the current lists, so only when the next step keeps
-// them): the next evaluation then skips k_water_prep.
-__global__ void k_md_step(const SysDev* __restrict__ sys, MdDev md) {
-    // descriptor pointers in registers and every load of a unit before its
-    // stores (stores through descriptor pointers would otherwise order the
-    // later reads behind them)
-    const SysDev& s = *sys;
-    const int nsa = s.n_solute_atoms, n = s.n_atoms, nscg = s.n_solute_cg;
-    const double* __restrict__ f_out = s.f_out;
-    double* __restrict__ pos = s.pos;
-    const int* __restrict__ cg_slot = s.cg_slot;
-    const double* __restrict__ charge = s.charge;
-    const bool excl = s.excl_atoms < n;
-    const int n_mol = md.settle ? (n - nsa) / 3 : 0;
-    const int n_units = md.settle ? nsa + n_mol : n;
-    const double lambda = berendsen_lambda(md);
-    long long ke = 0;
-    double e_excl = 0.0;
-    float m_ext = 0.f;
-    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < n_units; u += gridDim.x * blockDim.x) {
-        const bool mol = md.settle && u >= nsa;
-        const int a0 = mol ? nsa + 3 * (u - nsa) : u;
-        const int na = mol ? 3 : 1;
-        const bool rec = mol && md.prep_next;
-        const int slot = rec ? cg_slot[nscg + (u - nsa)] : -1;
-        double q3[3] = {0.0, 0.0, 0.0};
-        if (rec && excl)
+// (leap-frog of its atoms, then SETTLE).
+//
+// FUSED (the fixed-point kernel): the step is also its evaluation's k_finalize.
+// Each unit takes its forces from the fixed-point sums, writes the FP64
+// forces, clears what it read and moves on with them; the last block to finish
+// does the energies and the counters.  Separately the two kernels cost a launch
+// and two latencies per step, which is most of them for a few thousand waters
+// (1,000: 12.6 + 4.7 us, fused 12.4, ncu; 20 steps 1,328 -> 1,240 us).
+// Without it (the plain kernel) the forces are those that k_finalize wrote.
+//
+// With prep_next the kernel also does the next evaluation's k_water_prep for
+// each molecule from its new coordinates (same record, same cleared force
+// sums, same excluded energies and extent; the slots are those of the current
+// lists, so only when the next step keeps them): the next evaluation then
+// skips k_water_prep.  Their energies and extent wait in ke[3] and ke[4] until
+// the last block has read this step's accumulators.
+struct MdUnit {
+    long long ke;
+    double e_excl;
+    float m_ext;
+};
+
+// Forces of atom a: the fixed-point sums (cleared where nothing else clears
+// them) or the finalized ones.  `sl` are the water's short and long slot sums
+// of its first component, null for solute atoms.
+template <bool FUSED>
+__device__ __forceinline__ D3 md_force(const SysDev& s, double* __restrict__ f_out, int a, const long long* ws,
+                                       const long long* wl, bool pa, bool twin) {
+    if (!FUSED) return d3(f_out[3 * a], f_out[3 * a + 1], f_out[3 * a + 2]);
+    long long f[3] = {0, 0, 0};
+    if (pa) {
 #pragma unroll
-            for (int a = 0; a < 3; ++a) q3[a] = charge[a0 + a];
-        D3 old[3], nw[3], v[3];
-        double mass[3];
-        for (int k = 0; k < na; ++k) {
-            const int i = a0 + k;
-            const D3 f = d3(f_out[3 * i], f_out[3 * i + 1], f_out[3 * i + 2]);
-            const double im = md.inv_mass[i];
-            mass[k] = md.mass[i];
-            v[k] = (d3(md.vel[3 * i], md.vel[3 * i + 1], md.vel[3 * i + 2]) + f * im * md.dt) * lambda;
-            old[k] = d3(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]);
-            nw[k] = old[k] + v[k] * md.dt;
-        }
-        if (mol && !settle_molecule(old, nw, v, md)) atomicAdd(md.failures, 1);
-        if (rec && slot >= 0) {
-            const double p[9] = {nw[0].x, nw[0].y, nw[0].z, nw[1].x, nw[1].y, nw[1].z, nw[2].x, nw[2].y, nw[2].z};
-            water_record(s, slot, p, q3, excl, e_excl, m_ext);
-        }
-        for (int k = 0; k < na; ++k) {
-            const int i = a0 + k;
-            pos[3 * i] = nw[k].x;
-            pos[3 * i + 1] = nw[k].y;
-            pos[3 * i + 2] = nw[k].z;
-            md.vel[3 * i] = v[k].x;
-            md.vel[3 * i + 1] = v[k].y;
-            md.vel[3 * i + 2] = v[k].z;
-            ke += to_fixed_d(0.5 * mass[k] * dot3(v[k], v[k]), kEnergyScale);
+        for (int k = 0; k < 3; ++k) {
+            f[k] = s.f_short[3 * a + k];
+            if (twin) f[k] += s.f_long[3 * a + k];
         }
     }
-    if (md.prep_next) water_record_flush(s, m_ext, e_excl, excl);  // block-uniform
-    ke = warp_sum_ll(ke);
-    if ((threadIdx.x & 31) == 0 && ke) atomicAdd(reinterpret_cast<unsigned long long*>(md.ke + 1),
-                                                  static_cast<unsigned long long>(ke));
+    if (ws) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            f[k] += ws[k];
+            if (twin) f[k] += wl[k];
+        }
+    }
+    const double inv = 1.0 / kForceScale;
+    return d3(double(f[0]) * inv, double(f[1]) * inv, double(f[2]) * inv);
+}
+
+template <bool FUSED>
+__device__ __forceinline__ void md_store(const SysDev& s, const MdDev& md, double* __restrict__ f_out, int a, D3 f, D3 x,
+                                         D3 v, double mass, bool pa, long long& ke) {
+    if (FUSED) {
+        f_out[3 * a] = f.x;
+        f_out[3 * a + 1] = f.y;
+        f_out[3 * a + 2] = f.z;
+        if (pa) s.f_short[3 * a] = s.f_short[3 * a + 1] = s.f_short[3 * a + 2] = 0;
+    }
+    s.pos[3 * a] = x.x;
+    s.pos[3 * a + 1] = x.y;
+    s.pos[3 * a + 2] = x.z;
+    md.vel[3 * a] = v.x;
+    md.vel[3 * a + 1] = v.y;
+    md.vel[3 * a + 2] = v.z;
+    ke += to_fixed_d(0.5 * mass * dot3(v, v), kEnergyScale);
+}
+
+// NA atoms from a0 (1: an atom, 3: a molecule that SETTLE constrains).
+template <bool FUSED, int NA>
+__device__ __forceinline__ void md_unit(const SysDev& s, const MdDev& md, int a0, double lambda, MdUnit& r) {
+    double* __restrict__ f_out = s.f_out;
+    const int nsa = s.n_solute_atoms, nscg = s.n_solute_cg;
+    const bool twin = s.twin != 0, water = a0 >= nsa;
+    // a water atom's per-atom sums hold something only when solute kernels,
+    // excluded pairs or perturbation terms reach water atoms (as in k_finalize)
+    const bool pa = !water || nscg > 0 || s.excl_atoms > nsa || s.n_pert > 0 || s.n_pp > 0;
+    const bool rec = NA == 3 && md.prep_next;
+    const int w = water ? (a0 - nsa) / 3 : 0;
+    const int slot = water && (FUSED || rec) ? s.cg_slot[nscg + w] : -1;
+    const long long *ws = nullptr, *wl = nullptr;
+    if (FUSED && slot >= 0) {
+        const size_t o = static_cast<size_t>(slot) * 9 + 3 * (a0 - nsa - 3 * w);
+        ws = s.fs_short + o;
+        wl = s.fs_long + o;
+    }
+    const bool excl = s.excl_atoms < s.n_atoms;
+    double q3[3] = {0.0, 0.0, 0.0};
+    D3 f[NA], old[NA], nw[NA], v[NA];
+    double mass[NA];
+#pragma unroll
+    for (int k = 0; k < NA; ++k) {
+        const int i = a0 + k;
+        f[k] = md_force<FUSED>(s, f_out, i, ws ? ws + 3 * k : nullptr, wl ? wl + 3 * k : nullptr, pa, twin);
+        if (rec && excl) q3[k] = s.charge[i];
+        const double im = md.inv_mass[i];
+        mass[k] = md.mass[i];
+        v[k] = (d3(md.vel[3 * i], md.vel[3 * i + 1], md.vel[3 * i + 2]) + f[k] * im * md.dt) * lambda;
+        old[k] = d3(s.pos[3 * i], s.pos[3 * i + 1], s.pos[3 * i + 2]);
+        nw[k] = old[k] + v[k] * md.dt;
+    }
+    if constexpr (NA == 3) {
+        if (!settle_molecule(old, nw, v, md)) atomicAdd(md.failures, 1);
+        if (rec && slot >= 0) {
+            const double p[9] = {nw[0].x, nw[0].y, nw[0].z, nw[1].x, nw[1].y, nw[1].z, nw[2].x, nw[2].y, nw[2].z};
+            water_record(s, slot, p, q3, excl, r.e_excl, r.m_ext);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < NA; ++k) md_store<FUSED>(s, md, f_out, a0 + k, f[k], nw[k], v[k], mass[k], pa, r.ke);
+}
+
+template <bool FUSED>
+__global__ void __launch_bounds__(128) k_md_step(const SysDev* __restrict__ sys, MdDev md) {
+    const SysDev& s = *sys;
+    const int nsa = s.n_solute_atoms, n = s.n_atoms;
+    const int n_units = md.settle ? nsa + (n - nsa) / 3 : n;
+    const double lambda = berendsen_lambda(md);
+    MdUnit r{0, 0.0, 0.f};
+    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < n_units; u += gridDim.x * blockDim.x) {
+        if (md.settle && u >= nsa)
+            md_unit<FUSED, 3>(s, md, nsa + 3 * (u - nsa), lambda, r);
+        else
+            md_unit<FUSED, 1>(s, md, u, lambda, r);
+    }
+    // per-block sums: kinetic energy, the records' energies and extent
+    __shared__ unsigned long long sh[2];
+    __shared__ int mx, last;
+    if (threadIdx.x == 0) {
+        sh[0] = sh[1] = 0ull;
+        mx = 0;
+    }
+    __syncthreads();
+    const long long ke = warp_sum_ll(r.ke);
+    if ((threadIdx.x & 31) == 0 && ke) atomicAdd(&sh[0], static_cast<unsigned long long>(ke));
+    if (md.prep_next) {
+        const long long ex = warp_sum_ll(to_fixed_d(r.e_excl, kEnergyScale));
+        const int m = __reduce_max_sync(0xffffffffu, __float_as_int(r.m_ext));  // extents are >= 0: ordered as ints
+        if ((threadIdx.x & 31) == 0) {
+            if (ex) atomicAdd(&sh[1], static_cast<unsigned long long>(ex));
+            if (m) atomicMax(&mx, m);
+        }
+    }
+    __syncthreads();
+    unsigned long long* acc = reinterpret_cast<unsigned long long*>(md.ke);
+    if (threadIdx.x == 0) {
+        if (sh[0]) atomicAdd(acc + 1, sh[0]);
+        if (sh[1]) atomicAdd(acc + 3, sh[1]);
+        if (mx) atomicMax(reinterpret_cast<int*>(acc + 4), mx);
+        __threadfence();
+        last = atomicAdd(acc + 2, 1ull) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
     // The last block to finish makes the accumulated kinetic energy the next
-    // step's input (every block read ke[0] for its bath factor before adding).
-    __shared__ int last;
+    // step's input (every block read ke[0] for its bath factor before adding),
+    // and finalizes the step's energies.
     __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0)
-        last = atomicAdd(reinterpret_cast<unsigned long long*>(md.ke + 2), 1ull) == gridDim.x - 1;
-    __syncthreads();
-    if (last && threadIdx.x == 0) {
-        md.ke[0] = static_cast<long long>(atomicExch(reinterpret_cast<unsigned long long*>(md.ke + 1), 0ull));
-        md.ke[2] = 0;
+    const int G = s.n_egroups, gs = s.solvent_group < 0 ? 0 : s.solvent_group;
+    const int i_excl = G * G + gs * G + gs;
+    const long long next_excl = md.prep_next ? static_cast<long long>(__ldcg(acc + 3)) : 0ll;
+    if (FUSED) {
+        for (int i = threadIdx.x; i < acc_size(G); i += blockDim.x) {
+            double e = double(s.acc_short[i]) / kEnergyScale;
+            if (s.twin) e += double(s.acc_long[i]) / kEnergyScale;
+            s.e_out[i] = e;
+            s.acc_short[i] = i == i_excl ? next_excl : 0ll;
+        }
+    } else if (threadIdx.x == 0 && next_excl) {
+        s.acc_short[i_excl] += next_excl;
+    }
+    __syncthreads();  // next_excl read by every thread
+    if (threadIdx.x == 0) {
+        md.ke[0] = static_cast<long long>(__ldcg(acc + 1));
+        const int m = __ldcg(reinterpret_cast<int*>(acc + 4));
+        if (s.max_delta) *s.max_delta = md.prep_next ? __int_as_float(m) : 0.f;
+        md.ke[1] = md.ke[2] = md.ke[3] = md.ke[4] = 0;
+        if (FUSED)
+            for (int k = 0; k < 6; ++k) s.n_deferred[k] = 0;
     }
 }
 
@@ -247,7 +350,7 @@ gr_status NbSystem::md_init(const double* mass, const double* vel, const gr_md_p
     gr_status st;
     if ((st = upload_array(&md_mass, mass, N)) || (st = upload_array(&md_inv_mass, inv.data(), N)) ||
         (st = upload_array(&md_vel, v0.data(), size_t(N) * 3)) || (st = alloc(&md_pos_snap, size_t(N) * 3)) ||
-        (st = alloc(&md_vel_snap, size_t(N) * 3)) || (st = alloc(&md_ke, 3)) || (st = alloc(&md_ke_snap, 1)) ||
+        (st = alloc(&md_vel_snap, size_t(N) * 3)) || (st = alloc(&md_ke, 5)) || (st = alloc(&md_ke_snap, 1)) ||
         (st = alloc(&md_psnap_pos, size_t(N) * 3)) || (st = alloc(&md_psnap_vel, size_t(N) * 3)) ||
         (st = alloc(&md_psnap_ke, 1)) || (st = alloc(&md_fail, 1)) || (st = alloc(&md_t0, 1)))
         return st;
@@ -256,7 +359,7 @@ gr_status NbSystem::md_init(const double* mass, const double* vel, const gr_md_p
         double ke0 = 0.0;
         for (int i = 0; i < N; ++i)
             ke0 += 0.5 * mass[i] * (v0[3 * i] * v0[3 * i] + v0[3 * i + 1] * v0[3 * i + 1] + v0[3 * i + 2] * v0[3 * i + 2]);
-        const long long k[3] = {static_cast<long long>(std::llround(ke0 * kEnergyScale)), 0, 0};
+        const long long k[5] = {static_cast<long long>(std::llround(ke0 * kEnergyScale)), 0, 0, 0, 0};
         GR_CUDA(cudaMemcpy(md_ke, k, sizeof(k), cudaMemcpyHostToDevice));
     }
     GR_CUDA(cudaMemset(md_fail, 0, sizeof(int)));
@@ -285,7 +388,8 @@ gr_status NbSystem::md_init(const double* mass, const double* vel, const gr_md_p
     return GR_OK;
 }
 
-// Zeroes the kinetic-energy accumulator and launches one MD step kernel.
+// One MD step kernel: the finalization of the evaluation before it
+// (eval(..., false)) and the step itself.
 gr_status NbSystem::md_step_launch(cudaStream_t s, bool fuse_prep) {
     MdDev md;
     md.vel = md_vel;
@@ -308,10 +412,17 @@ gr_status NbSystem::md_step_launch(cudaStream_t s, bool fuse_prep) {
     // records come from this kernel
     md.prep_next = fuse_prep && md_settle && NCG > NSCG && h.wrec && !in_capture && built &&
                    steps_since_update < prm.nsnb;
-    prepped_next = md.prep_next != 0;
+    prepped_next = prep_in_acc = md.prep_next != 0;
     const int n_units = md_settle ? NSA + (N - NSA) / 3 : N;
-    const unsigned grid = std::max(1u, std::min(unsigned((n_units + 255) / 256), unsigned(sm_count() * 8)));
-    (++launches, k_md_step<<<grid, 256, 0, s>>>(d_sys, md));
+    // a unit is one long FP64 chain: small blocks spread few units over more SMs
+    const unsigned bt = n_units <= 128 * sm_count() ? 64 : 128;
+    const unsigned grid = std::max(1u, std::min(unsigned((n_units + bt - 1) / bt), unsigned(sm_count() * 8)));
+    if (prm.kernel == GR_KERNEL_FIXED) {
+        (++launches, k_md_step<true><<<grid, bt, 0, s>>>(d_sys, md));
+        acc_clean = true;  // the step leaves the short-range accumulators zero
+    } else {
+        (++launches, k_md_step<false><<<grid, bt, 0, s>>>(d_sys, md));
+    }
     return GR_OK;
 }
 
@@ -398,7 +509,7 @@ gr_status NbSystem::md_run(cudaStream_t s, int n_steps, gr_md_stats* out) {
                     md_psnap_step = md_step_idx;
                     md_psnap_valid = true;
                 }
-                if ((st = eval(s, 0, false))) return st;
+                if ((st = eval(s, 0, false, prm.kernel != GR_KERNEL_FIXED))) return st;
                 if ((st = md_step_launch(s, true))) return st;
                 ++md_step_idx;
                 if (r < replay) {

@@ -32,7 +32,8 @@ class NbSystem {
     gr_status build_pairlist(cudaStream_t s, bool sync);
     gr_status resolve_pending(bool* overflowed);
     gr_status expand_cg_pairs(cudaStream_t s);
-    gr_status eval(cudaStream_t s, int flags, bool record_events);
+    gr_status eval(cudaStream_t s, int flags, bool record_events, bool finalize = true);
+    gr_status drop_prep(cudaStream_t s);
     gr_status eval_graph(cudaStream_t s, int flags);
     void drop_graphs();
     gr_status download(cudaStream_t s, gr_result* out);
@@ -133,6 +134,7 @@ class NbSystem {
     bool step_check = false;
     bool in_capture = false;  // recording a CUDA graph: the device descriptor is already current
     bool last_staged = false; // the last timed evaluation recorded its stage events (kernel by kernel)
+    bool prep_in_acc = false; // the accumulators hold the energies of water records written by the last MD step
     bool prepped_next = false; // the last MD step wrote this evaluation's water records (k_water_prep skipped)
 
    private:

@@ -1,0 +1,57 @@
+"""GPU: the MD step kernel that also finalizes its evaluation."""
+import numpy as np
+import pytest
+
+from gromos_nb import generators
+from gromos_nb.nonbonded import Forcefield
+
+pytestmark = pytest.mark.gpu
+
+
+def start(s, **kw):
+    ff = Forcefield(s)
+    ff.upload_positions(s.pos)
+    m = generators.masses(s)
+    ff.md_init(m, generators.maxwell_velocities(m, 300.0, 3), dist_hh=generators.SPC_DHH, **kw)
+    return ff
+
+
+def systems():
+    twin = generators.spc_water_system(700, generators.box_for_waters(700), 12, rcutp=0.8, rcutl=1.2)
+    return [twin, generators.solvated_solute_system(900, 40, seed=13, single_atom_cgs=True)]
+
+
+# units around a block (64) and several, with and without SETTLE, a solute, a twin range
+@pytest.mark.parametrize("k,settle", [(0, True), (0, False), (1, True), (1, False)])
+@pytest.mark.parametrize("steps", [1, 4, 6])
+def test_forces_and_energies_of_the_last_step(k, settle, steps):
+    """After md_run the context holds the last evaluation's results: those of evaluating its positions at
+    the same step of the same pairlist period."""
+    s = systems()[k]
+    ff, ref = start(s, settle=settle), start(s, settle=settle)
+    if steps > 1:
+        ff.md_run(steps - 1)
+        ref.md_run(steps - 1)
+    st = ff.md_run(1)
+    r = ff.result()
+    want = ref.apply(ref.md_state()[0])  # the same step of the same period, finalized by its own kernel
+    assert np.array_equal(r["forces"], want["forces"]) and np.array_equal(r["virial"], want["virial"])
+    assert r["e_lj"] == want["e_lj"] and r["e_crf"] == want["e_crf"]
+    assert st["e_lj"] + st["e_crf"] == pytest.approx(want["e_lj"] + want["e_crf"], rel=1e-12)
+    ff.close()
+    ref.close()
+
+
+def test_records_written_ahead_do_not_reach_another_evaluation():
+    """The step kernel writes the next step's water records; an evaluation of other positions, a graph
+    replay and a batch must not count their energies twice."""
+    s = systems()[0]
+    want = Forcefield(s).apply(s.pos)
+    for graph in (False, True):
+        ff = start(s)
+        for _ in range(2):
+            ff.apply(s.pos, graph=graph)
+        ff.md_run(2)  # inside a pairlist period: the next records are written
+        got = ff.apply(s.pos, force_rebuild=True, graph=graph)
+        assert got["e_crf"] == want["e_crf"] and np.array_equal(got["forces"], want["forces"])
+        ff.close()
