@@ -552,6 +552,14 @@ gr_status NbSystem::upload(const gr_topology* t) {
                 h.w_qq[a * 4 + b] = float(t->charge[f + a] * t->charge[f + b] * fpe);
                 if ((a || b) && (lj[0] != 0.0 || lj[1] != 0.0)) h.water_lj00_only = 0;
             }
+        h.solvent_uniform = 1;
+        for (int a = 0; a < aps; ++a) {
+            h.w_iac[a] = t->iac[f + a];
+            h.w_q[a] = float(t->charge[f + a]);
+        }
+        for (int a = NSA; a < N && h.solvent_uniform; ++a)
+            if (t->iac[a] != t->iac[f + (a - f) % aps] || t->charge[a] != t->charge[f + (a - f) % aps])
+                h.solvent_uniform = 0;
         double qs = 0.0;  // sum of the charges of one solvent molecule (zero for a neutral one)
         for (int a = 0; a < aps; ++a) qs += t->charge[f + a];
         w_qq_sum = qs * qs * fpe;
@@ -568,7 +576,8 @@ gr_status NbSystem::upload(const gr_topology* t) {
     if ((st = alloc(&h.cg_spos, size_t(NCG)))) return st;
     if ((st = alloc(&h.cg_slot, size_t(NCG)))) return st;
     if ((st = alloc(&h.n_clusters, 1))) return st;
-    if ((st = alloc(&h.sn, size_t(std::max(NSCG, 1))))) return st;
+    if ((st = alloc(&h.sn, 2 * size_t(std::max(NSCG, 1))))) return st;
+    if ((st = alloc(&h.sn_max, 2))) return st;
     if ((st = alloc(&h.n_pert_pairs, 1))) return st;
     if ((st = alloc(&h.n_cgp, 2))) return st;
     if ((st = alloc(&h.pos32, size_t(N)))) return st;
@@ -1104,7 +1113,7 @@ gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events, bool fin
             if (stage) GR_CUDA(record_event(evk[1], s));
         }
         // solute work items: (CG, chunk of list entries), 4 warps per block
-        const unsigned sgrid = std::max(1u, std::min(blocks_for((long long)NSCG * ((h.scap + kSoluteChunk - 1) / kSoluteChunk), 4),
+        const unsigned sgrid = std::max(1u, std::min(blocks_for((long long)NSCG * ((h.scap - 1) / solute_chunk(h.twin != 0) + 1), 4),
                                                      unsigned(sm * 8)));
         if (NSCG > 0) (++launches, k_solute_force<false><<<sgrid, 128, shg, s>>>(d_sys));
         if (stage) GR_CUDA(record_event(ev[2], s));

@@ -169,37 +169,52 @@ __device__ __forceinline__ void block_flush(long long (&acc)[NV], long long* __r
 }
 
 // ---------------------------------------------------------------------------
-// Pair vector for solute pairs: CG shift (cg_grouped short) or per-atom image.
-__device__ __forceinline__ void solute_pair_vector(const SysDev& s, bool per_atom, int ai, int aj,
-                                                   float Dx, float Dy, float Dz, float dix, float diy,
-                                                   float diz, float djx, float djy, float djz,
-                                                   float& rx, float& ry, float& rz) {
-    rx = (Dx + dix) - djx;
-    ry = (Dy + diy) - djy;
-    rz = (Dz + diz) - djz;
-    if (per_atom && s.boundary) {
-        const float m = 1e-4f;
-        if (!(fabsf(rx) < s.half_boxf[0] - m && fabsf(ry) < s.half_boxf[1] - m && fabsf(rz) < s.half_boxf[2] - m)) {
-            double x, y, z;
-            nearest_image_exact(s, s.pos[3 * ai], s.pos[3 * ai + 1], s.pos[3 * ai + 2], s.pos[3 * aj],
-                                s.pos[3 * aj + 1], s.pos[3 * aj + 2], x, y, z);
-            rx = float(x);
-            ry = float(y);
-            rz = float(z);
-        }
+// Adds a warp's fixed-point (LJ, CRF) energies to the block's group sums, one
+// value pair per lane under its group slot (-1: none).  Lanes of one slot, the
+// common case, are summed by shuffles: 32 lanes adding to one 64-bit shared
+// word retry one after the other.
+__device__ __forceinline__ void warp_add_energies(unsigned long long* sh, int G, int sl, long long el, long long ec) {
+    const int lead = __reduce_max_sync(0xffffffffu, sl);
+    if (lead < 0) return;
+    if (__all_sync(0xffffffffu, sl == lead || sl < 0)) {
+        el = warp_sum_ll(el);
+        ec = warp_sum_ll(ec);
+        if ((threadIdx.x & 31) != 0) return;
+        sl = lead;
     }
+    if (el) atomicAdd(&sh[sl], static_cast<unsigned long long>(el));
+    if (ec) atomicAdd(&sh[G * G + sl], static_cast<unsigned long long>(ec));
 }
 
-// Solute CG pairs (solute-solute, solute-solvent, intra-CG).  One warp per
-// solute CG i, one lane per j entry.  Entries of the other range are skipped.
-// Work items are (solute CG, chunk of kSoluteChunk list entries): a CG's list
-// is spread over several warps, each adding its share of the CG's forces with
-// fixed-point reductions.  Group energies are summed per lane in FP32 for the
-// current energy-group slot and the virial per lane in FP32; both go to
-// fixed point when the slot changes and at the end of every item, so every
-// FP32 sum covers pairs of one item only and the results do not depend on
-// the grid or on which warp took which item.
-constexpr int kSoluteChunk = 64;
+// Solute CG pairs (solute-solute, solute-solvent, intra-CG) of one range: the
+// short entries fill a CG's list from the front, the long ones from the back.
+// Work items are (solute CG, 64 or 32 of its entries), one warp per item and one
+// lane per entry, so a CG's list is spread over many warps, each adding its
+// share of the CG's forces with fixed-point reductions; sn_max bounds the
+// items, so no warp walks the unused capacity of the lists.  Group energies
+// and the virial are summed per lane in FP32 within one item and taken to
+// fixed point at its end (energies also when the group slot changes), so the
+// results do not depend on the grid or on which warp took which item.
+//
+// The kernel is bound by the latency of an item's dependent loads, not by its
+// arithmetic, so an entry of the solvent (uniform solvent: every molecule has
+// the first one's types and charges) needs one level of them after the list:
+// the molecule's nine coordinates, at an address the index gives.  Its
+// charges come from the descriptor, the CG's LJ rows against the three
+// solvent sites and its own atoms from shared memory, once per item.  The
+// second round's molecule is loaded while the first one is computed.  200 ions in
+// 3,000 waters: 32 us before, 25 now (ncu); replica exchange of eight systems of
+// 1,500 waters and 200 ions 1.23x as fast.
+
+// With a twin range the two lists are short and an item is one round of 32, else
+// a system of few solute CGs has fewer items than the chip has warps.
+__host__ __device__ constexpr int solute_chunk(bool twin) { return twin ? 32 : 64; }
+
+struct SoluteWarp {
+    float4 at[kMaxCGAtoms];      // i atoms: offset from the CG's first atom, charge x fpe
+    int2 tg[kMaxCGAtoms];        // LJ row (type x n_types), energy group
+    float4 lj[kMaxCGAtoms * 3];  // c6, c12, 6 c6, 12 c12 against solvent site b at 3 a + b
+};
 
 template <bool LONG>
 __global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__ sys) {
@@ -209,123 +224,204 @@ __global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__
     const int G = s.n_egroups;
     long long* __restrict__ F = LONG ? s.f_long : s.f_short;
     extern __shared__ unsigned long long shg[];  // 2*G*G group energies (fixed)
+    __shared__ SoluteWarp sw_all[4];
+    SoluteWarp& sw = sw_all[threadIdx.x >> 5];
     for (int v = threadIdx.x; v < 2 * G * G; v += blockDim.x) shg[v] = 0ull;
     __syncthreads();
+    const double* __restrict__ pos = s.pos;
+    const int* __restrict__ cg_off = s.cg_off;
+    const int* __restrict__ iac = s.iac;
+    const double* __restrict__ charge = s.charge;
+    const int* __restrict__ egroup = s.egroup;
+    const int nsa = s.n_solute_atoms, nscg = s.n_solute_cg, scap = s.scap, n_types = s.n_types;
+    const bool uniform = s.solvent_uniform != 0;
+    const bool per_atom = LONG || !s.cg_grouped;
+    const float crf2 = s.crf_2cut3i_f, crfc = s.crf_cut_f, crf3 = s.crf_cut3i_f;
     float v6[6] = {0, 0, 0, 0, 0, 0};
     long long vfix[6] = {0, 0, 0, 0, 0, 0};
     int cur_slot = -1;
     float e_lj = 0.f, e_cr = 0.f;
-    auto flush_slot = [&]() {
+    auto to_slot = [&](int sl) {
+        if (sl == cur_slot) return;
         if (cur_slot >= 0) {
             const long long fl = to_fixed_f(e_lj, kE), fc = to_fixed_f(e_cr, kE);
             if (fl) atomicAdd(&shg[cur_slot], static_cast<unsigned long long>(fl));
             if (fc) atomicAdd(&shg[G * G + cur_slot], static_cast<unsigned long long>(fc));
         }
         e_lj = e_cr = 0.f;
+        cur_slot = sl;
     };
-    const int per = (s.scap + kSoluteChunk - 1) / kSoluteChunk;
-    const int nitems = s.n_solute_cg * per;
+    const int chunk = solute_chunk(s.twin != 0);
+    const int nitems = nscg * ((s.sn_max[LONG ? 1 : 0] + chunk - 1) / chunk);
     for (int it = blockIdx.x * wpb + (threadIdx.x >> 5); it < nitems; it += gridDim.x * wpb) {
-        const int ci = it / per;
-        const int e_beg = (it - ci * per) * kSoluteChunk;
-        const int cnt = min(s.sn[ci], e_beg + kSoluteChunk);
+        const int ci = it % nscg, e_beg = (it / nscg) * chunk;
+        const int cnt = min(s.sn[2 * ci + (LONG ? 1 : 0)], e_beg + chunk);
         if (e_beg >= cnt) continue;  // warp-uniform
-        const int i0 = s.cg_off[ci], ni = s.cg_off[ci + 1] - i0;
-        const double xi0 = s.pos[3 * i0], yi0 = s.pos[3 * i0 + 1], zi0 = s.pos[3 * i0 + 2];
-        float dix[kMaxCGAtoms], diy[kMaxCGAtoms], diz[kMaxCGAtoms];
-        float fix[kMaxCGAtoms], fiy[kMaxCGAtoms], fiz[kMaxCGAtoms];
+        // entry e of the CG's list of this range
+        const size_t l0 = static_cast<size_t>(ci) * scap + (LONG ? scap - 1 : 0);
+        auto place = [&](int e) { return LONG ? l0 - e : l0 + e; };
+        int entry = e_beg + lane < cnt ? s.sl[place(e_beg + lane)] : -1;
+        int entry_n = e_beg + 32 + lane < cnt ? s.sl[place(e_beg + 32 + lane)] : -1;  // (cnt ends the item)
+        double p[9];
+        auto load_solvent = [&](int entry_l) {
+            if (entry_l >= 0 && (entry_l >> 1) >= nscg && uniform) {
+                const double* __restrict__ pj = pos + 3 * static_cast<size_t>(nsa + 3 * ((entry_l >> 1) - nscg));
 #pragma unroll
-        for (int a = 0; a < kMaxCGAtoms; ++a) {
-            fix[a] = fiy[a] = fiz[a] = 0.f;
-            if (a < ni) {
-                dix[a] = float(s.pos[3 * (i0 + a)] - xi0);
-                diy[a] = float(s.pos[3 * (i0 + a) + 1] - yi0);
-                diz[a] = float(s.pos[3 * (i0 + a) + 2] - zi0);
-            } else {
-                dix[a] = diy[a] = diz[a] = 0.f;
+                for (int k = 0; k < 9; ++k) p[k] = pj[k];
+            }
+        };
+        load_solvent(entry);
+        const int i0 = cg_off[ci], ni = cg_off[ci + 1] - i0;
+        double px = 0.0, py = 0.0, pz = 0.0;
+        int ti = 0;
+        if (lane < ni) {
+            const int a = i0 + lane;
+            px = pos[3 * a];
+            py = pos[3 * a + 1];
+            pz = pos[3 * a + 2];
+            ti = iac[a] * n_types;
+        }
+        const double xi0 = __shfl_sync(0xffffffffu, px, 0), yi0 = __shfl_sync(0xffffffffu, py, 0);
+        const double zi0 = __shfl_sync(0xffffffffu, pz, 0);
+        __syncwarp();  // the previous item's reads are done
+        if (lane < ni) {
+            sw.at[lane] = make_float4(float(px - xi0), float(py - yi0), float(pz - zi0),
+                                      float(charge[i0 + lane] * s.fpe));
+            sw.tg[lane] = make_int2(ti, egroup[i0 + lane]);
+        }
+        if (uniform) {
+            const int row = __shfl_sync(0xffffffffu, ti, lane / 3);
+            if (lane < 3 * ni) {
+                const float2 c = s.lj32[row + s.w_iac[lane % 3]];
+                sw.lj[lane] = make_float4(c.x, c.y, 6.f * c.x, 12.f * c.y);
             }
         }
-        const int* __restrict__ list = s.sl + static_cast<size_t>(ci) * s.scap;
-        const unsigned long long* __restrict__ xl = s.sl_excl + static_cast<size_t>(ci) * s.scap;
-        for (int e0 = e_beg; e0 < cnt; e0 += 32) {
-            const int e = e0 + lane;
-            int entry = e < cnt ? list[e] : -1;
-            if (entry >= 0 && (entry & 1) != (LONG ? 1 : 0)) entry = -1;
-            if (entry < 0) continue;
-            const int cj = entry >> 1;
-            const unsigned long long xm = xl[e];
-            const int j0 = s.cg_off[cj], nj = s.cg_off[cj + 1] - j0;
-            const bool per_atom = LONG || !s.cg_grouped;
-            double dx, dy, dz;
-            nearest_image_exact(s, xi0, yi0, zi0, s.pos[3 * j0], s.pos[3 * j0 + 1], s.pos[3 * j0 + 2], dx, dy, dz);
-            const float Dx = float(dx), Dy = float(dy), Dz = float(dz);
-            for (int b = 0; b < nj; ++b) {
-                const int aj = j0 + b;
-                const float djx = float(s.pos[3 * aj] - s.pos[3 * j0]);
-                const float djy = float(s.pos[3 * aj + 1] - s.pos[3 * j0 + 1]);
-                const float djz = float(s.pos[3 * aj + 2] - s.pos[3 * j0 + 2]);
-                const int tj = s.iac[aj];
-                const float qj = float(s.charge[aj]);
-                const int gj = s.egroup[aj];
-                float gxs = 0.f, gys = 0.f, gzs = 0.f;
+        __syncwarp();
+        float fix[kMaxCGAtoms], fiy[kMaxCGAtoms], fiz[kMaxCGAtoms];
 #pragma unroll
-                for (int a = 0; a < kMaxCGAtoms; ++a) {
-                    if (a >= ni) break;
-                    if (xm & (1ull << (a * 8 + b))) continue;
+        for (int a = 0; a < kMaxCGAtoms; ++a) fix[a] = fiy[a] = fiz[a] = 0.f;
+        // one atom pair: i atom a, j atom at its offset (djx, djy, djz) from its CG's
+        // first atom, D the imaged vector between the first atoms; g the j force
+        auto pair = [&](int a, int aj, float Dx, float Dy, float Dz, float djx, float djy, float djz, float4 c, float qj,
+                        int gj, float& gx, float& gy, float& gz) {
+            const float4 pi = sw.at[a];
+            float x = (Dx + pi.x) - djx, y = (Dy + pi.y) - djy, z = (Dz + pi.z) - djz;
+            if (per_atom && s.boundary) {
+                const float m = 1e-4f;
+                if (!(fabsf(x) < s.half_boxf[0] - m && fabsf(y) < s.half_boxf[1] - m && fabsf(z) < s.half_boxf[2] - m)) {
                     const int ai = i0 + a;
-                    float x, y, z;
-                    solute_pair_vector(s, per_atom, ai, aj, Dx, Dy, Dz, dix[a], diy[a], diz[a], djx, djy, djz, x,
-                                       y, z);
-                    const float r2 = fmaf(x, x, fmaf(y, y, z * z));
-                    if (r2 < 1e-10f) continue;
-                    // one Newton step on the hardware reciprocal square root removes its
-                    // bias from the (cancelling) CRF energy sums of solute pairs
-                    float ri = rsqrtf(r2);
-                    ri = fmaf(0.5f * ri, fmaf(-r2 * ri, ri, 1.0f), ri);
-                    const float ri2 = ri * ri, ri6 = ri2 * ri2 * ri2;
-                    const float2 lj = s.lj32[s.iac[ai] * s.n_types + tj];
-                    const float q = float(s.charge[ai] * s.fpe) * qj;
-                    const float el = fmaf(lj.y, ri6, -lj.x) * ri6;
-                    const float ec = q * (fmaf(-s.crf_2cut3i_f, r2, ri) - s.crf_cut_f);
-                    const float fs = fmaf(fmaf(12.f * lj.y, ri6, -6.f * lj.x), ri6 * ri2, q * fmaf(ri, ri2, s.crf_cut3i_f));
-                    const float fxx = x * fs, fyy = y * fs, fzz = z * fs;
-                    fix[a] += fxx;
-                    fiy[a] += fyy;
-                    fiz[a] += fzz;
-                    gxs -= fxx;
-                    gys -= fyy;
-                    gzs -= fzz;
-                    v6[0] = fmaf(x, fxx, v6[0]);
-                    v6[1] = fmaf(x, fyy, v6[1]);
-                    v6[2] = fmaf(x, fzz, v6[2]);
-                    v6[3] = fmaf(y, fyy, v6[3]);
-                    v6[4] = fmaf(y, fzz, v6[4]);
-                    v6[5] = fmaf(z, fzz, v6[5]);
-                    const int sl = group_slot(G, s.egroup[ai], gj);
-                    if (sl != cur_slot) {
-                        flush_slot();
-                        cur_slot = sl;
-                    }
-                    e_lj += el;
-                    e_cr += ec;
+                    double dx, dy, dz;
+                    nearest_image_exact(s, pos[3 * ai], pos[3 * ai + 1], pos[3 * ai + 2], pos[3 * aj], pos[3 * aj + 1],
+                                        pos[3 * aj + 2], dx, dy, dz);
+                    x = float(dx);
+                    y = float(dy);
+                    z = float(dz);
                 }
-                red_add(&F[3 * aj], to_fixed_f(gxs, kF));
-                red_add(&F[3 * aj + 1], to_fixed_f(gys, kF));
-                red_add(&F[3 * aj + 2], to_fixed_f(gzs, kF));
             }
+            const float r2 = fmaf(x, x, fmaf(y, y, z * z));
+            if (r2 < 1e-10f) return;
+            // one Newton step on the hardware reciprocal square root removes its
+            // bias from the (cancelling) CRF energy sums of solute pairs
+            float ri = rsqrtf(r2);
+            ri = fmaf(0.5f * ri, fmaf(-r2 * ri, ri, 1.0f), ri);
+            const float ri2 = ri * ri, ri6 = ri2 * ri2 * ri2;
+            const float q = pi.w * qj;
+            to_slot(group_slot(G, sw.tg[a].y, gj));
+            e_lj += fmaf(c.y, ri6, -c.x) * ri6;
+            e_cr += q * (fmaf(-crf2, r2, ri) - crfc);
+            const float fs = fmaf(fmaf(c.w, ri6, -c.z), ri6 * ri2, q * fmaf(ri, ri2, crf3));
+            const float fxx = x * fs, fyy = y * fs, fzz = z * fs;
+            fix[a] += fxx;
+            fiy[a] += fyy;
+            fiz[a] += fzz;
+            gx -= fxx;
+            gy -= fyy;
+            gz -= fzz;
+            v6[0] = fmaf(x, fxx, v6[0]);
+            v6[1] = fmaf(x, fyy, v6[1]);
+            v6[2] = fmaf(x, fzz, v6[2]);
+            v6[3] = fmaf(y, fyy, v6[3]);
+            v6[4] = fmaf(y, fzz, v6[4]);
+            v6[5] = fmaf(z, fzz, v6[5]);
+        };
+        for (int e0 = e_beg; e0 < cnt; e0 += 32) {
+            const int cj = entry >> 1;
+            const bool solvent = entry >= 0 && cj >= nscg && uniform;
+            int j0 = 0;
+            float Dx = 0.f, Dy = 0.f, Dz = 0.f, dj[9];
+            if (solvent) {
+                j0 = nsa + 3 * (cj - nscg);
+                double dx, dy, dz;
+                nearest_image_exact(s, xi0, yi0, zi0, p[0], p[1], p[2], dx, dy, dz);
+                Dx = float(dx);
+                Dy = float(dy);
+                Dz = float(dz);
+#pragma unroll
+                for (int k = 0; k < 9; ++k) dj[k] = float(p[k] - p[k % 3]);
+            }
+            load_solvent(entry_n);
+            if (solvent) {
+                const int gj = s.solvent_group;
+                long long* __restrict__ Fj = F + 3 * static_cast<size_t>(j0);
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    float gx = 0.f, gy = 0.f, gz = 0.f;
+#pragma unroll
+                    for (int a = 0; a < kMaxCGAtoms; ++a) {
+                        if (a >= ni) break;
+                        pair(a, j0 + b, Dx, Dy, Dz, dj[3 * b], dj[3 * b + 1], dj[3 * b + 2], sw.lj[3 * a + b], s.w_q[b],
+                             gj, gx, gy, gz);
+                    }
+                    red_add(Fj + 3 * b, to_fixed_f(gx, kF));
+                    red_add(Fj + 3 * b + 1, to_fixed_f(gy, kF));
+                    red_add(Fj + 3 * b + 2, to_fixed_f(gz, kF));
+                }
+            } else if (entry >= 0) {
+                const unsigned long long xm = s.sl_excl[place(e0 + lane)];
+                j0 = cg_off[cj];
+                const int nj = cg_off[cj + 1] - j0;
+                double dx, dy, dz;
+                nearest_image_exact(s, xi0, yi0, zi0, pos[3 * j0], pos[3 * j0 + 1], pos[3 * j0 + 2], dx, dy, dz);
+                Dx = float(dx);
+                Dy = float(dy);
+                Dz = float(dz);
+                for (int b = 0; b < nj; ++b) {
+                    const int aj = j0 + b;
+                    const float djx = float(pos[3 * aj] - pos[3 * j0]);
+                    const float djy = float(pos[3 * aj + 1] - pos[3 * j0 + 1]);
+                    const float djz = float(pos[3 * aj + 2] - pos[3 * j0 + 2]);
+                    const int tj = iac[aj], gj = egroup[aj];
+                    const float qj = float(charge[aj]);
+                    float gx = 0.f, gy = 0.f, gz = 0.f;
+#pragma unroll
+                    for (int a = 0; a < kMaxCGAtoms; ++a) {
+                        if (a >= ni) break;
+                        if (xm & (1ull << (a * 8 + b))) continue;
+                        const float2 c = s.lj32[sw.tg[a].x + tj];
+                        pair(a, aj, Dx, Dy, Dz, djx, djy, djz, make_float4(c.x, c.y, 6.f * c.x, 12.f * c.y), qj, gj, gx,
+                             gy, gz);
+                    }
+                    red_add(&F[3 * aj], to_fixed_f(gx, kF));
+                    red_add(&F[3 * aj + 1], to_fixed_f(gy, kF));
+                    red_add(&F[3 * aj + 2], to_fixed_f(gz, kF));
+                }
+            }
+            entry = entry_n;
+            entry_n = -1;
         }
         __syncwarp();
 #pragma unroll
         for (int a = 0; a < kMaxCGAtoms; ++a) {
             if (a >= ni) break;
-            float vx = warp_sum(fix[a]), vy = warp_sum(fiy[a]), vz = warp_sum(fiz[a]);
-            if (lane == (a & 31)) {
+            const float vx = warp_sum(fix[a]), vy = warp_sum(fiy[a]), vz = warp_sum(fiz[a]);
+            if (lane == a) {
                 red_add(&F[3 * (i0 + a)], to_fixed_f(vx, kF));
                 red_add(&F[3 * (i0 + a) + 1], to_fixed_f(vy, kF));
                 red_add(&F[3 * (i0 + a) + 2], to_fixed_f(vz, kF));
             }
         }
-        flush_slot();
+        warp_add_energies(shg, G, cur_slot, to_fixed_f(e_lj, kE), to_fixed_f(e_cr, kE));
+        e_lj = e_cr = 0.f;
         cur_slot = -1;
 #pragma unroll
         for (int v = 0; v < 6; ++v) {
@@ -337,10 +433,10 @@ __global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__
     __syncthreads();
     for (int v = threadIdx.x; v < 2 * G * G; v += blockDim.x)
         if (shg[v]) atomicAdd(reinterpret_cast<unsigned long long*>(dst + v), shg[v]);
-    long long acc[9];
-    const long long vv[9] = {vfix[0], vfix[1], vfix[2], vfix[1], vfix[3], vfix[4], vfix[2], vfix[4], vfix[5]};
+    long long vs[6];
 #pragma unroll
-    for (int v = 0; v < 9; ++v) acc[v] = warp_sum_ll(vv[v]);
+    for (int v = 0; v < 6; ++v) vs[v] = warp_sum_ll(vfix[v]);
+    long long acc[9] = {vs[0], vs[1], vs[2], vs[1], vs[3], vs[4], vs[2], vs[4], vs[5]};
     int idx[9];
 #pragma unroll
     for (int v = 0; v < 9; ++v) idx[v] = 2 * G * G + v;
@@ -447,23 +543,6 @@ __device__ __forceinline__ void add_force_fixed(long long* F, int a, double fx, 
 __device__ __forceinline__ void shared_add(unsigned long long* sh, int idx, double v) {
     long long f = to_fixed_d(v, kEnergyScale);
     if (f) atomicAdd(&sh[idx], static_cast<unsigned long long>(f));
-}
-
-// Adds a warp's fixed-point (LJ, CRF) energies to the block's group sums, one
-// value pair per lane under its group slot (-1: none).  Lanes of one slot, the
-// common case, are summed by shuffles: 32 lanes adding to one 64-bit shared
-// word retry one after the other.
-__device__ __forceinline__ void warp_add_energies(unsigned long long* sh, int G, int sl, long long el, long long ec) {
-    const int lead = __reduce_max_sync(0xffffffffu, sl);
-    if (lead < 0) return;
-    if (__all_sync(0xffffffffu, sl == lead || sl < 0)) {
-        el = warp_sum_ll(el);
-        ec = warp_sum_ll(ec);
-        if ((threadIdx.x & 31) != 0) return;
-        sl = lead;
-    }
-    if (el) atomicAdd(&sh[sl], static_cast<unsigned long long>(el));
-    if (ec) atomicAdd(&sh[G * G + sl], static_cast<unsigned long long>(ec));
 }
 
 // rf_excluded_interactions (excluded.rs:25-112) + one_four_interaction_loop

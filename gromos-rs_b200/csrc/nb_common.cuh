@@ -56,6 +56,9 @@ struct SysDev {
     int W;               // solvent cluster width
     int has_pert;
     int water_lj00_only; // solvent LJ only between site 0 and site 0
+    int solvent_uniform; // every solvent molecule has the types and charges of the first
+    int w_iac[4];        // ... which are these
+    float w_q[4];
     int solvent_group;   // energy group of all solvent atoms (-1 = mixed)
     int excl_atoms;      // atoms [0, excl_atoms) go through k_excluded_14; the
                          // intra-molecular solvent exclusions are done in k_water_prep
@@ -133,9 +136,11 @@ struct SysDev {
     int* wn_s;                 // [max_clusters]
     int* wn_l;
     int wcap;
-    int* sl;                   // [n_solute_cg * scap] (j_cg << 1 | long)
+    int* sl;                   // [n_solute_cg * scap] (j_cg << 1 | long): short entries from the front of a
+                               // CG's scap places, long ones from the back
     unsigned long long* sl_excl; // [n_solute_cg * scap] excluded atom-pair bits
-    int* sn;                   // [n_solute_cg]
+    int* sn;                   // [2 * n_solute_cg] short, long entries
+    int* sn_max;               // [2] the longest of each
     int scap;
     int* pert_pairs;           // [pcap*3] (i, j, long)
     int* n_pert_pairs;         // [1]

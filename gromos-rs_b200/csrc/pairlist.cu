@@ -175,6 +175,7 @@ __global__ void k_refpos(const SysDev* __restrict__ sys, unsigned long long* __r
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < s.n_cg) refpos_one(s, c, cg_key);
     if (last_block(s.build_ctr)) {
+        if (threadIdx.x < 2) s.sn_max[threadIdx.x] = 0;  // the solute search's list lengths
         block_scan8(s.cell_count, s.cell_start, s.n_cells, nullptr);
         __syncthreads();
         for (int i = threadIdx.x; i < s.n_cells; i += blockDim.x) {
@@ -881,7 +882,9 @@ __device__ __forceinline__ unsigned long long excl_mask_warp(const SysDev& s, in
 // neighbour cells' sorted runs are one concatenated candidate range swept 256
 // at a time (positions from the sorted copy, the next round loaded while this
 // one is tested); the hits are compacted in candidate order with the warps'
-// counts, one barrier per round, so the lists are those of a serial sweep.
+// counts, one barrier per round, so the lists are those of a serial sweep:
+// the short entries from the front of the CG's list, the long ones from its
+// back, so that the force kernel of either range reads only its own.
 // Exclusion masks are only looked up for the CGs that share an excluded or
 // 1-4 pair with this one (cgx, from the topology), after the sweep, one
 // warp per mask.
@@ -947,7 +950,7 @@ __global__ void __launch_bounds__(kSoluteSearchWarps * 32) k_solute_search(const
         }
         return c;
     };
-    int cnt = 1;  // the CG's own entry is written last
+    int cnt_s = 1, cnt_l = 0;  // the CG's own entry (short, place 0) is written last
     Cand cur = load(threadIdx.x);
     for (int v0 = 0, par = 0; v0 < total; v0 += blockDim.x, par ^= 1) {
         const Cand nxt = load(v0 + int(blockDim.x) + int(threadIdx.x));
@@ -969,10 +972,11 @@ __global__ void __launch_bounds__(kSoluteSearchWarps * 32) k_solute_search(const
                 }
             }
         }
-        const unsigned bal = __ballot_sync(0xffffffffu, entry >= 0);
-        if (lane == 0) wcnt[par][w] = __popc(bal);
+        const unsigned bs = __ballot_sync(0xffffffffu, entry >= 0 && !(entry & 1));
+        const unsigned bl = __ballot_sync(0xffffffffu, entry >= 0 && (entry & 1));
+        if (lane == 0) wcnt[par][w] = __popc(bs) | (__popc(bl) << 16);
         __syncthreads();
-        int before = 0, round = 0;
+        int before = 0, round = 0;  // short hits in the low half, long ones in the high half
 #pragma unroll
         for (int k = 0; k < kSoluteSearchWarps; ++k) {
             const int c = wcnt[par][k];
@@ -980,8 +984,10 @@ __global__ void __launch_bounds__(kSoluteSearchWarps * 32) k_solute_search(const
             round += c;
         }
         if (entry >= 0) {
-            const int p = cnt + before + __popc(bal & ((1u << lane) - 1u));
-            if (p < scap) {
+            const unsigned below = (1u << lane) - 1u;
+            int p = cnt_s + (before & 0xffff) + __popc(bs & below);
+            if (entry & 1) p = scap - 1 - (cnt_l + (before >> 16) + __popc(bl & below));
+            if (p >= 0 && p < scap) {
                 out[p] = entry;
                 unsigned long long xm = 0ull;
                 if (masked) {
@@ -996,7 +1002,8 @@ __global__ void __launch_bounds__(kSoluteSearchWarps * 32) k_solute_search(const
                 outx[p] = xm;
             }
         }
-        cnt += round;
+        cnt_s += round & 0xffff;
+        cnt_l += round >> 16;
         cur = nxt;
     }
     __syncthreads();  // the queue, and the zero masks of its entries
@@ -1010,8 +1017,13 @@ __global__ void __launch_bounds__(kSoluteSearchWarps * 32) k_solute_search(const
         }
     }
     if (threadIdx.x == 0) {
-        if (cnt > scap) atomicOr(&s.err[0], ERR_SLIST_OVERFLOW);
-        s.sn[ci] = min(cnt, scap);
+        if (cnt_s + cnt_l > scap) atomicOr(&s.err[0], ERR_SLIST_OVERFLOW);
+        cnt_s = min(cnt_s, scap);
+        cnt_l = min(cnt_l, scap - cnt_s);
+        s.sn[2 * ci] = cnt_s;
+        s.sn[2 * ci + 1] = cnt_l;
+        atomicMax(&s.sn_max[0], cnt_s);
+        atomicMax(&s.sn_max[1], cnt_l);
     }
 }
 
@@ -1022,7 +1034,7 @@ __global__ void k_pert_pairs(const SysDev* __restrict__ sys) {
     const SysDev& s = sys[blockIdx.y];
     int gid = blockIdx.x * blockDim.x + threadIdx.x;
     int ci = gid / s.scap, e = gid % s.scap;
-    if (ci >= s.n_solute_cg || e >= s.sn[ci]) return;
+    if (ci >= s.n_solute_cg || (e >= s.sn[2 * ci] && e < s.scap - s.sn[2 * ci + 1])) return;
     int entry = s.sl[static_cast<size_t>(ci) * s.scap + e];
     unsigned long long xm = s.sl_excl[static_cast<size_t>(ci) * s.scap + e];
     int cj = entry >> 1, lr = entry & 1;
@@ -1078,7 +1090,7 @@ __global__ void k_expand_cgpairs(const SysDev* __restrict__ sys, int long_range)
     }
     long long g2 = gid - nwater;
     int ci = static_cast<int>(g2 / s.scap), e = static_cast<int>(g2 % s.scap);
-    if (ci >= s.n_solute_cg || e >= s.sn[ci]) return;
+    if (ci >= s.n_solute_cg || (e >= s.sn[2 * ci] && e < s.scap - s.sn[2 * ci + 1])) return;
     int entry = s.sl[static_cast<size_t>(ci) * s.scap + e];
     if ((entry & 1) != long_range) return;
     int p = atomicAdd(&s.n_cgp[long_range], 1);
