@@ -24,8 +24,8 @@
 //   k_plain_force       baseline: thread per CG pair, absolute FP32, FP32 atomics
 //   k_excluded_14       FP64 RF excluded / self terms (excluded.rs:25-112) and
 //                       1-4 pairs (excluded.rs:131-206)
-//   k_pert_pairs_force  FP64 soft-core pair correction (perturbed.rs:309-386)
-//   k_pert_terms        FP64 self / excluded / 1-4 / atom-pair corrections
+//   k_pert              FP64 soft-core pair correction (perturbed.rs:309-386) and the
+//                       self / excluded / 1-4 / atom-pair corrections
 //   k_finalize          fixed point -> FP64 outputs
 #include "nb_common.cuh"
 
@@ -647,16 +647,19 @@ __device__ void pert_interaction(const SysDev& s, double rx, double ry, double r
     const double r6 = r2 * r2 * r2, r4 = r2 * r2;
     const double a_c126 = fabs(a_c6) > 1e-10 ? a_c12 / a_c6 : 0.0;
     const double b_c126 = fabs(b_c6) > 1e-10 ? b_c12 / b_c6 : 0.0;
-    const double a_d2s = r2 + acrf * b_crfs2, a_dis = 1.0 / sqrt(a_d2s), a_d3is = a_dis / a_d2s;
+    // 1/sqrt and its powers from one rsqrt each: an FP64 division or square root is about
+    // ten FP64 operations, and these are most of a pair's work
+    const double a_dis = rsqrt(r2 + acrf * b_crfs2), a_d3is = a_dis * a_dis * a_dis;
     const double a_d6i = 1.0 / (r6 + alj * b_ljs2 * a_c126);
-    const double b_d2s = r2 + acrf * a_crfs2, b_dis = 1.0 / sqrt(b_d2s), b_d3is = b_dis / b_d2s;
+    const double b_dis = rsqrt(r2 + acrf * a_crfs2), b_d3is = b_dis * b_dis * b_dis;
     const double b_d6i = 1.0 / (r6 + alj * a_ljs2 * b_c126);
     const double cut2 = s.cutoff_sq;
-    const double a_c2s = cut2 + acrf * b_crfs2, b_c2s = cut2 + acrf * a_crfs2;
-    const double a_crf_2cut3i = s.crf_2cut3i / sqrt(a_c2s * a_c2s * a_c2s);
-    const double b_crf_2cut3i = s.crf_2cut3i / sqrt(b_c2s * b_c2s * b_c2s);
+    const double a_ci = rsqrt(cut2 + acrf * b_crfs2), b_ci = rsqrt(cut2 + acrf * a_crfs2);
+    const double a_ci2 = a_ci * a_ci, b_ci2 = b_ci * b_ci;
+    const double a_crf_2cut3i = s.crf_2cut3i * (a_ci2 * a_ci);
+    const double b_crf_2cut3i = s.crf_2cut3i * (b_ci2 * b_ci);
     const double a_crf_cut3i = 2.0 * a_crf_2cut3i, b_crf_cut3i = 2.0 * b_crf_2cut3i;
-    const double a_crf_pert = 3.0 * a_crf_2cut3i / a_c2s, b_crf_pert = 3.0 * b_crf_2cut3i / b_c2s;
+    const double a_crf_pert = 3.0 * a_crf_2cut3i * a_ci2, b_crf_pert = 3.0 * b_crf_2cut3i * b_ci2;
     double force = (a_crf_n * a_q * (a_d3is + a_crf_cut3i) + b_crf_n * b_q * (b_d3is + b_crf_cut3i)) * s.fpe;
     force += -6.0 * (a_lj_n * a_c6 * a_d6i * a_d6i + b_lj_n * b_c6 * b_d6i * b_d6i) * r4;
     force += 12.0 * (a_lj_n * a_c12 * a_d6i * a_d6i * a_d6i + b_lj_n * b_c12 * b_d6i * b_d6i * b_d6i) * r4;
@@ -699,117 +702,108 @@ __device__ __forceinline__ PInfo pinfo(const SysDev& s, int a) {
 
 // perturbed_pairlist_correction (perturbed.rs:309-386) for the explicit list
 // of (i perturbed, j) pairs of all lists, every step, per-atom image.
-// Each thread takes kPertRun consecutive pairs of the list (pairs are listed
-// per perturbed atom, so i rarely changes within a run).  Every pair's
-// contribution goes to fixed point first and the integers are summed in
-// registers -- the i-force until i changes, the energies until their group
-// slot changes -- so far fewer same-address atomics are issued than one per
-// pair, and the totals do not depend on the list's order (which the atomic
-// appends of k_pert_pairs do not fix).
-constexpr int kPertRun = 16;
-
-__global__ void k_pert_pairs_force(const SysDev* __restrict__ sys) {
-    const SysDev& s = sys[blockIdx.y];
-    const int G = s.n_egroups;
-    const int NA = acc_size(G);
-    extern __shared__ unsigned long long sh[];
-    for (int v = threadIdx.x; v < NA; v += blockDim.x) sh[v] = 0ull;
-    __syncthreads();
+// One thread per pair: the pairs are some tens of thousands of FP64 chains, so
+// runs of pairs per thread left most SMs without a block (35,000 pairs in runs of
+// 16: 66 us, and 9.5 for the per-atom terms, launched over every atom; one launch of
+// 18 us now, ncu).  Every pair's contribution goes to fixed point first
+// and a warp's integers are summed by shuffles -- the i-force per distinct i
+// (pairs are listed per solute charge group, so a warp has few) and the
+// energies per group slot -- so the totals do not depend on the list's order,
+// which the atomic appends of k_pert_pairs do not fix, and few same-address
+// additions are issued.
+__device__ __forceinline__ void pert_pairs(const SysDev& s, unsigned long long* sh, int block, int nblocks) {
+    const int G = s.n_egroups, lane = threadIdx.x & 31;
     const int np = min(s.n_pert_pairs[0], s.pcap);
-    const int p0 = (blockIdx.x * blockDim.x + threadIdx.x) * kPertRun;
-    const int p1 = min(np, p0 + kPertRun);
-    int cur_i = -1, cur_sl = -1;
-    long long fxi = 0, fyi = 0, fzi = 0, el = 0, ec = 0, dh = 0;
-    auto flush_i = [&]() {
-        if (cur_i >= 0) {
-            red_add(&s.f_short[3 * cur_i], fxi);
-            red_add(&s.f_short[3 * cur_i + 1], fyi);
-            red_add(&s.f_short[3 * cur_i + 2], fzi);
+    for (int p0 = block * blockDim.x + threadIdx.x - lane; p0 < np; p0 += nblocks * blockDim.x) {  // warp-uniform
+        const int p = p0 + lane;
+        int i = -1, sl = -1;
+        long long fx = 0, fy = 0, fz = 0, el = 0, ec = 0, dh = 0;
+        if (p < np) {
+            i = s.pert_pairs[3 * p];
+            const int j = s.pert_pairs[3 * p + 1];
+            const PInfo pi = pinfo(s, i), pj = pinfo(s, j);
+            const double* lja = s.lj64 + 4 * (pi.a_iac * s.n_types + pj.a_iac);
+            const double* ljb = s.lj64 + 4 * (pi.b_iac * s.n_types + pj.b_iac);
+            const double a_q = pi.a_q * pj.a_q, b_q = pi.b_q * pj.b_q;
+            const double alj = pj.on ? (pi.alj + pj.alj) * 0.5 : pi.alj;
+            const double acrf = pj.on ? (pi.acrf + pj.acrf) * 0.5 : pi.acrf;
+            double rx, ry, rz;
+            nearest_image_exact(s, s.pos[3 * i], s.pos[3 * i + 1], s.pos[3 * i + 2], s.pos[3 * j], s.pos[3 * j + 1],
+                                s.pos[3 * j + 2], rx, ry, rz);
+            const double r2 = len2_exact(rx, ry, rz);
+            double fa = 0, ela = 0, eca = 0;
+            if (!(r2 < 1e-10)) {  // lj_crf_interaction, state A
+                const double ir = rsqrt(r2), ir2 = ir * ir, ir6 = ir2 * ir2 * ir2;
+                const double qa = a_q * s.fpe;
+                ela = (lja[1] * ir6 - lja[0]) * ir6;
+                eca = qa * (ir - s.crf_2cut3i * r2 - s.crf_cut);
+                fa = (12.0 * lja[1] * ir6 - 6.0 * lja[0]) * ir6 * ir2 + qa * (ir * ir2 + s.crf_cut3i);
+            }
+            double o[5];
+            pert_interaction(s, rx, ry, rz, lja[0], lja[1], ljb[0], ljb[1], a_q, b_q, alj, acrf, o);
+            const double df = o[0] - fa;
+            fx = to_fixed_d(rx * df, kForceScale);
+            fy = to_fixed_d(ry * df, kForceScale);
+            fz = to_fixed_d(rz * df, kForceScale);
+            add_force_fixed(s.f_short, j, -rx * df, -ry * df, -rz * df);
+            sl = group_slot(G, s.egroup[i], s.egroup[j]);
+            el = to_fixed_d(o[1] - ela, kEnergyScale);
+            ec = to_fixed_d(o[2] - eca, kEnergyScale);
+            dh = to_fixed_d(o[3] + o[4], kEnergyScale);
         }
-        fxi = fyi = fzi = 0;
-    };
-    auto flush_e = [&]() {
-        if (cur_sl >= 0) {
-            if (el) atomicAdd(&sh[cur_sl], static_cast<unsigned long long>(el));
-            if (ec) atomicAdd(&sh[G * G + cur_sl], static_cast<unsigned long long>(ec));
+        unsigned left = __ballot_sync(0xffffffffu, i >= 0);
+        while (left) {
+            const int lead = __shfl_sync(0xffffffffu, i, __ffs(left) - 1);
+            const bool mine = i == lead;
+            const long long tx = warp_sum_ll(mine ? fx : 0), ty = warp_sum_ll(mine ? fy : 0);
+            const long long tz = warp_sum_ll(mine ? fz : 0);
+            if (lane == 0) {
+                red_add(&s.f_short[3 * lead], tx);
+                red_add(&s.f_short[3 * lead + 1], ty);
+                red_add(&s.f_short[3 * lead + 2], tz);
+            }
+            left &= ~__ballot_sync(0xffffffffu, mine);
         }
-        el = ec = 0;
-    };
-    for (int p = p0; p < p1; ++p) {
-        const int i = s.pert_pairs[3 * p], j = s.pert_pairs[3 * p + 1];
-        const PInfo pi = pinfo(s, i), pj = pinfo(s, j);
-        const double* lja = s.lj64 + 4 * (pi.a_iac * s.n_types + pj.a_iac);
-        const double* ljb = s.lj64 + 4 * (pi.b_iac * s.n_types + pj.b_iac);
-        const double a_q = pi.a_q * pj.a_q, b_q = pi.b_q * pj.b_q;
-        const double alj = pj.on ? (pi.alj + pj.alj) * 0.5 : pi.alj;
-        const double acrf = pj.on ? (pi.acrf + pj.acrf) * 0.5 : pi.acrf;
-        double rx, ry, rz;
-        nearest_image_exact(s, s.pos[3 * i], s.pos[3 * i + 1], s.pos[3 * i + 2], s.pos[3 * j], s.pos[3 * j + 1],
-                            s.pos[3 * j + 2], rx, ry, rz);
-        const double r2 = len2_exact(rx, ry, rz);
-        double fa = 0, ela = 0, eca = 0;
-        if (!(r2 < 1e-10)) {  // lj_crf_interaction, state A
-            const double ir2 = 1.0 / r2, ir6 = ir2 * ir2 * ir2, ir = sqrt(ir2);
-            const double qa = a_q * s.fpe;
-            ela = (lja[1] * ir6 - lja[0]) * ir6;
-            eca = qa * (ir - s.crf_2cut3i * r2 - s.crf_cut);
-            fa = (12.0 * lja[1] * ir6 - 6.0 * lja[0]) * ir6 * ir2 + qa * (ir * ir2 + s.crf_cut3i);
-        }
-        double o[5];
-        pert_interaction(s, rx, ry, rz, lja[0], lja[1], ljb[0], ljb[1], a_q, b_q, alj, acrf, o);
-        const double df = o[0] - fa;
-        if (i != cur_i) {
-            flush_i();
-            cur_i = i;
-        }
-        fxi += to_fixed_d(rx * df, kForceScale);
-        fyi += to_fixed_d(ry * df, kForceScale);
-        fzi += to_fixed_d(rz * df, kForceScale);
-        add_force_fixed(s.f_short, j, -rx * df, -ry * df, -rz * df);
-        const int sl = group_slot(G, s.egroup[i], s.egroup[j]);
-        if (sl != cur_sl) {
-            flush_e();
-            cur_sl = sl;
-        }
-        el += to_fixed_d(o[1] - ela, kEnergyScale);
-        ec += to_fixed_d(o[2] - eca, kEnergyScale);
-        dh += to_fixed_d(o[3] + o[4], kEnergyScale);
+        warp_add_energies(sh, G, sl, el, ec);
+        dh = warp_sum_ll(dh);
+        if (lane == 0 && dh) atomicAdd(&sh[acc_size(G) - 1], static_cast<unsigned long long>(dh));
     }
-    flush_i();
-    flush_e();
-    if (dh) atomicAdd(&sh[NA - 1], static_cast<unsigned long long>(dh));
-    __syncthreads();
-    for (int v = threadIdx.x; v < NA; v += blockDim.x)
-        if (sh[v]) atomicAdd(reinterpret_cast<unsigned long long*>(s.acc_short + v), sh[v]);
 }
 
 // Self / excluded / 1-4 / PERTATOMPAIR corrections (perturbed.rs:395-707).
-// One thread per atom i (excluded and 1-4 pairs with j > i); PERTATOMPAIR
-// entries are handled by the threads i < n_pp.
-__global__ void k_pert_terms(const SysDev* __restrict__ sys) {
-    const SysDev& s = sys[blockIdx.y];
+// One thread per solute atom i (excluded and 1-4 pairs with j > i: only
+// solute atoms are perturbed, so a pair with a perturbed atom starts at one);
+// PERTATOMPAIR entries are handled by the threads i < n_pp.
+__device__ __forceinline__ void pert_terms(const SysDev& s, unsigned long long* sh, int block) {
     const int G = s.n_egroups;
     const int NA = acc_size(G);
-    extern __shared__ unsigned long long sh[];
-    for (int v = threadIdx.x; v < NA; v += blockDim.x) sh[v] = 0ull;
-    __syncthreads();
     const double* lp = s.lp;
     const double a_lj_n = lp[0], b_lj_n = lp[1], a_crf_n = lp[2], b_crf_n = lp[3];
     const double a_lj_n1 = lp[4], b_lj_n1 = lp[5], a_crf_n1 = lp[6], b_crf_n1 = lp[7];
     const double a_crfs = lp[12], b_crfs = lp[13], a_crfs2 = lp[14], b_crfs2 = lp[15];
     const double nexp = lp[16];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < s.n_atoms) {
-        const PInfo pi = pinfo(s, i);
-        const int gi = s.egroup[i];
-        if (pi.on) {  // perturbed_self_energy_correction
+    const int i = block * blockDim.x + threadIdx.x;
+    {  // perturbed_self_energy_correction
+        int sl = -1;
+        long long e = 0, dh = 0;
+        if (i < s.n_solute_atoms && s.pert_idx[i] >= 0) {
+            const PInfo pi = pinfo(s, i);
             const double qa2 = pi.a_q * pi.a_q, qb2 = pi.b_q * pi.b_q;
             const double e_rf = (-(a_crf_n * qa2) - b_crf_n * qb2 + qa2) * s.crf_cut * s.fpe;
             const double de_rf = nexp * (a_crf_n1 * qa2 - b_crf_n1 * qb2) * s.crf_cut * s.fpe;
-            shared_add(sh, G * G + group_slot(G, gi, gi), 0.5 * e_rf);
-            shared_add(sh, NA - 1, 0.5 * de_rf);
+            sl = group_slot(G, s.egroup[i], s.egroup[i]);
+            e = to_fixed_d(0.5 * e_rf, kEnergyScale);
+            dh = to_fixed_d(0.5 * de_rf, kEnergyScale);
         }
-        if (i < s.n_solute_atoms) {  // perturbed_excluded_correction
+        warp_add_energies(sh, G, sl, 0, e);
+        dh = warp_sum_ll(dh);
+        if ((threadIdx.x & 31) == 0 && dh) atomicAdd(&sh[NA - 1], static_cast<unsigned long long>(dh));
+    }
+    if (i < s.n_solute_atoms || i < s.n_pp) {
+        if (i < s.n_solute_atoms) {
+            const PInfo pi = pinfo(s, i);
+            const int gi = s.egroup[i];
+            // perturbed_excluded_correction
             for (int k = s.excl_off[i]; k < s.excl_off[i + 1]; ++k) {
                 const int j = s.excl[k];
                 if (j <= i) continue;
@@ -842,7 +836,6 @@ __global__ void k_pert_terms(const SysDev* __restrict__ sys) {
                 shared_add(sh, G * G + group_slot(G, gi, s.egroup[j]), e_p - e_a);
                 shared_add(sh, NA - 1, de);
             }
-        }
         for (int k = s.o14_off[i]; k < s.o14_off[i + 1]; ++k) {  // perturbed_one_four_correction
             const int j = s.o14[k];
             if (j <= i) continue;
@@ -872,6 +865,7 @@ __global__ void k_pert_terms(const SysDev* __restrict__ sys) {
             shared_add(sh, sl, o[1] - e_lj_a);
             shared_add(sh, G * G + sl, o[2] - e_crf_a);
             shared_add(sh, NA - 1, o[3] + o[4]);
+        }
         }
         if (i < s.n_pp) {  // perturbed_atom_pair_correction
             const int a = s.pp[4 * i], b = s.pp[4 * i + 1], at = s.pp[4 * i + 2], bt = s.pp[4 * i + 3];
@@ -914,6 +908,20 @@ __global__ void k_pert_terms(const SysDev* __restrict__ sys) {
             }
         }
     }
+}
+
+// All perturbation corrections in one launch: the first term_blocks blocks
+// take the per-atom terms, the others the listed pairs.
+__global__ void __launch_bounds__(128) k_pert(const SysDev* __restrict__ sys, int term_blocks) {
+    const SysDev& s = sys[blockIdx.y];
+    const int NA = acc_size(s.n_egroups);
+    extern __shared__ unsigned long long sh[];
+    for (int v = threadIdx.x; v < NA; v += blockDim.x) sh[v] = 0ull;
+    __syncthreads();
+    if (int(blockIdx.x) < term_blocks)
+        pert_terms(s, sh, blockIdx.x);
+    else
+        pert_pairs(s, sh, blockIdx.x - term_blocks, gridDim.x - term_blocks);
     __syncthreads();
     for (int v = threadIdx.x; v < NA; v += blockDim.x)
         if (sh[v]) atomicAdd(reinterpret_cast<unsigned long long*>(s.acc_short + v), sh[v]);

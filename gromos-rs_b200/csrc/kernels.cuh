@@ -30,8 +30,7 @@ __global__ void k_solute_force(const SysDev* __restrict__ sys);
 __global__ void k_pos32(const SysDev* __restrict__ sys);
 __global__ void k_plain_force(const SysDev* __restrict__ sys, int long_range);
 __global__ void k_excluded_14(const SysDev* __restrict__ sys);
-__global__ void k_pert_pairs_force(const SysDev* __restrict__ sys);
-__global__ void k_pert_terms(const SysDev* __restrict__ sys);
+__global__ void k_pert(const SysDev* __restrict__ sys, int term_blocks);
 __global__ void k_finalize(const SysDev* __restrict__ sys, int plain);
 __global__ void k_finalize_plain_energies(const SysDev* __restrict__ sys);
 __global__ void k_ffma_peak(float* out, int iters, float a, float b);
