@@ -2052,7 +2052,7 @@ extern "C" gr_status gr_lj_crf_innerloop(const float* positions, const float* ch
     } else {
         float bx = boundary_type ? float(box_data[0]) : 1.f, by = boundary_type ? float(box_data[1]) : 1.f;
         float bz = boundary_type ? float(box_data[2]) : 1.f;
-        unsigned grid = std::min(4096u, (n_pairs + 255) / 256);
+        const unsigned grid = innerloop_grid(n_pairs);
         k_innerloop_pairs<<<grid, 256>>>(dpos, dq, diac, dpairs, n_pairs, dlj, n_types, bx, by, bz,
                                          int(boundary_type), float(crf_cut), float(crf_2cut3i), float(crf_cut3i),
                                          138.9354f, dF, dE);

@@ -117,8 +117,7 @@ extern "C" gr_status gr_lj_crf_innerloop_noalloc(const float* positions, const f
         if (n_pairs > 0) {
             const float bx = boundary_type ? float(box_data[0]) : 1.f, by = boundary_type ? float(box_data[1]) : 1.f;
             const float bz = boundary_type ? float(box_data[2]) : 1.f;
-            unsigned grid = (n_pairs + 255) / 256;
-            if (grid > 4096) grid = 4096;
+            const unsigned grid = innerloop_grid(n_pairs);
             k_innerloop_pairs<<<grid, 256, 0, s>>>(positions, charges, iac, pairlist, n_pairs, scr->lj, n_types, bx,
                                                    by, bz, int(boundary_type), float(crf_cut), float(crf_2cut3i),
                                                    float(crf_cut3i), 138.9354f, forces, scr->acc);

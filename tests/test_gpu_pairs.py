@@ -1,0 +1,85 @@
+"""GPU: the explicit pair loop over list orders, lengths and alignments, against FP64 numpy."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from gromos_nb import _lib
+from gromos_nb.nonbonded import CRFParameters
+
+pytestmark = pytest.mark.gpu
+
+N, BOX = 600, np.array([3.1, 2.9, 3.3])
+
+
+def inputs(n_pairs, order, seed=4):
+    rng = np.random.default_rng(seed)
+    # a jittered lattice: no two atoms nearer than 0.1 nm
+    g = np.stack(np.meshgrid(*[np.arange(9)] * 3, indexing="ij"), -1).reshape(-1, 3)[:N]
+    x = (g * 0.3 + rng.uniform(-0.1, 0.1, (N, 3))).astype(np.float32)
+    i, j = np.triu_indices(N, 1)
+    k = rng.permutation(len(i))[:n_pairs]
+    if order == "sorted":
+        k = np.sort(k)
+    elif order == "one":      # one atom's pairs, long runs
+        i, j = np.zeros(n_pairs, dtype=int), 1 + np.arange(n_pairs) % (N - 1)
+        k = np.arange(n_pairs)
+    elif order == "mixed":    # rounds of a few i's
+        k = k[np.argsort(i[k] // 3, kind="stable")]
+    pairs = np.stack([i[k], j[k]], 1).astype(np.uint32)
+    q = rng.normal(0, 0.4, N).astype(np.float32)
+    iac = rng.integers(0, 5, N).astype(np.uint32)
+    lj = np.abs(rng.normal(1.0, 0.3, (5, 5, 2))) * [2.6e-3, 2.6e-7]
+    return x, q, iac, pairs, lj + lj.transpose(1, 0, 2)
+
+
+def reference(x, q, iac, pairs, lj, crf, box):
+    i, j = pairs[:, 0].astype(int), pairs[:, 1].astype(int)
+    x, q = x.astype(np.float64), q.astype(np.float64)
+    r = x[i] - x[j]
+    if box is not None:
+        r -= box * np.round(r / box)
+    r2 = (r * r).sum(1)
+    c = lj[iac[i], iac[j]]
+    i6, ir, qq = r2 ** -3.0, r2 ** -0.5, q[i] * q[j] * 138.9354
+    fs = (12 * c[:, 1] * i6 - 6 * c[:, 0]) * i6 / r2 + qq * (ir / r2 + crf.crf_cut3i)
+    f = np.zeros_like(x)
+    np.add.at(f, i, r * fs[:, None])
+    np.add.at(f, j, -r * fs[:, None])
+    return f, ((c[:, 1] * i6 - c[:, 0]) * i6).sum(), (qq * (ir - crf.crf_2cut3i * r2 - crf.crf_cut)).sum(), \
+        r.T @ (r * fs[:, None])
+
+
+# a round is 32 pairs, a warp's chunk 256, a block's 2048; offsets put pairs and forces 4 bytes off
+@pytest.mark.parametrize("n_pairs,order,offset,periodic", [
+    (1, "sorted", 0, True), (31, "random", 1, True), (33, "sorted", 0, False), (256, "one", 1, True),
+    (257, "mixed", 0, True), (2049, "random", 1, False), (20000, "sorted", 1, True), (60000, "mixed", 0, True),
+    (60000, "one", 0, True)])
+def test_pair_loop(n_pairs, order, offset, periodic):
+    import torch
+
+    x, q, iac, pairs, lj = inputs(n_pairs, order)
+    crf = CRFParameters.new(1.4, 1.0, 61.0, 0.0)
+    f_ref, lj_ref, crf_ref, v_ref = reference(x, q, iac, pairs, lj, crf, BOX if periodic else None)
+    dev = "cuda"
+
+    def shifted(a):  # `offset` 4-byte words into an allocation
+        t = torch.zeros(a.size + offset, dtype=torch.int32, device=dev)
+        t[offset:] = torch.from_numpy(a.view(np.int32).reshape(-1)).to(dev)
+        return t[offset:]
+
+    xd, qd, td, pd, fd = (shifted(a) for a in (x, q, iac, pairs, np.full_like(x, 3.0)))
+    ljd = torch.tensor(lj, dtype=torch.float64, device=dev)
+    e, v = torch.empty(2, dtype=torch.float64, device=dev), torch.empty(9, dtype=torch.float64, device=dev)
+    _lib.check(_lib.lib().gr_lj_crf_innerloop_noalloc(
+        xd.data_ptr(), qd.data_ptr(), td.data_ptr(), N, pd.data_ptr(), n_pairs, ljd.data_ptr(), 5,
+        BOX.ctypes.data_as(C.c_void_p), 1 if periodic else 0, crf.crf_cut, crf.crf_2cut3i, crf.crf_cut3i,
+        fd.data_ptr(), e.data_ptr(), v.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    f = fd.cpu().numpy().view(np.float32).reshape(-1, 3).astype(np.float64)
+    # a pair's force carries the FP32 rounding of its coordinates (2.7 nm: 1.2e-7 on r >= 0.1 nm, times 13
+    # for r^-13), the sums of up to 60,000 pairs on one atom sqrt(n) 6e-8: 2e-5 of the largest covers both
+    assert np.abs(f - f_ref).max() <= 2e-5 * np.abs(f_ref).max()
+    el, ec = e.tolist()
+    assert abs(el - lj_ref) <= 2e-5 * max(abs(lj_ref), abs(crf_ref))
+    assert abs(ec - crf_ref) <= 2e-5 * max(abs(lj_ref), abs(crf_ref))
+    assert np.abs(v.cpu().numpy().reshape(3, 3) - v_ref).max() <= 2e-5 * np.abs(v_ref).max()
