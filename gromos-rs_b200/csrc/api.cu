@@ -1312,6 +1312,8 @@ WaterParams NbSystem::water_params() const {
         wp.inv_box[k] = h.inv_box[k];
         wp.boxf[k] = h.boxf[k];
         wp.inv_boxf[k] = h.inv_boxf[k];
+        wp.boxlo[k] = float(h.box[k] - double(h.boxf[k]));
+        wp.half[k] = wp.lim[k];
     }
     wp.boundary = h.boundary;
     wp.G = G;
