@@ -229,6 +229,7 @@ void NbSystem::release() {
     allocs.clear();
     if (d_sys) dev_free(d_sys);
     d_sys = nullptr;
+    sent_valid = false;
     if (any) cudaStreamSynchronize(mem_stream);  // the blocks are back in the pool before the stream goes
     std::memset(&h, 0, sizeof(h));
     d_cg_key = nullptr;
@@ -861,8 +862,16 @@ cudaError_t NbSystem::record_event(cudaEvent_t e, cudaStream_t s) {
 }
 
 gr_status NbSystem::push_descriptor(cudaStream_t s) {
-    if (in_capture) return GR_OK;
+    // Only what changed travels: the copy is an operation of its own between two
+    // steps' kernels (with the snapshots' three per pairlist period, 5 of the 61 us
+    // of a 1,000-water MD step).  The comparison is by
+    // content, with what this context last sent; h is zeroed before it is filled,
+    // so its padding compares equal.
+    if (in_capture || (sent_valid && std::memcmp(&h, &sent, sizeof(SysDev)) == 0)) return GR_OK;
+    sent_valid = false;
     GR_CUDA(cudaMemcpyAsync(d_sys, &h, sizeof(SysDev), cudaMemcpyHostToDevice, s));
+    std::memcpy(&sent, &h, sizeof(SysDev));
+    sent_valid = true;
     return GR_OK;
 }
 
@@ -938,7 +947,8 @@ gr_status NbSystem::build_pairlist(cudaStream_t s, bool sync) {
         gr_status st = ensure_capacity();
         if (st) return st;
         if ((st = push_descriptor(s))) return st;
-        (++launches, k_refpos<<<blocks_for(NCG, 256), 256, 0, s>>>(d_sys, d_cg_key));
+        (++launches, k_refpos<<<blocks_for(NCG, 256), 256, 0, s>>>(d_sys, d_cg_key, snapshot));
+        snapshot = MdSnapshot{};  // taken once (a retry builds the same positions)
         (++launches, k_scatter<<<blocks_for(NCG, 256), 256, 0, s>>>(d_sys, d_cg_key));
         (++launches, k_cell_sort<<<h.n_cells, 256, 0, s>>>(d_sys));
         (++launches, k_cluster_setup<<<h.n_cells, 128, 0, s>>>(d_sys));
@@ -1042,6 +1052,8 @@ gr_status NbSystem::drop_prep(cudaStream_t s) {
 // Without `finalize` the caller's MD step kernel does k_finalize's work
 // (the fixed-point kernel only).
 gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events, bool finalize) {
+    const MdSnapshot snap = snapshot;  // for this evaluation's build alone, whatever becomes of it
+    snapshot = MdSnapshot{};
     if (!uploaded || !params_set || !box_set || !pos_set) {
         set_error("gr_forces_eval before topology, parameters, box and positions are set");
         return GR_ERR_STATE;
@@ -1071,7 +1083,10 @@ gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events, bool fin
     if (record_events) GR_CUDA(record_event(ev[0], s));
     if (rebuild) {
         // the first build of a system synchronises to size the list capacities
-        if ((st = build_pairlist(s, !ever_built))) return st;
+        snapshot = snap;
+        st = build_pairlist(s, !ever_built);
+        snapshot = MdSnapshot{};
+        if (st) return st;
         ever_built = true;
         if (prm.kernel == GR_KERNEL_PLAIN)
             if ((st = expand_cg_pairs(s))) return st;

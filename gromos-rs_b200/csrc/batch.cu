@@ -177,13 +177,8 @@ gr_status batch_capture_graphs(gr_batch* b) {
             const int ph = int((p + mb.offset) % b->nsnb);
             e = cudaStreamWaitEvent(si, b->fork, 0);
             if (e != cudaSuccess) break;
-            const size_t bytes3 = size_t(S.N) * 3 * sizeof(double);
             if (ph == 0) {  // pairlist period starts: snapshot for rollback, then rebuild
-                e = cudaMemcpyAsync(S.md_pos_snap, S.h.pos, bytes3, cudaMemcpyDeviceToDevice, si);
-                if (e == cudaSuccess) e = cudaMemcpyAsync(S.md_vel_snap, S.md_vel, bytes3, cudaMemcpyDeviceToDevice, si);
-                if (e == cudaSuccess)
-                    e = cudaMemcpyAsync(S.md_ke_snap, S.md_ke, sizeof(long long), cudaMemcpyDeviceToDevice, si);
-                if (e != cudaSuccess) break;
+                S.snapshot = gnb::MdSnapshot{S.md_pos_snap, S.md_vel_snap, S.md_ke_snap, S.md_vel, S.md_ke};
                 S.steps_since_update = S.prm.nsnb;
             } else {
                 S.steps_since_update = 1;

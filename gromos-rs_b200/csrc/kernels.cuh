@@ -4,7 +4,7 @@
 #include "nb_common.cuh"
 
 namespace gnb {
-__global__ void k_refpos(const SysDev* __restrict__ sys, unsigned long long* __restrict__ cg_key);
+__global__ void k_refpos(const SysDev* __restrict__ sys, unsigned long long* __restrict__ cg_key, const MdSnapshot snap);
 __global__ void k_scatter(const SysDev* __restrict__ sys, const unsigned long long* __restrict__ cg_key);
 __global__ void k_cell_sort(const SysDev* __restrict__ sys);
 __global__ void k_cluster_setup(const SysDev* __restrict__ sys);

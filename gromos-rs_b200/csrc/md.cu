@@ -503,9 +503,7 @@ gr_status NbSystem::md_run(cudaStream_t s, int n_steps, gr_md_stats* out) {
                     }
                 }
                 if (!built || steps_since_update >= prm.nsnb) {  // this step starts a pairlist period
-                    GR_CUDA(cudaMemcpyAsync(md_psnap_pos, h.pos, bytes3, cudaMemcpyDeviceToDevice, s));
-                    GR_CUDA(cudaMemcpyAsync(md_psnap_vel, md_vel, bytes3, cudaMemcpyDeviceToDevice, s));
-                    GR_CUDA(cudaMemcpyAsync(md_psnap_ke, md_ke, sizeof(long long), cudaMemcpyDeviceToDevice, s));
+                    snapshot = MdSnapshot{md_psnap_pos, md_psnap_vel, md_psnap_ke, md_vel, md_ke};
                     md_psnap_step = md_step_idx;
                     md_psnap_valid = true;
                 }

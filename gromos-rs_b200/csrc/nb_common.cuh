@@ -173,6 +173,14 @@ struct SysDev {
     int* err;                  // [4] error flags, counters
 };
 
+// The MD state that a pairlist build copies aside for a rollback (null pos: none).
+struct MdSnapshot {
+    double *pos, *vel;
+    long long* ke;
+    const double* cur_vel;
+    const long long* cur_ke;
+};
+
 __host__ __device__ inline int acc_size(int G) { return 2 * G * G + 9 + 1; }
 
 // ---------------------------------------------------------------------------

@@ -71,6 +71,9 @@ class NbSystem {
     // device descriptor (host mirror + device copy)
     SysDev h{};
     SysDev* d_sys = nullptr;
+    SysDev sent{};            // what d_sys holds
+    bool sent_valid = false;
+    MdSnapshot snapshot{};    // MD state that the next pairlist build copies aside (null: none)
     unsigned long long* d_cg_key = nullptr;
     // state
     bool uploaded = false, params_set = false, box_set = false, pos_set = false;

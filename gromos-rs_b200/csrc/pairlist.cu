@@ -169,10 +169,35 @@ __device__ __forceinline__ bool last_block(int* ctr) {
 }
 
 // The last block scans the cell counts into the cell starts and clears the
-// counts and the scatter's fill counters for the next build.
-__global__ void k_refpos(const SysDev* __restrict__ sys, unsigned long long* __restrict__ cg_key) {
+// counts and the scatter's fill counters for the next build.  At the start of an
+// MD run's pairlist period the kernel also copies the MD state aside, instead of
+// three copies of their own between the steps.
+__global__ void k_refpos(const SysDev* __restrict__ sys, unsigned long long* __restrict__ cg_key,
+                         const MdSnapshot snap) {
     const SysDev& s = sys[blockIdx.y];
     int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (snap.pos) {
+        // three values of either array in flight per thread (the copies' stores
+        // could alias the next loads, for all the compiler knows)
+        const double* __restrict__ pos = s.pos;
+        const int n3 = 3 * s.n_atoms, step = gridDim.x * blockDim.x;
+        for (int i = c; i < n3; i += 3 * step) {
+            double x[3], v[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (i + k * step < n3) {
+                    x[k] = pos[i + k * step];
+                    v[k] = snap.cur_vel[i + k * step];
+                }
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (i + k * step < n3) {
+                    snap.pos[i + k * step] = x[k];
+                    snap.vel[i + k * step] = v[k];
+                }
+        }
+        if (c == 0) *snap.ke = *snap.cur_ke;
+    }
     if (c < s.n_cg) refpos_one(s, c, cg_key);
     if (last_block(s.build_ctr)) {
         if (threadIdx.x < 2) s.sn_max[threadIdx.x] = 0;  // the solute search's list lengths
