@@ -128,6 +128,8 @@ __device__ __forceinline__ void water_record_flush(const SysDev& s, float m, dou
 }
 
 __global__ void k_water_prep(const SysDev* __restrict__ sys) {
+    pdl_wait();
+    pdl_trigger();
     // One thread per solvent molecule in atom order (coalesced position
     // reads); the record goes to the molecule's slot.  Every load is issued
     // before the slot is tested: the coordinates do not depend on it.
@@ -219,7 +221,9 @@ struct SoluteWarp {
 };
 
 template <bool LONG>
-__global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__ sys) {
+__global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__ sys, int beside) {
+    if (!beside) pdl_wait();
+    pdl_trigger();
     const SysDev& s = sys[blockIdx.y];
     const int lane = threadIdx.x & 31;
     const int wpb = blockDim.x >> 5;
@@ -443,6 +447,7 @@ __global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__
 #pragma unroll
     for (int v = 0; v < 9; ++v) idx[v] = 2 * G * G + v;
     block_flush<9>(acc, dst, idx);
+    if (beside) pdl_wait();
 }
 
 // ---------------------------------------------------------------------------
@@ -556,7 +561,9 @@ __device__ __forceinline__ void shared_add(unsigned long long* sh, int idx, doub
 // multi-atom CGs and 11 us for 200 ions (ncu).  Here every value is taken to
 // fixed point by its thread and the warp's integers are summed by shuffles (the
 // same totals), one shared add per warp: 7.2 and 4.6 us.
-__global__ void k_excluded_14(const SysDev* __restrict__ sys) {
+__global__ void k_excluded_14(const SysDev* __restrict__ sys, int beside) {
+    if (!beside) pdl_wait();
+    pdl_trigger();
     const SysDev& s = sys[blockIdx.y];
     const int G = s.n_egroups;
     const int NA = acc_size(G);
@@ -629,6 +636,7 @@ __global__ void k_excluded_14(const SysDev* __restrict__ sys) {
     __syncthreads();
     for (int v = threadIdx.x; v < NA; v += blockDim.x)
         if (sh[v]) atomicAdd(reinterpret_cast<unsigned long long*>(s.acc_short + v), sh[v]);
+    if (beside) pdl_wait();
 }
 
 // perturbed_lj_crf_interaction (perturbed.rs:124-266), FP64.
@@ -914,7 +922,9 @@ __device__ __forceinline__ void pert_terms(const SysDev& s, unsigned long long* 
 
 // All perturbation corrections in one launch: the first term_blocks blocks
 // take the per-atom terms, the others the listed pairs.
-__global__ void __launch_bounds__(128) k_pert(const SysDev* __restrict__ sys, int term_blocks) {
+__global__ void __launch_bounds__(128) k_pert(const SysDev* __restrict__ sys, int term_blocks, int beside) {
+    if (!beside) pdl_wait();
+    pdl_trigger();
     const SysDev& s = sys[blockIdx.y];
     const int NA = acc_size(s.n_egroups);
     extern __shared__ unsigned long long sh[];
@@ -927,10 +937,13 @@ __global__ void __launch_bounds__(128) k_pert(const SysDev* __restrict__ sys, in
     __syncthreads();
     for (int v = threadIdx.x; v < NA; v += blockDim.x)
         if (sh[v]) atomicAdd(reinterpret_cast<unsigned long long*>(s.acc_short + v), sh[v]);
+    if (beside) pdl_wait();
 }
 
 // Fixed point -> FP64 results.  plain != 0 adds the FP32 baseline buffers.
 __global__ void k_finalize(const SysDev* __restrict__ sys, int plain) {
+    pdl_wait();
+    pdl_trigger();
     // One thread per force component; a water atom's component also gathers
     // its cluster slot's sum (solvent CG w = atoms nsa + 3w .. nsa + 3w + 2).
     // The descriptor's fields are read into registers first and every load is
@@ -1012,8 +1025,8 @@ __global__ void k_finalize_plain_energies(const SysDev* __restrict__ sys) {
 }
 
 // Explicit instantiations used by the host runtime.
-template __global__ void k_solute_force<false>(const SysDev*);
-template __global__ void k_solute_force<true>(const SysDev*);
+template __global__ void k_solute_force<false>(const SysDev*, int);
+template __global__ void k_solute_force<true>(const SysDev*, int);
 
 }  // namespace gnb
 

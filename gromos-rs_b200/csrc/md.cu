@@ -236,6 +236,8 @@ __device__ __forceinline__ void md_unit(const SysDev& s, const MdDev& md, int a0
 
 template <bool FUSED>
 __global__ void __launch_bounds__(128) k_md_step(const SysDev* __restrict__ sys, MdDev md) {
+    pdl_wait();
+    pdl_trigger();
     const SysDev& s = *sys;
     const int nsa = s.n_solute_atoms, n = s.n_atoms;
     const int n_units = md.settle ? nsa + (n - nsa) / 3 : n;
@@ -418,10 +420,10 @@ gr_status NbSystem::md_step_launch(cudaStream_t s, bool fuse_prep) {
     const unsigned bt = n_units <= 128 * sm_count() ? 64 : 128;
     const unsigned grid = std::max(1u, std::min(unsigned((n_units + bt - 1) / bt), unsigned(sm_count() * 8)));
     if (prm.kernel == GR_KERNEL_FIXED) {
-        (++launches, k_md_step<true><<<grid, bt, 0, s>>>(d_sys, md));
+        GR_CUDA(launch(k_md_step<true>, grid, bt, 0, s, d_sys, md));
         acc_clean = true;  // the step leaves the short-range accumulators zero
     } else {
-        (++launches, k_md_step<false><<<grid, bt, 0, s>>>(d_sys, md));
+        GR_CUDA(launch(k_md_step<false>, grid, bt, 0, s, d_sys, md));
     }
     return GR_OK;
 }

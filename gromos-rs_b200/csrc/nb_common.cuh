@@ -228,6 +228,19 @@ __device__ __forceinline__ void red_add(long long* addr, long long v) {
     if (v != 0) asm volatile("red.global.add.u64 [%0], %1;" ::"l"(addr), "l"(v) : "memory");
 }
 
+// Programmatic dependent launch: a kernel launched with the attribute starts
+// while its predecessor in the stream still runs.  pdl_wait() returns when the
+// predecessors have completed and their writes are visible; pdl_trigger() lets
+// the successor start once every block has called it (or ended).  Without the
+// attribute both do nothing.  Every kernel launched so calls pdl_wait before it
+// touches memory and then pdl_trigger -- except the ones that only add to
+// fixed-point sums beside the water kernel (`beside` below), which wait at
+// their end: they start when every block of the kernel before them has passed
+// its own wait, so what they read is complete, and their end still means that
+// everything before them has ended.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

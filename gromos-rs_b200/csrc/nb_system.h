@@ -44,6 +44,8 @@ class NbSystem {
     void dev_free(void* p);
     cudaStream_t mem_stream = nullptr;  // the context's stream: pool allocations and releases are ordered on it
     cudaError_t record_event(cudaEvent_t e, cudaStream_t s);
+    template <class... P, class... A>
+    cudaError_t launch(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, A... args);
     int sm_count();
     // Resident blocks per SM of `kernel` at this launch shape, looked up once
     // per context: function attributes (the dynamic shared-memory opt-in) and
@@ -135,6 +137,7 @@ class NbSystem {
     int e_dl_n = 0;
     cudaEvent_t ev_step = nullptr;
     bool step_check = false;
+    bool pdl = false;         // this evaluation's kernels start while their predecessors end (see eval)
     bool in_capture = false;  // recording a CUDA graph: the device descriptor is already current
     bool last_staged = false; // the last timed evaluation recorded its stage events (kernel by kernel)
     bool prep_in_acc = false; // the accumulators hold the energies of water records written by the last MD step

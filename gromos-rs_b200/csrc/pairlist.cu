@@ -174,6 +174,8 @@ __device__ __forceinline__ bool last_block(int* ctr) {
 // three copies of their own between the steps.
 __global__ void k_refpos(const SysDev* __restrict__ sys, unsigned long long* __restrict__ cg_key,
                          const MdSnapshot snap) {
+    pdl_wait();
+    pdl_trigger();
     const SysDev& s = sys[blockIdx.y];
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (snap.pos) {
@@ -211,6 +213,8 @@ __global__ void k_refpos(const SysDev* __restrict__ sys, unsigned long long* __r
 }
 
 __global__ void k_scatter(const SysDev* __restrict__ sys, const unsigned long long* __restrict__ cg_key) {
+    pdl_wait();
+    pdl_trigger();
     const SysDev& s = sys[blockIdx.y];
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= s.n_cg) return;
@@ -224,6 +228,8 @@ __global__ void k_scatter(const SysDev* __restrict__ sys, const unsigned long lo
 // with the sorted CG maps and the sorted FP64 reference positions.  The last
 // block scans the cells' cluster counts into cluster starts.
 __global__ void __launch_bounds__(256) k_cell_sort(const SysDev* __restrict__ sys) {
+    pdl_wait();
+    pdl_trigger();
     const SysDev& s = sys[blockIdx.y];
     __shared__ unsigned long long sk[kMaxCellCGs];
     __shared__ int nsol;
@@ -293,6 +299,8 @@ __global__ void __launch_bounds__(256) k_cell_sort(const SysDev* __restrict__ sy
 // cluster's lanes, its record and search geometry (FP64 first atom, bounding
 // box of the first atoms, radius of the offsets).
 __global__ void __launch_bounds__(256) k_cluster_setup(const SysDev* __restrict__ sys) {
+    pdl_wait();
+    pdl_trigger();
     const SysDev& s = sys[blockIdx.y];
     const int cell = blockIdx.x;
     const int W = s.W;  // 4 or 8: a cluster's lanes are an aligned group
@@ -379,6 +387,8 @@ __global__ void __launch_bounds__(256) k_cluster_setup(const SysDev* __restrict_
 // are about equally long.  The lists are placed by an atomic counter: where
 // a list lies does not change what it holds.
 __global__ void __launch_bounds__(256) k_cell_candidates(const SysDev* __restrict__ sys) {
+    pdl_wait();
+    pdl_trigger();
     const SysDev& s = sys[0];
     const int cell = blockIdx.x, par = blockIdx.y;
     constexpr int kSegs = 29;  // runs A and B, 27 stencil lanes
@@ -607,6 +617,8 @@ __device__ __forceinline__ void sort_write_entries_pop(const uint32_t* __restric
 
 template <int W, bool POPSORT>
 __global__ void __launch_bounds__(kSearchWarps * 32, W == 4 ? 8 : 4) k_water_search(const SysDev* __restrict__ sys, const SearchParams P) {
+    pdl_wait();
+    pdl_trigger();
     const SysDev& s = sys[blockIdx.y];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     __shared__ uint32_t ebuf_s[kSearchWarps][kEntBuf], ebuf_l[kSearchWarps][kEntBuf];
@@ -912,16 +924,20 @@ __device__ __forceinline__ unsigned long long excl_mask_warp(const SysDev& s, in
 // back, so that the force kernel of either range reads only its own.
 // Exclusion masks are only looked up for the CGs that share an excluded or
 // 1-4 pair with this one (cgx, from the topology), after the sweep, one
-// warp per mask.
+// warp per mask.  The kernel needs nothing of the water search and runs beside
+// it (nb_common.cuh, pdl_wait).
 constexpr int kSoluteSearchWarps = 8;
 constexpr int kMaskQueue = 64;
 
-__global__ void __launch_bounds__(kSoluteSearchWarps * 32) k_solute_search(const SysDev* __restrict__ sys) {
+__global__ void __launch_bounds__(kSoluteSearchWarps * 32) k_solute_search(const SysDev* __restrict__ sys, int beside) {
+    if (!beside) pdl_wait();
+    pdl_trigger();
     const SysDev& s = sys[blockIdx.y];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int ci = blockIdx.x;
     if (s.cg_off[ci + 1] - s.cg_off[ci] > kMaxCGAtoms) {
         if (threadIdx.x == 0) atomicOr(&s.err[0], ERR_CG_TOO_LARGE);
+        if (beside) pdl_wait();
         return;
     }
     __shared__ int seg_lo[27], seg_pre[28];
@@ -1050,12 +1066,15 @@ __global__ void __launch_bounds__(kSoluteSearchWarps * 32) k_solute_search(const
         atomicMax(&s.sn_max[0], cnt_s);
         atomicMax(&s.sn_max[1], cnt_l);
     }
+    if (beside) pdl_wait();
 }
 
 // Explicit list of atom pairs that the FEP correction visits: pairs of the
 // solute lists whose first atom (the atom of the lower-index CG) is
 // perturbed (perturbed.rs:324-332).  One thread per (solute CG, entry).
 __global__ void k_pert_pairs(const SysDev* __restrict__ sys) {
+    pdl_wait();
+    pdl_trigger();
     const SysDev& s = sys[blockIdx.y];
     int gid = blockIdx.x * blockDim.x + threadIdx.x;
     int ci = gid / s.scap, e = gid % s.scap;

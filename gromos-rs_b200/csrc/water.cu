@@ -331,6 +331,8 @@ constexpr int kWaterWarps = 4;
 // copied while the current cluster's forces are reduced.
 template <bool LJ00, bool LONG>
 __global__ void __launch_bounds__(128, 4) k_water_force(const SysDev* __restrict__ sys, const WaterParams wp) {
+    pdl_wait();
+    pdl_trigger();
     constexpr int W = 4;
     const SysDev& s = sys[blockIdx.y];
     const int lane = threadIdx.x & 31;
@@ -950,6 +952,8 @@ __device__ __forceinline__ void packed_column_sums(const float4* __restrict__ fi
 template <int W, bool LJ00, bool LONG, bool PK>
 __global__ void __launch_bounds__(128, 3)
     k_water_force_it(const SysDev* __restrict__ sys, const WaterParams wp, const WaterScaled pp) {
+    pdl_wait();
+    pdl_trigger();
     constexpr int ROW = W * 3 + 1;  // float4 per lane row (+1 keeps 8 consecutive lanes on distinct banks)
     const SysDev& s = sys[blockIdx.y];
     const int lane = threadIdx.x & 31;
@@ -1351,6 +1355,8 @@ constexpr size_t water_it_smem() {
 // evaluates its own in its last block).
 template <bool LJ00, bool LONG>
 __global__ void __launch_bounds__(128) k_water_deferred(const SysDev* __restrict__ sys, const WaterParams wp) {
+    pdl_wait();
+    pdl_trigger();
     process_deferred<LJ00, LONG>(sys[blockIdx.y], wp, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 

@@ -52,6 +52,8 @@ __device__ __forceinline__ int ps_entry(int r, int ph, int lane) { return 32 * r
 template <bool LJ00>
 __global__ void __launch_bounds__(128, 3)
     k_water_force_ps(const SysDev* __restrict__ sys, const WaterParams wp, const WaterScaled pp) {
+    pdl_wait();
+    pdl_trigger();
     constexpr int W = 4;
     const SysDev& s = sys[blockIdx.y];
     const int lane = threadIdx.x & 31;
