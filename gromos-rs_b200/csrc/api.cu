@@ -780,6 +780,8 @@ gr_status NbSystem::ensure_capacity() {
         if ((st = alloc(&h.slot_cg, size_t(maxc) * W))) return st;
         if ((st = alloc(&h.clus_geo, size_t(maxc)))) return st;
         if ((st = alloc(&h.clus_ext, size_t(maxc)))) return st;
+        if ((st = alloc(&h.clus_tgeo, size_t(maxc)))) return st;
+        if ((st = alloc(&h.clus_text, size_t(maxc)))) return st;
         // each cluster is a candidate in both lists of its own cell and in one
         // list of each of its at most 26 neighbour cells
         h.cand_cap = int(std::min<long long>(28LL * maxc, (1LL << 31) - 1));
@@ -979,7 +981,10 @@ gr_status NbSystem::build_pairlist(cudaStream_t s, bool sync) {
                 P.boxf[k] = h.boxf[k];
                 P.inv_boxf[k] = h.inv_boxf[k];
                 P.half_boxf[k] = h.half_boxf[k];
+                P.wide[k] = 0.25f * h.boxf[k];
             }
+            // members in different images: only a periodic system has them (k_water_search)
+            const bool filter = h.boundary == 1 && std::min({h.gdim[0], h.gdim[1], h.gdim[2]}) >= 3;
             P.c2s = h.c2s;
             P.c2l = h.c2l;
             P.boundary = h.boundary;
@@ -990,18 +995,19 @@ gr_status NbSystem::build_pairlist(cudaStream_t s, bool sync) {
             auto search_grid = [&](int occ) {
                 return unsigned(std::max<long long>(1, std::min<long long>(static_cast<long long>(sm_count()) * occ, need)));
             };
-#define GR_WATER_SEARCH(WW, POP)                                                                            \
+#define GR_WATER_SEARCH(WW, POP, FIL)                                                                       \
     do {                                                                                                    \
         int occ = 1;                                                                                        \
-        GR_CUDA(occupancy(k_water_search<WW, POP>, kSearchWarps * 32, 0, &occ));                            \
-        GR_CUDA(launch(k_water_search<WW, POP>, search_grid(occ), kSearchWarps * 32, 0, s, d_sys, P));      \
+        GR_CUDA(occupancy(k_water_search<WW, POP, FIL>, kSearchWarps * 32, 0, &occ));                       \
+        GR_CUDA(launch(k_water_search<WW, POP, FIL>, search_grid(occ), kSearchWarps * 32, 0, s, d_sys, P)); \
     } while (0)
-            if (layout == 1)
-                GR_WATER_SEARCH(4, false);
-            else if (W == 4)
-                GR_WATER_SEARCH(4, true);
-            else
-                GR_WATER_SEARCH(8, true);
+            if (layout == 1) {
+                if (filter) GR_WATER_SEARCH(4, false, true); else GR_WATER_SEARCH(4, false, false);
+            } else if (W == 4) {
+                if (filter) GR_WATER_SEARCH(4, true, true); else GR_WATER_SEARCH(4, true, false);
+            } else {
+                if (filter) GR_WATER_SEARCH(8, true, true); else GR_WATER_SEARCH(8, true, false);
+            }
 #undef GR_WATER_SEARCH
         }
         if (NSCG > 0)

@@ -10,7 +10,7 @@ __global__ void k_cell_sort(const SysDev* __restrict__ sys);
 __global__ void k_cluster_setup(const SysDev* __restrict__ sys);
 __global__ void k_cell_candidates(const SysDev* __restrict__ sys);
 struct SearchParams;
-template <int W, bool POPSORT>
+template <int W, bool POPSORT, bool FILTER>
 __global__ void k_water_search(const SysDev* __restrict__ sys, const SearchParams P);
 __global__ void k_solute_search(const SysDev* __restrict__ sys, int beside);
 __global__ void k_pert_pairs(const SysDev* __restrict__ sys);

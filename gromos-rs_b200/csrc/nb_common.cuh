@@ -122,10 +122,12 @@ struct SysDev {
     int* cg_spos;              // n_cg: CG -> sorted position
     int* clus_cell;            // cluster -> cell
     int* clus_first;           // cluster -> first sorted position
-    float4* clus_geo;          // cluster: FP32 bounding-box centre, radius of the offsets from the first atom
+    float4* clus_geo;          // cluster: FP32 bounding-box centre, radius of slot_off
     float4* clus_ext;          // cluster: FP32 bounding-box half extents
+    float4* clus_tgeo;         // cluster: the same box with every member in the image nearest to the first
+    float4* clus_text;         // atom (clus_geo / clus_ext take the members' coordinates as they are)
     double* clus_x64;          // cluster*4: FP64 first-atom position (x, y, z, 0)
-    float4* slot_off;          // slot: FP32 offset from the cluster's first atom
+    float4* slot_off;          // slot: FP32 offset from the cluster's first atom, nearest image
     int* clus_n;               // cluster -> #CGs (<= W)
     int* n_clusters;           // [1]
     int max_clusters;
