@@ -390,6 +390,8 @@ gr_status NbSystem::upload(const gr_topology* t) {
     aps = t->atoms_per_solvent;
     fpe = t->four_pi_eps_i;
     h_cg_off.assign(t->cg_offsets, t->cg_offsets + NCG + 1);
+    max_cg = 1;
+    for (int c = 0; c < NSCG; ++c) max_cg = std::max(max_cg, h_cg_off[c + 1] - h_cg_off[c]);
     h_excl_off.assign(t->excl_offsets, t->excl_offsets + N + 1);
     h_excl.assign(t->excl, t->excl + h_excl_off[N]);
     if (t->o14_offsets) {
@@ -1162,7 +1164,9 @@ gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events, bool fin
         const unsigned sgrid = std::max(1u, std::min(blocks_for((long long)NSCG * ((h.scap - 1) / solute_chunk(h.twin != 0) + 1), 4),
                                                      unsigned(sm * 8)));
         const bool beside = pdl && NCG > NSCG;
-        if (NSCG > 0) GR_CUDA(launch(k_solute_force<false>, sgrid, 128, shg, s, d_sys, beside));
+        auto* solute_s = max_cg == 1 ? k_solute_force<false, 1> : max_cg <= 4 ? k_solute_force<false, 4> : k_solute_force<false, 8>;
+        auto* solute_l = max_cg == 1 ? k_solute_force<true, 1> : max_cg <= 4 ? k_solute_force<true, 4> : k_solute_force<true, 8>;
+        if (NSCG > 0) GR_CUDA(launch(solute_s, sgrid, 128, shg, s, d_sys, beside));
         if (stage) GR_CUDA(record_event(ev[2], s));
         if (do_long) {
             GR_CUDA(cudaMemsetAsync(h.f_long, 0, size_t(N) * 3 * sizeof(long long), s));
@@ -1174,7 +1178,7 @@ gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events, bool fin
                 if ((st = launch_water(s, wp, true))) return st;
                 if (stage) GR_CUDA(record_event(evk[3], s));
             }
-            if (NSCG > 0) GR_CUDA(launch(k_solute_force<true>, sgrid, 128, shg, s, d_sys, beside));
+            if (NSCG > 0) GR_CUDA(launch(solute_l, sgrid, 128, shg, s, d_sys, beside));
             lr_computed = true;
             if (stage && NCG > NSCG) evk_long = true;
         }

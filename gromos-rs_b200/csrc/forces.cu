@@ -203,7 +203,11 @@ __device__ __forceinline__ void warp_add_energies(unsigned long long* sh, int G,
 // The kernel is bound by the latency of an item's dependent loads, not by its
 // arithmetic, so an entry of the solvent (uniform solvent: every molecule has
 // the first one's types and charges) needs one level of them after the list:
-// the molecule's nine coordinates, at an address the index gives.  Its
+// the molecule's nine coordinates, at an address the index gives.
+// MAXA bounds the atoms of the i groups (the largest solute CG: 1, up to 4, or
+// up to 8): the per-atom force sums are registers and their loops unrolled code (168
+// registers at 8, 128 at 1; eight replicas with single-atom groups gain 6%, an MD
+// step of 3,000 waters with 200 ions 3%).  The molecule's
 // charges come from the descriptor, the CG's LJ rows against the three
 // solvent sites and its own atoms from shared memory, once per item.  The
 // second round's molecule is loaded while the first one is computed.  200 ions in
@@ -214,13 +218,14 @@ __device__ __forceinline__ void warp_add_energies(unsigned long long* sh, int G,
 // a system of few solute CGs has fewer items than the chip has warps.
 __host__ __device__ constexpr int solute_chunk(bool twin) { return twin ? 32 : 64; }
 
+template <int MAXA>
 struct SoluteWarp {
-    float4 at[kMaxCGAtoms];      // i atoms: offset from the CG's first atom, charge x fpe
-    int2 tg[kMaxCGAtoms];        // LJ row (type x n_types), energy group
-    float4 lj[kMaxCGAtoms * 3];  // c6, c12, 6 c6, 12 c12 against solvent site b at 3 a + b
+    float4 at[MAXA];      // i atoms: offset from the CG's first atom, charge x fpe
+    int2 tg[MAXA];        // LJ row (type x n_types), energy group
+    float4 lj[MAXA * 3];  // c6, c12, 6 c6, 12 c12 against solvent site b at 3 a + b
 };
 
-template <bool LONG>
+template <bool LONG, int MAXA>
 __global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__ sys, int beside) {
     if (!beside) pdl_wait();
     pdl_trigger();
@@ -230,8 +235,8 @@ __global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__
     const int G = s.n_egroups;
     long long* __restrict__ F = LONG ? s.f_long : s.f_short;
     extern __shared__ unsigned long long shg[];  // 2*G*G group energies (fixed)
-    __shared__ SoluteWarp sw_all[4];
-    SoluteWarp& sw = sw_all[threadIdx.x >> 5];
+    __shared__ SoluteWarp<MAXA> sw_all[4];
+    SoluteWarp<MAXA>& sw = sw_all[threadIdx.x >> 5];
     for (int v = threadIdx.x; v < 2 * G * G; v += blockDim.x) shg[v] = 0ull;
     __syncthreads();
     const double* __restrict__ pos = s.pos;
@@ -244,7 +249,9 @@ __global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__
     const bool per_atom = LONG || !s.cg_grouped;
     const float crf2 = s.crf_2cut3i_f, crfc = s.crf_cut_f, crf3 = s.crf_cut3i_f;
     float v6[6] = {0, 0, 0, 0, 0, 0};
-    long long vfix[6] = {0, 0, 0, 0, 0, 0};
+    __shared__ long long vfix[6][128];  // per lane, touched once per item
+#pragma unroll
+    for (int v = 0; v < 6; ++v) vfix[v][threadIdx.x] = 0;
     int cur_slot = -1;
     float e_lj = 0.f, e_cr = 0.f;
     auto to_slot = [&](int sl) {
@@ -303,9 +310,9 @@ __global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__
             }
         }
         __syncwarp();
-        float fix[kMaxCGAtoms], fiy[kMaxCGAtoms], fiz[kMaxCGAtoms];
+        float fix[MAXA], fiy[MAXA], fiz[MAXA];
 #pragma unroll
-        for (int a = 0; a < kMaxCGAtoms; ++a) fix[a] = fiy[a] = fiz[a] = 0.f;
+        for (int a = 0; a < MAXA; ++a) fix[a] = fiy[a] = fiz[a] = 0.f;
         // one atom pair: i atom a, j atom at its offset (djx, djy, djz) from its CG's
         // first atom, D the imaged vector between the first atoms; g the j force
         auto pair = [&](int a, int aj, float Dx, float Dy, float Dz, float djx, float djy, float djz, float4 c, float qj,
@@ -373,7 +380,7 @@ __global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__
                 for (int b = 0; b < 3; ++b) {
                     float gx = 0.f, gy = 0.f, gz = 0.f;
 #pragma unroll
-                    for (int a = 0; a < kMaxCGAtoms; ++a) {
+                    for (int a = 0; a < MAXA; ++a) {
                         if (a >= ni) break;
                         pair(a, j0 + b, Dx, Dy, Dz, dj[3 * b], dj[3 * b + 1], dj[3 * b + 2], sw.lj[3 * a + b], s.w_q[b],
                              gj, gx, gy, gz);
@@ -400,7 +407,7 @@ __global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__
                     const float qj = float(charge[aj]);
                     float gx = 0.f, gy = 0.f, gz = 0.f;
 #pragma unroll
-                    for (int a = 0; a < kMaxCGAtoms; ++a) {
+                    for (int a = 0; a < MAXA; ++a) {
                         if (a >= ni) break;
                         if (xm & (1ull << (a * 8 + b))) continue;
                         const float2 c = s.lj32[sw.tg[a].x + tj];
@@ -417,7 +424,7 @@ __global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__
         }
         __syncwarp();
 #pragma unroll
-        for (int a = 0; a < kMaxCGAtoms; ++a) {
+        for (int a = 0; a < MAXA; ++a) {
             if (a >= ni) break;
             const float vx = warp_sum(fix[a]), vy = warp_sum(fiy[a]), vz = warp_sum(fiz[a]);
             if (lane == a) {
@@ -431,7 +438,7 @@ __global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__
         cur_slot = -1;
 #pragma unroll
         for (int v = 0; v < 6; ++v) {
-            vfix[v] += to_fixed_f(v6[v], kE);
+            vfix[v][threadIdx.x] += to_fixed_f(v6[v], kE);
             v6[v] = 0.f;
         }
     }
@@ -441,7 +448,7 @@ __global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__
         if (shg[v]) atomicAdd(reinterpret_cast<unsigned long long*>(dst + v), shg[v]);
     long long vs[6];
 #pragma unroll
-    for (int v = 0; v < 6; ++v) vs[v] = warp_sum_ll(vfix[v]);
+    for (int v = 0; v < 6; ++v) vs[v] = warp_sum_ll(vfix[v][threadIdx.x]);
     long long acc[9] = {vs[0], vs[1], vs[2], vs[1], vs[3], vs[4], vs[2], vs[4], vs[5]};
     int idx[9];
 #pragma unroll
@@ -1025,8 +1032,12 @@ __global__ void k_finalize_plain_energies(const SysDev* __restrict__ sys) {
 }
 
 // Explicit instantiations used by the host runtime.
-template __global__ void k_solute_force<false>(const SysDev*, int);
-template __global__ void k_solute_force<true>(const SysDev*, int);
+template __global__ void k_solute_force<false, 8>(const SysDev*, int);
+template __global__ void k_solute_force<true, 8>(const SysDev*, int);
+template __global__ void k_solute_force<false, 4>(const SysDev*, int);
+template __global__ void k_solute_force<true, 4>(const SysDev*, int);
+template __global__ void k_solute_force<false, 1>(const SysDev*, int);
+template __global__ void k_solute_force<true, 1>(const SysDev*, int);
 
 }  // namespace gnb
 

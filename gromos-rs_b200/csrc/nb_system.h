@@ -64,6 +64,7 @@ class NbSystem {
 
     // sizes
     int N = 0, NCG = 0, NSCG = 0, NSA = 0, NT = 0, G = 1, aps = 3, W = 4, layout = 2;
+    int max_cg = 1;  // atoms of the largest solute CG
     int n_pert = 0, solvent_group = -1;
     double fpe = 138.9354;
     double w_qq_sum = 0.0;  // sum over a solvent molecule's atom pairs of q_a q_b fpe
