@@ -43,7 +43,8 @@ constexpr float kE = 16777216.0f;     // energy / virial fixed-point scale (2^24
 // this member pulls into L2; returns the molecule's extent in m and adds its
 // excluded-pair RF energies (-q_i q_j fpe crf_2cut3i r^2, rf_excluded_interactions,
 // excluded.rs:81-96) to e_excl.  Used by k_water_prep and, for the next step,
-// by the MD step kernel.
+// by the MD step kernel (the tiled one clears the force sums itself: CLEAR false).
+template <bool CLEAR = true>
 __device__ __forceinline__ void water_record(const SysDev& s, int slot, const double (&p)[9], const double (&q3)[3],
                                              bool excl, double& e_excl, float& m) {
     // descriptor fields first: the stores below go through pointers the
@@ -88,9 +89,11 @@ __device__ __forceinline__ void water_record(const SysDev& s, int slot, const do
     wrec[slot] = w;
     // the slot's short-range force sums start at zero for this evaluation
     // (only slots that hold a water are ever added to or read)
-    long long* __restrict__ fz = fs_short + static_cast<size_t>(slot) * 9;
+    if (CLEAR) {
+        long long* __restrict__ fz = fs_short + static_cast<size_t>(slot) * 9;
 #pragma unroll
-    for (int c = 0; c < 9; ++c) fz[c] = 0;
+        for (int c = 0; c < 9; ++c) fz[c] = 0;
+    }
     // the member k of a cluster pulls line k of the cluster's short list
     // into L2 for the force kernel (the list was written at the last rebuild)
     const int k = slot % W;

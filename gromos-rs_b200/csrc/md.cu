@@ -24,7 +24,7 @@ struct MdDev {
     const double* mass;       // n_atoms
     double dt, dt_i;
     int settle;               // SETTLE every solvent molecule
-    double m_o, m_h, ra, rb, rc;  // canonical SETTLE triangle (constraints.rs:836-840)
+    double m_o, m_h, im_o, im_h, ra, rb, rc;  // canonical SETTLE triangle (constraints.rs:836-840)
     long long* ke;            // [5]: [0] kinetic energy of the velocities entering the step, [1] accumulator
                               // of the velocities leaving it (fixed point 2^24), [2] blocks finished,
                               // [3] excluded energies and [4] largest extent of the next step's records
@@ -234,21 +234,10 @@ __device__ __forceinline__ void md_unit(const SysDev& s, const MdDev& md, int a0
     for (int k = 0; k < NA; ++k) md_store<FUSED>(s, md, f_out, a0 + k, f[k], nw[k], v[k], mass[k], pa, r.ke);
 }
 
+// The end of a step kernel: the block's sums and, by the last block to finish,
+// the step's energies and the counters.  Every thread of every block calls it.
 template <bool FUSED>
-__global__ void __launch_bounds__(128) k_md_step(const SysDev* __restrict__ sys, MdDev md) {
-    pdl_wait();
-    pdl_trigger();
-    const SysDev& s = *sys;
-    const int nsa = s.n_solute_atoms, n = s.n_atoms;
-    const int n_units = md.settle ? nsa + (n - nsa) / 3 : n;
-    const double lambda = berendsen_lambda(md);
-    MdUnit r{0, 0.0, 0.f};
-    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < n_units; u += gridDim.x * blockDim.x) {
-        if (md.settle && u >= nsa)
-            md_unit<FUSED, 3>(s, md, nsa + 3 * (u - nsa), lambda, r);
-        else
-            md_unit<FUSED, 1>(s, md, u, lambda, r);
-    }
+__device__ __forceinline__ void md_step_end(const SysDev& s, const MdDev& md, const MdUnit& r) {
     // per-block sums: kinetic energy, the records' energies and extent
     __shared__ unsigned long long sh[2];
     __shared__ int mx, last;
@@ -304,6 +293,147 @@ __global__ void __launch_bounds__(128) k_md_step(const SysDev* __restrict__ sys,
         if (FUSED)
             for (int k = 0; k < 6; ++k) s.n_deferred[k] = 0;
     }
+}
+
+template <bool FUSED>
+__global__ void __launch_bounds__(128) k_md_step(const SysDev* __restrict__ sys, MdDev md) {
+    pdl_wait();
+    pdl_trigger();
+    const SysDev& s = *sys;
+    const int nsa = s.n_solute_atoms, n = s.n_atoms;
+    const int n_units = md.settle ? nsa + (n - nsa) / 3 : n;
+    const double lambda = berendsen_lambda(md);
+    MdUnit r{0, 0.0, 0.f};
+    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < n_units; u += gridDim.x * blockDim.x) {
+        if (md.settle && u >= nsa)
+            md_unit<FUSED, 3>(s, md, nsa + 3 * (u - nsa), lambda, r);
+        else
+            md_unit<FUSED, 1>(s, md, u, lambda, r);
+    }
+    md_step_end<FUSED>(s, md, r);
+}
+
+constexpr int kTile = 128;
+
+// The fused step with SETTLE for a system that fills the chip (md_step_launch):
+// a block takes kTile molecules, whose positions, velocities and force sums come
+// in component by component, neighbouring threads on neighbouring addresses, and go
+// through shared memory to the molecule's thread and back.  There a thread
+// that reads its molecule's 72-byte rows itself touches a sector per lane with
+// every load, and these set the time; a smaller system's time is the latency
+// of one molecule, to which the tile only adds barriers.  All loads of a
+// stage are issued before its first store, which they might alias.
+__global__ void __launch_bounds__(kTile) k_md_step_tiled(const SysDev* __restrict__ sys, MdDev md) {
+    pdl_wait();
+    pdl_trigger();
+    const SysDev& s = *sys;
+    const int nsa = s.n_solute_atoms, nscg = s.n_solute_cg, n_mol = (s.n_atoms - nsa) / 3;
+    const bool twin = s.twin != 0, excl = s.excl_atoms < s.n_atoms;
+    const bool pa = nscg > 0 || s.excl_atoms > nsa || s.n_pert > 0 || s.n_pp > 0;  // as in md_unit
+    const double lambda = berendsen_lambda(md);
+    const double inv = 1.0 / kForceScale;
+    MdUnit r{0, 0.0, 0.f};
+    for (int u = blockIdx.x * kTile + threadIdx.x; u < nsa; u += gridDim.x * kTile)
+        md_unit<true, 1>(s, md, u, lambda, r);
+    __shared__ double sx[kTile * 9], sv[kTile * 9], sf[kTile * 9];
+    __shared__ int sslot[kTile];
+    double* f_out = s.f_out;
+    double* pos = s.pos;
+    double* vel = md.vel;
+    const int t = threadIdx.x;
+    for (int base = blockIdx.x * kTile; base < n_mol; base += gridDim.x * kTile) {
+        const int cnt = min(kTile, n_mol - base);
+        const int i0 = 3 * (nsa + 3 * base);  // the tile's first component
+        if (t < cnt) sslot[t] = s.cg_slot[nscg + base + t];
+        double x[9], v9[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const int c = t + k * kTile;
+            x[k] = c < 9 * cnt ? pos[i0 + c] : 0.0;
+            v9[k] = c < 9 * cnt ? vel[i0 + c] : 0.0;
+        }
+        __syncthreads();
+        long long f[9], g[9];
+        size_t o[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const int c = t + k * kTile, m = c / 9;
+            const int slot = c < 9 * cnt ? sslot[m] : -1;
+            o[k] = static_cast<size_t>(slot) * 9 + (c - 9 * m);
+            f[k] = slot >= 0 ? s.fs_short[o[k]] : 0;
+            g[k] = slot >= 0 && twin ? s.fs_long[o[k]] : 0;
+            if (slot < 0) o[k] = ~size_t(0);
+        }
+        if (pa) {
+            long long p[9], q[9];
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+                const int c = t + k * kTile;
+                p[k] = c < 9 * cnt ? s.f_short[i0 + c] : 0;
+                q[k] = c < 9 * cnt && twin ? s.f_long[i0 + c] : 0;
+            }
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+                const int c = t + k * kTile;
+                f[k] += p[k] + q[k];
+                if (c < 9 * cnt) s.f_short[i0 + c] = 0;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const int c = t + k * kTile;
+            if (c >= 9 * cnt) continue;
+            const double fc = double(f[k] + g[k]) * inv;
+            sx[c] = x[k];
+            sv[c] = v9[k];
+            sf[c] = fc;
+            f_out[i0 + c] = fc;
+            if (md.prep_next && o[k] != ~size_t(0)) s.fs_short[o[k]] = 0;  // for the records written below
+        }
+        __syncthreads();
+        if (t < cnt) {
+            D3 old[3], nw[3], v[3];
+            const double im[3] = {md.im_o, md.im_h, md.im_h}, mass[3] = {md.m_o, md.m_h, md.m_h};
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const int c = 9 * t + 3 * k;
+                v[k] = (d3(sv[c], sv[c + 1], sv[c + 2]) + d3(sf[c], sf[c + 1], sf[c + 2]) * im[k] * md.dt) * lambda;
+                old[k] = d3(sx[c], sx[c + 1], sx[c + 2]);
+                nw[k] = old[k] + v[k] * md.dt;
+            }
+            if (!settle_molecule(old, nw, v, md)) atomicAdd(md.failures, 1);
+            const int slot = sslot[t];
+            if (md.prep_next && slot >= 0) {
+                double q3[3] = {0.0, 0.0, 0.0};
+                if (excl)
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) q3[k] = s.charge[nsa + 3 * (base + t) + k];
+                const double p[9] = {nw[0].x, nw[0].y, nw[0].z, nw[1].x, nw[1].y, nw[1].z, nw[2].x, nw[2].y, nw[2].z};
+                water_record<false>(s, slot, p, q3, excl, r.e_excl, r.m_ext);
+            }
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const int c = 9 * t + 3 * k;
+                sx[c] = nw[k].x;
+                sx[c + 1] = nw[k].y;
+                sx[c + 2] = nw[k].z;
+                sv[c] = v[k].x;
+                sv[c + 1] = v[k].y;
+                sv[c + 2] = v[k].z;
+                r.ke += to_fixed_d(0.5 * mass[k] * dot3(v[k], v[k]), kEnergyScale);
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const int c = t + k * kTile;
+            if (c >= 9 * cnt) continue;
+            pos[i0 + c] = sx[c];
+            vel[i0 + c] = sv[c];
+        }
+        __syncthreads();  // the next tile reuses the buffers
+    }
+    md_step_end<true>(s, md, r);
 }
 
 }  // namespace gnb
@@ -402,6 +532,8 @@ gr_status NbSystem::md_step_launch(cudaStream_t s, bool fuse_prep) {
     md.settle = md_settle ? 1 : 0;
     md.m_o = md_m_o;
     md.m_h = md_m_h;
+    md.im_o = md_m_o > 0.0 ? 1.0 / md_m_o : 0.0;  // (SETTLE: every molecule has these masses)
+    md.im_h = md_m_h > 0.0 ? 1.0 / md_m_h : 0.0;
     md.ra = md_ra;
     md.rb = md_rb;
     md.rc = md_rc;
@@ -420,7 +552,10 @@ gr_status NbSystem::md_step_launch(cudaStream_t s, bool fuse_prep) {
     const unsigned bt = n_units <= 128 * sm_count() ? 64 : 128;
     const unsigned grid = std::max(1u, std::min(unsigned((n_units + bt - 1) / bt), unsigned(sm_count() * 8)));
     if (prm.kernel == GR_KERNEL_FIXED) {
-        GR_CUDA(launch(k_md_step<true>, grid, bt, 0, s, d_sys, md));
+        if (md_settle && n_units > 128 * sm_count())
+            GR_CUDA(launch(k_md_step_tiled, grid, kTile, 0, s, d_sys, md));
+        else
+            GR_CUDA(launch(k_md_step<true>, grid, bt, 0, s, d_sys, md));
         acc_clean = true;  // the step leaves the short-range accumulators zero
     } else {
         GR_CUDA(launch(k_md_step<false>, grid, bt, 0, s, d_sys, md));
