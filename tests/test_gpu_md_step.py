@@ -2,6 +2,7 @@
 import numpy as np
 import pytest
 
+import oracle_binding as ob
 from gromos_nb import generators
 from gromos_nb.nonbonded import Forcefield
 
@@ -55,3 +56,26 @@ def test_records_written_ahead_do_not_reach_another_evaluation():
         got = ff.apply(s.pos, force_rebuild=True, graph=graph)
         assert got["e_crf"] == want["e_crf"] and np.array_equal(got["forces"], want["forces"])
         ff.close()
+
+
+def test_tiled_step_of_a_large_system():
+    """More than 128 units per SM take the tiled step kernel: a last tile that is not full, solute atoms
+    before the molecules, steps inside a pairlist period and across its end."""
+    s = generators.solvated_solute_system(19411, 7, seed=14, single_atom_cgs=True)
+    s.params.rcutp, s.params.rcutl = 0.8, 1.0
+    m = generators.masses(s)
+    v = generators.maxwell_velocities(m, 300.0, 3)
+    ff, ref = start(s), start(s)
+    ff.md_run(4)
+    ref.md_run(4)
+    ff.md_run(1)
+    got, want = ff.result(), ref.apply(ref.md_state()[0])
+    assert np.array_equal(got["forces"], want["forces"]) and got["e_crf"] == want["e_crf"]
+    st = ff.md_run(1)
+    x, vel = ff.md_state()
+    ox, ov, so = ob.OracleForcefield(s).md_run(s.pos, v, m, 6, dist_hh=generators.SPC_DHH)
+    # the bounds of the MD parity tests (FP32 pair forces over some ten steps)
+    assert np.abs(x - ox).max() <= 1e-5 and np.linalg.norm(vel - ov) <= 1e-4 * np.linalg.norm(ov)
+    assert abs(st["e_kin"] - so["e_kin"]) <= 1e-5 * so["e_kin"] and st["settle_failures"] == 0
+    ff.close()
+    ref.close()

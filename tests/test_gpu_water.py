@@ -1,10 +1,13 @@
-"""GPU: the solvent kernels at their edges (lists shared by several warps, the search's buffers, clusters in
-several periodic images, long-range pairs near half a box edge), against the FP64 oracle."""
+"""GPU: the solvent kernels at their edges (clusters with members in several periodic images, long-range
+pairs near half a box edge), against the FP64 oracle."""
 import numpy as np
 import pytest
 
+import oracle_binding as ob
 from gromos_nb import generators
-from test_gpu_parity import check_pairlist, compare_eval
+from gromos_nb.nonbonded import Forcefield
+from gromos_nb.system import System
+from test_gpu_parity import compare_eval, sorted_pairs
 
 pytestmark = pytest.mark.gpu
 
@@ -15,3 +18,22 @@ pytestmark = pytest.mark.gpu
 def test_long_range_images_in_small_boxes(waters, rcutp, rcutl, width):
     s = generators.spc_water_system(waters, generators.box_for_waters(waters), 9, rcutp=rcutp, rcutl=rcutl)
     compare_eval(s, steps=2, move=0.001, cluster_size=width)
+
+
+# a seam through a layer of cells and molecules up to two boxes away: clusters with members in
+# several periodic images; boxes of 2 (1,000 waters at 1.4 nm) and 3 cells per axis and more
+@pytest.mark.parametrize("waters,rcutp,rcutl,layout,width", [(1000, 1.4, 1.4, 0, 0), (1000, 0.8, 1.0, 0, 8),
+                                                             (3000, 0.8, 1.4, 0, 0), (3000, 1.4, 1.4, 1, 0)])
+def test_lists_of_clusters_in_several_images(waters, rcutp, rcutl, layout, width):
+    s = generators.spc_water_system(waters, generators.box_for_waters(waters), 6, rcutp=rcutp, rcutl=rcutl)
+    rng = np.random.default_rng(waters)
+    for away in (0, 2):
+        x = s.pos + np.array([0.37, -0.21, 0.5]) * s.box[0]
+        x = x + np.repeat(rng.integers(-away, away + 1, (waters, 3)), 3, axis=0) * s.box
+        ref = ob.pairlist(System(s.topo, x, s.box, s.params), algorithm=2)
+        ff = Forcefield(s, water_layout=layout, cluster_size=width)
+        ff.upload_positions(x)
+        ff.build_pairlist()
+        for got, want in zip(ff.pairlist_lists(), ref):
+            assert np.array_equal(sorted_pairs(got), sorted_pairs(want))
+        ff.close()
