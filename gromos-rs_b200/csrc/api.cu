@@ -1005,6 +1005,17 @@ gr_status NbSystem::build_pairlist(cudaStream_t s, bool sync) {
     } while (0)
             if (layout == 1) {
                 if (filter) GR_WATER_SEARCH(4, false, true); else GR_WATER_SEARCH(4, false, false);
+            } else if (W == 4 && !(in_capture && crowded) && h.max_clusters <= kBlockClusters) {
+                int occ = 1;
+                if (filter) {
+                    GR_CUDA(occupancy(k_water_search_block<true>, kSearchWarps * 32, 0, &occ));
+                    GR_CUDA(launch(k_water_search_block<true>, std::min(h.max_clusters, sm_count() * occ), kSearchWarps * 32,
+                                   0, s, d_sys, P));
+                } else {
+                    GR_CUDA(occupancy(k_water_search_block<false>, kSearchWarps * 32, 0, &occ));
+                    GR_CUDA(launch(k_water_search_block<false>, std::min(h.max_clusters, sm_count() * occ), kSearchWarps * 32,
+                                   0, s, d_sys, P));
+                }
             } else if (W == 4) {
                 if (filter) GR_WATER_SEARCH(4, true, true); else GR_WATER_SEARCH(4, true, false);
             } else {
@@ -1289,6 +1300,7 @@ gr_status NbSystem::eval_graph(cudaStream_t s, int flags) {
         const bool built0 = built, lr0 = lr_computed;
         const long long l0 = launches;
         in_capture = true;
+        crowded = false;
         for (int v = 0; v < 2 && !st; ++v) {
             steps_since_update = v ? prm.nsnb : 1;
             built = true;

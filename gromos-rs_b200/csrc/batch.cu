@@ -147,7 +147,15 @@ gr_status batch_capture_graphs(gr_batch* b) {
     }
     GR_CUDA(cudaMemcpy(b->d_errp, errp.data(), sizeof(int*) * n, cudaMemcpyHostToDevice));
     for (auto& mb : b->m) GR_CUDA(cudaStreamSynchronize(mb.ctx->stream));
-    for (auto& mb : b->m) mb.ctx->sys.in_capture = true;
+    // Members that fill the chip between them (16 clusters per SM, the warps that the
+    // water kernel keeps resident) take the water search with the least work, below
+    // that the one with the shortest way from start to end (k_water_search_block).
+    long long clusters = 0;
+    for (auto& mb : b->m) clusters += mb.ctx->sys.h.max_clusters;
+    for (auto& mb : b->m) {
+        mb.ctx->sys.in_capture = true;
+        mb.ctx->sys.crowded = clusters > 16LL * mb.ctx->sys.sm_count();
+    }
     std::vector<long long> launches0(n);  // recording is not launching: restored below
     for (int i = 0; i < n; ++i) launches0[i] = b->m[i].ctx->sys.launches;
     b->g.assign(b->nsnb, nullptr);

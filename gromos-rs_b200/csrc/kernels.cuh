@@ -12,6 +12,8 @@ __global__ void k_cell_candidates(const SysDev* __restrict__ sys);
 struct SearchParams;
 template <int W, bool POPSORT, bool FILTER>
 __global__ void k_water_search(const SysDev* __restrict__ sys, const SearchParams P);
+template <bool FILTER>
+__global__ void k_water_search_block(const SysDev* __restrict__ sys, const SearchParams P);
 __global__ void k_solute_search(const SysDev* __restrict__ sys, int beside);
 __global__ void k_pert_pairs(const SysDev* __restrict__ sys);
 __global__ void k_expand_cgpairs(const SysDev* __restrict__ sys, int long_range);

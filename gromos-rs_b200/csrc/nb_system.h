@@ -140,6 +140,7 @@ class NbSystem {
     bool step_check = false;
     bool pdl = false;         // this evaluation's kernels start while their predecessors end (see eval)
     bool in_capture = false;  // recording a CUDA graph: the device descriptor is already current
+    bool crowded = false;     // ... a batch's, whose members fill the chip between them
     bool last_staged = false; // the last timed evaluation recorded its stage events (kernel by kernel)
     bool prep_in_acc = false; // the accumulators hold the energies of water records written by the last MD step
     bool prepped_next = false; // the last MD step wrote this evaluation's water records (k_water_prep skipped)

@@ -654,6 +654,159 @@ __device__ __forceinline__ void sort_write_entries_pop(const uint32_t* __restric
     }
 }
 
+// W bits per member m of a lane's j-cluster.
+template <int W>
+using SearchMask = std::conditional_t<W == 4, uint32_t, unsigned long long>;
+
+// FP32 bounds of the search: the band around either cutoff whose members are
+// decided in FP64, the box tests' reach, the certain-image limits.
+struct SearchBounds {
+    float s_lo, s_hi, l_lo, l_hi, rcl, limx, limy, limz;
+};
+
+__device__ __forceinline__ SearchBounds search_bounds(const SearchParams& P) {
+    SearchBounds B;
+    const float c2s = float(P.c2s), c2l = float(P.c2l);
+    B.s_lo = c2s * (1.f - 1e-5f);
+    B.s_hi = c2s * (1.f + 1e-5f);
+    B.l_lo = c2l * (1.f - 1e-5f);
+    B.l_hi = c2l * (1.f + 1e-5f);
+    B.rcl = sqrtf(c2l) * (1.f + 1e-6f) + 1e-3f;
+    B.limx = P.boundary ? P.half_boxf[0] - 1e-4f : 3e38f;
+    B.limy = P.boundary ? P.half_boxf[1] - 1e-4f : 3e38f;
+    B.limz = P.boundary ? P.half_boxf[2] - 1e-4f : 3e38f;
+    return B;
+}
+
+// The gap between two clusters' boxes (centres g, half extents h) is within reach.
+__device__ __forceinline__ bool boxes_near(const SearchParams& P, float rcl, float4 gi, float4 hi, float4 gj, float4 hj) {
+    float dx = gi.x - gj.x, dy = gi.y - gj.y, dz = gi.z - gj.z;
+    if (P.boundary) {
+        dx -= P.boxf[0] * rintf(dx * P.inv_boxf[0]);
+        dy -= P.boxf[1] * rintf(dy * P.inv_boxf[1]);
+        dz -= P.boxf[2] * rintf(dz * P.inv_boxf[2]);
+    }
+    dx = fmaxf(fabsf(dx) - hi.x - hj.x, 0.f);
+    dy = fmaxf(fabsf(dy) - hi.y - hj.y, 0.f);
+    dz = fmaxf(fabsf(dz) - hi.z - hj.z, 0.f);
+    return dx * dx + dy * dy + dz * dz <= rcl * rcl;
+}
+
+__device__ __forceinline__ bool box_wide(const SearchParams& P, float4 h) {
+    return h.x > P.wide[0] || h.y > P.wide[1] || h.z > P.wide[2];
+}
+
+// One lane per surviving j-cluster (active lanes): the cluster-to-cluster
+// vector C (FP64 image of the first atoms, rounded once), then per member m
+// the W x W pair vectors i offset + C - j offset (FP32); the pairs inside the
+// band are decided in FP64.  ms / ml: the member pairs in the short / long
+// range.  Called by the whole warp.
+template <int W>
+__device__ __forceinline__ void classify_survivor(const SysDev& s, const SearchParams& P, const SearchBounds& B, int ci,
+                                                  int n_i, int first_i, double X0, double Y0, double Z0, float rad_i,
+                                                  const float4* ioff, bool active, int jc, float rad_j,
+                                                  SearchMask<W>& ms, SearchMask<W>& ml) {
+    using Mask = SearchMask<W>;
+    constexpr unsigned kRow = (1u << W) - 1u;
+    const float4* __restrict__ soff = s.slot_off;
+    const double* __restrict__ x64 = s.clus_x64;
+    const double* __restrict__ sref = s.sref;
+    const int stride = s.n_cg + 2;
+    const float s_lo = B.s_lo, s_hi = B.s_hi, l_lo = B.l_lo, l_hi = B.l_hi;
+    const float limx = B.limx, limy = B.limy, limz = B.limz;
+    float ex[W], ey[W], ez[W];
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+        const float4 o = ioff[k];
+        ex[k] = o.x;
+        ey[k] = o.y;
+        ez[k] = o.z;
+    }
+    Mask am = 0;
+    ms = ml = 0;
+    if (active) {
+        const int n_j = s.clus_n[jc];
+        const float span = rad_i + rad_j;
+        double cdx = X0 - x64[4 * jc], cdy = Y0 - x64[4 * jc + 1], cdz = Z0 - x64[4 * jc + 2];
+        if (P.boundary) {
+            cdx -= P.box[0] * rint(cdx * P.inv_box[0]);
+            cdy -= P.box[1] * rint(cdy * P.inv_box[1]);
+            cdz -= P.box[2] * rint(cdz * P.inv_box[2]);
+        }
+        const float Cx = float(cdx), Cy = float(cdy), Cz = float(cdz);
+        // |C + i offset - j offset| per axis stays below |C| + both
+        // radii: when that is below half a box edge, the sum is the
+        // minimum image of every member pair
+        const bool edge = P.boundary && !(fabsf(Cx) + span < limx && fabsf(Cy) + span < limy &&
+                                          fabsf(Cz) + span < limz);
+        // pairs {i_k, j_m} with k < n_i, m < n_j and i_k before j_m in sorted order
+        const unsigned valid_i = (1u << n_i) - 1u;
+#pragma unroll
+        for (int m = 0; m < W; ++m) {
+            const float4 o = soff[jc * W + m];
+            float Dx = Cx - o.x, Dy = Cy - o.y, Dz = Cz - o.z;
+            if (edge) {  // the sum of two minimum images need not be one
+                Dx -= P.boxf[0] * rintf(Dx * P.inv_boxf[0]);
+                Dy -= P.boxf[1] * rintf(Dy * P.inv_boxf[1]);
+                Dz -= P.boxf[2] * rintf(Dz * P.inv_boxf[2]);
+            }
+            unsigned valid = m < n_j ? valid_i : 0u;
+            if (jc == ci) valid &= (1u << m) - 1u;
+            unsigned s_m = 0, l_m = 0, a_m = 0;
+#pragma unroll
+            for (int k = 0; k < W; ++k) {
+                const float kx = ex[k] + Dx, ky = ey[k] + Dy, kz = ez[k] + Dz;
+                const float d2 = kx * kx + ky * ky + kz * kz;
+                s_m |= unsigned(d2 < s_lo) << k;
+                l_m |= unsigned(d2 > s_hi && d2 < l_lo) << k;
+                a_m |= unsigned((d2 >= s_lo && d2 <= s_hi) || (d2 >= l_lo && d2 <= l_hi)) << k;
+                if (edge) {
+                    const bool inbox = fabsf(kx) < limx && fabsf(ky) < limy && fabsf(kz) < limz;
+                    a_m |= unsigned(!inbox) << k;
+                }
+            }
+            ms |= Mask(s_m & valid & ~a_m) << (m * W);
+            ml |= Mask(l_m & valid & ~a_m) << (m * W);
+            am |= Mask(a_m & valid) << (m * W);
+        }
+    }
+    // the rare ambiguous pairs: the exact FP64 decision
+    // (nearest_image_exact + len2_exact, box from the kernel
+    // parameters) for the lanes that have some
+    if (__any_sync(0xffffffffu, am != 0) && am) {
+        const int fj = s.clus_first[jc];
+#pragma unroll
+        for (int m = 0; m < W; ++m) {
+            unsigned a = unsigned(am >> (m * W)) & kRow;
+            if (!a) continue;
+            const int sp = fj + m;
+            const double tjx = sref[sp], tjy = sref[stride + sp], tjz = sref[2 * stride + sp];
+            unsigned add_s = 0u, add_l = 0u;
+            while (a) {
+                const int k = __ffs(a) - 1;
+                a &= a - 1u;
+                double rx = __dsub_rn(sref[first_i + k], tjx);
+                double ry = __dsub_rn(sref[stride + first_i + k], tjy);
+                double rz = __dsub_rn(sref[2 * stride + first_i + k], tjz);
+                if (P.boundary) {
+                    rx = image_exact(rx, P.box[0], P.inv_box[0]);
+                    ry = image_exact(ry, P.box[1], P.inv_box[1]);
+                    rz = image_exact(rz, P.box[2], P.inv_box[2]);
+                }
+                const double e2 = len2_exact(rx, ry, rz);
+                if (!(e2 > P.c2l)) {
+                    if (e2 > P.c2s)
+                        add_l |= 1u << k;
+                    else
+                        add_s |= 1u << k;
+                }
+            }
+            ms |= Mask(add_s) << (m * W);
+            ml |= Mask(add_l) << (m * W);
+        }
+    }
+}
+
 template <int W, bool POPSORT, bool FILTER>
 __global__ void __launch_bounds__(kSearchWarps * 32, W == 4 ? 8 : 4) k_water_search(const SysDev* __restrict__ sys, const SearchParams P) {
     pdl_wait();
@@ -667,8 +820,6 @@ __global__ void __launch_bounds__(kSearchWarps * 32, W == 4 ? 8 : 4) k_water_sea
     __shared__ int p_jc[FILTER ? kSearchWarps : 1][32], p_batch[FILTER ? kSearchWarps : 1][32];
     __shared__ float p_sp[FILTER ? kSearchWarps : 1][32];
     __shared__ float4 ioff[kSearchWarps][W];        // the i members' offsets
-    // W bits per member m of a lane's j-cluster: short, long, undecided pairs
-    using Mask = std::conditional_t<W == 4, uint32_t, unsigned long long>;
     constexpr unsigned kRow = (1u << W) - 1u;
     constexpr int kWide = 1 << 30;                  // flag in q_jc (slots stay below 2^24)
     const int nclus = s.n_clusters[0];
@@ -676,15 +827,7 @@ __global__ void __launch_bounds__(kSearchWarps * 32, W == 4 ? 8 : 4) k_water_sea
     const float4* __restrict__ ext = s.clus_ext;
     const float4* __restrict__ soff = s.slot_off;
     const double* __restrict__ x64 = s.clus_x64;
-    const double* __restrict__ sref = s.sref;
-    const int stride = s.n_cg + 2;
-    const float c2s = float(P.c2s), c2l = float(P.c2l);
-    const float s_lo = c2s * (1.f - 1e-5f), s_hi = c2s * (1.f + 1e-5f);
-    const float l_lo = c2l * (1.f - 1e-5f), l_hi = c2l * (1.f + 1e-5f);
-    const float rcl = sqrtf(c2l) * (1.f + 1e-6f) + 1e-3f;
-    const float limx = P.boundary ? P.half_boxf[0] - 1e-4f : 3e38f;
-    const float limy = P.boundary ? P.half_boxf[1] - 1e-4f : 3e38f;
-    const float limz = P.boundary ? P.half_boxf[2] - 1e-4f : 3e38f;
+    const SearchBounds B = search_bounds(P);
     const unsigned below = (1u << lane) - 1u;
     for (;;) {
         int ci = 0;
@@ -713,7 +856,7 @@ __global__ void __launch_bounds__(kSearchWarps * 32, W == 4 ? 8 : 4) k_water_sea
         uint32_t* outl = s.wl_l + static_cast<size_t>(ci) * P.wcap;
         int cnt_s = 0, cnt_l = 0, qn = 0, v0 = 0;
         int np = 0, batch = 0;  // survivors waiting in the group, batches taken so far
-        const bool wide_i = hi.x > P.wide[0] || hi.y > P.wide[1] || hi.z > P.wide[2];
+        const bool wide_i = box_wide(P, hi);
         for (;;) {
             // box tests until 32 survivors are queued or the candidates end
             while (v0 < total && qn < 32) {
@@ -726,19 +869,9 @@ __global__ void __launch_bounds__(kSearchWarps * 32, W == 4 ? 8 : 4) k_water_sea
                     const int pos = v + (v < n_ab ? skip_a : skip_ab);
                     const float4 gj = cgeo[pos], hj = cext[pos];
                     jc = min(max(__float_as_int(hj.w), 0), nclus - 1);
-                    if (FILTER && (hj.x > P.wide[0] || hj.y > P.wide[1] || hj.z > P.wide[2])) jc |= kWide;
+                    if (FILTER && box_wide(P, hj)) jc |= kWide;
                     rj = gj.w;
-                    float dx = gi.x - gj.x, dy = gi.y - gj.y, dz = gi.z - gj.z;
-                    if (P.boundary) {
-                        dx -= P.boxf[0] * rintf(dx * P.inv_boxf[0]);
-                        dy -= P.boxf[1] * rintf(dy * P.inv_boxf[1]);
-                        dz -= P.boxf[2] * rintf(dz * P.inv_boxf[2]);
-                    }
-                    // gap between the two boxes along each axis
-                    dx = fmaxf(fabsf(dx) - hi.x - hj.x, 0.f);
-                    dy = fmaxf(fabsf(dy) - hi.y - hj.y, 0.f);
-                    dz = fmaxf(fabsf(dz) - hi.z - hj.z, 0.f);
-                    surv = dx * dx + dy * dy + dz * dz <= rcl * rcl;
+                    surv = boxes_near(P, B.rcl, gi, hi, gj, hj);
                 }
                 const unsigned b = __ballot_sync(0xffffffffu, surv);
                 if (surv) {
@@ -760,120 +893,23 @@ __global__ void __launch_bounds__(kSearchWarps * 32, W == 4 ? 8 : 4) k_water_sea
             }
             if (FILTER && __any_sync(0xffffffffu, keep && (wide_i || (bj & kWide)))) {
                 bj &= ~kWide;
-                if (keep) {
-                    const float4 ti = s.clus_tgeo[ci], ei = s.clus_text[ci], tj = s.clus_tgeo[bj], ej = s.clus_text[bj];
-                    float dx = ti.x - tj.x, dy = ti.y - tj.y, dz = ti.z - tj.z;
-                    dx -= P.boxf[0] * rintf(dx * P.inv_boxf[0]);  // (there are wide boxes in periodic systems only)
-                    dy -= P.boxf[1] * rintf(dy * P.inv_boxf[1]);
-                    dz -= P.boxf[2] * rintf(dz * P.inv_boxf[2]);
-                    dx = fmaxf(fabsf(dx) - ei.x - ej.x, 0.f);
-                    dy = fmaxf(fabsf(dy) - ei.y - ej.y, 0.f);
-                    dz = fmaxf(fabsf(dz) - ei.z - ej.z, 0.f);
-                    keep = dx * dx + dy * dy + dz * dz <= rcl * rcl;
-                }
+                if (keep) keep = boxes_near(P, B.rcl, s.clus_tgeo[ci], s.clus_text[ci], s.clus_tgeo[bj], s.clus_text[bj]);
             }
             const unsigned kept = __ballot_sync(0xffffffffu, keep);
             const int nk = __popc(kept);
             if (!FILTER && nq == 0) break;
             if (!FILTER || (np > 0 && (nq == 0 || np + nk > 32))) {  // classify the group, or the batch itself
                 const int ng = FILTER ? np : nq;
-                // lane q classifies survivor q: the cluster-to-cluster vector C
-                // (FP64 image of the first atoms, rounded once), then per member
-                // m the W x W pair vectors i offset + C - j offset (FP32)
                 int jc = 0;
-                float ex[W], ey[W], ez[W];
-#pragma unroll
-                for (int k = 0; k < W; ++k) {
-                    const float4 o = ioff[w][k];
-                    ex[k] = o.x;
-                    ey[k] = o.y;
-                    ez[k] = o.z;
-                }
-                Mask ms = 0, ml = 0, am = 0;
+                SearchMask<W> ms, ml;
                 int my_batch = -1;
+                float rad_j = 0.f;
                 if (lane < ng) {
                     jc = FILTER ? p_jc[w][lane] : bj;
                     my_batch = FILTER ? p_batch[w][lane] : 0;
-                    const int n_j = s.clus_n[jc];
-                    const float span = gi.w + (FILTER ? p_sp[w][lane] : bsp);
-                    double cdx = X0 - x64[4 * jc], cdy = Y0 - x64[4 * jc + 1], cdz = Z0 - x64[4 * jc + 2];
-                    if (P.boundary) {
-                        cdx -= P.box[0] * rint(cdx * P.inv_box[0]);
-                        cdy -= P.box[1] * rint(cdy * P.inv_box[1]);
-                        cdz -= P.box[2] * rint(cdz * P.inv_box[2]);
-                    }
-                    const float Cx = float(cdx), Cy = float(cdy), Cz = float(cdz);
-                    // |C + i offset - j offset| per axis stays below |C| + both
-                    // radii: when that is below half a box edge, the sum is the
-                    // minimum image of every member pair
-                    const bool edge = P.boundary && !(fabsf(Cx) + span < limx && fabsf(Cy) + span < limy &&
-                                                      fabsf(Cz) + span < limz);
-                    // pairs {i_k, j_m} with k < n_i, m < n_j and i_k before j_m in sorted order
-                    const unsigned valid_i = (1u << n_i) - 1u;
-#pragma unroll
-                    for (int m = 0; m < W; ++m) {
-                        const float4 o = soff[jc * W + m];
-                        float Dx = Cx - o.x, Dy = Cy - o.y, Dz = Cz - o.z;
-                        if (edge) {  // the sum of two minimum images need not be one
-                            Dx -= P.boxf[0] * rintf(Dx * P.inv_boxf[0]);
-                            Dy -= P.boxf[1] * rintf(Dy * P.inv_boxf[1]);
-                            Dz -= P.boxf[2] * rintf(Dz * P.inv_boxf[2]);
-                        }
-                        unsigned valid = m < n_j ? valid_i : 0u;
-                        if (jc == ci) valid &= (1u << m) - 1u;
-                        unsigned s_m = 0, l_m = 0, a_m = 0;
-#pragma unroll
-                        for (int k = 0; k < W; ++k) {
-                            const float kx = ex[k] + Dx, ky = ey[k] + Dy, kz = ez[k] + Dz;
-                            const float d2 = kx * kx + ky * ky + kz * kz;
-                            s_m |= unsigned(d2 < s_lo) << k;
-                            l_m |= unsigned(d2 > s_hi && d2 < l_lo) << k;
-                            a_m |= unsigned((d2 >= s_lo && d2 <= s_hi) || (d2 >= l_lo && d2 <= l_hi)) << k;
-                            if (edge) {
-                                const bool inbox = fabsf(kx) < limx && fabsf(ky) < limy && fabsf(kz) < limz;
-                                a_m |= unsigned(!inbox) << k;
-                            }
-                        }
-                        ms |= Mask(s_m & valid & ~a_m) << (m * W);
-                        ml |= Mask(l_m & valid & ~a_m) << (m * W);
-                        am |= Mask(a_m & valid) << (m * W);
-                    }
+                    rad_j = FILTER ? p_sp[w][lane] : bsp;
                 }
-                // the rare ambiguous pairs: the exact FP64 decision
-                // (nearest_image_exact + len2_exact, box from the kernel
-                // parameters) for the lanes that have some
-                if (__any_sync(0xffffffffu, am != 0) && am) {
-                    const int fj = s.clus_first[jc];
-#pragma unroll
-                    for (int m = 0; m < W; ++m) {
-                        unsigned a = unsigned(am >> (m * W)) & kRow;
-                        if (!a) continue;
-                        const int sp = fj + m;
-                        const double tjx = sref[sp], tjy = sref[stride + sp], tjz = sref[2 * stride + sp];
-                        unsigned add_s = 0u, add_l = 0u;
-                        while (a) {
-                            const int k = __ffs(a) - 1;
-                            a &= a - 1u;
-                            double rx = __dsub_rn(sref[first_i + k], tjx);
-                            double ry = __dsub_rn(sref[stride + first_i + k], tjy);
-                            double rz = __dsub_rn(sref[2 * stride + first_i + k], tjz);
-                            if (P.boundary) {
-                                rx = image_exact(rx, P.box[0], P.inv_box[0]);
-                                ry = image_exact(ry, P.box[1], P.inv_box[1]);
-                                rz = image_exact(rz, P.box[2], P.inv_box[2]);
-                            }
-                            const double e2 = len2_exact(rx, ry, rz);
-                            if (!(e2 > P.c2l)) {
-                                if (e2 > P.c2s)
-                                    add_l |= 1u << k;
-                                else
-                                    add_s |= 1u << k;
-                            }
-                        }
-                        ms |= Mask(add_s) << (m * W);
-                        ml |= Mask(add_l) << (m * W);
-                    }
-                }
+                classify_survivor<W>(s, P, B, ci, n_i, first_i, X0, Y0, Z0, gi.w, ioff[w], lane < ng, jc, rad_j, ms, ml);
                 // batch by batch, entries of member m of every lane's survivor, compacted in lane order
                 const int first_batch = FILTER ? __shfl_sync(0xffffffffu, my_batch, 0) : 0;
                 const int last_batch = FILTER ? __shfl_sync(0xffffffffu, my_batch, ng - 1) : 0;
@@ -950,6 +986,249 @@ __global__ void __launch_bounds__(kSearchWarps * 32, W == 4 ? 8 : 4) k_water_sea
             s.wn_l[ci] = min(cnt_l, P.wcap);
         }
         __syncwarp();  // the entry buffers and queues are reused by the next cluster
+    }
+}
+
+// The search of a small system: one block per i-cluster, so that a system with
+// fewer clusters than the chip holds warps does not wait for one warp's whole
+// sweep.  The lists are those of k_water_search, entry for entry: the warps test
+// the candidates in turns and compact the survivors in candidate order; batches
+// of 32 of them, the unit of that kernel's order, go to the warps in turns,
+// each batch's entries to its own place in shared memory; the counts per batch
+// and popcount then give every entry its place.  Width 4 and popcount order only,
+// and at most kBlockSurvivors candidates per cluster: a cluster owns half of
+// the others at most, so the host takes this kernel up to kBlockClusters of
+// them (NbSystem::build_pairlist).  What bounds it is the chain from candidate
+// to entry: box test, classification, counts, places.  With 250 to 1,250
+// clusters the warps of k_water_search sit mostly alone on their SMs, and four
+// warps on one cluster shorten the chain: 20 MD steps of 1,000 waters 983 -> 916
+// us, of 3,000 waters + 200 ions 1,311 -> 1,191, 16 frames of 3,000 waters
+// 3,471 -> 3,051, 5 evaluations of 5,000 waters + 200 solute atoms 991 -> 971.
+// The line is the shared memory of 24 batches (32.8 KB a block); the members of
+// a batch that fill the chip between them keep one warp per cluster, as the work
+// counts there (21 windows of 5,000 waters 9,825 us, 10,056 with blocks).
+constexpr int kBlockBatches = 24, kBlockSurvivors = 32 * kBlockBatches;
+constexpr int kBlockClusters = 2 * (kBlockSurvivors - 32);  // own half + 1, and half of each stencil cell rounded up
+
+template <bool FILTER>
+__global__ void __launch_bounds__(kSearchWarps * 32, 6) k_water_search_block(const SysDev* __restrict__ sys,
+                                                                             const SearchParams P) {
+    pdl_wait();
+    pdl_trigger();
+    constexpr int W = 4;
+    const SysDev& s = sys[blockIdx.y];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __shared__ int q_jc[kBlockSurvivors];
+    __shared__ float q_sp[kBlockSurvivors];
+    __shared__ uint32_t ent_s[kBlockBatches][32 * W], ent_l[kBlockBatches][32 * W];
+    __shared__ int n_s[kBlockBatches], n_l[kBlockBatches];
+    __shared__ uint32_t hist_s[kBlockBatches], hist_l[kBlockBatches];  // entries of 4, 3, 2, 1 bits, 8 bits each
+    __shared__ int wcnt[2][kSearchWarps], next;
+    __shared__ int p_jc[kSearchWarps][32], p_batch[kSearchWarps][32];
+    __shared__ float p_sp[kSearchWarps][32];
+    __shared__ float4 ioff[W];
+    constexpr int kWide = 1 << 30;
+    constexpr unsigned kRow = (1u << W) - 1u;
+    const int nclus = s.n_clusters[0];
+    const SearchBounds B = search_bounds(P);
+    const unsigned below = (1u << lane) - 1u;
+    for (;;) {
+        __syncthreads();  // the previous cluster's buffers are read
+        if (threadIdx.x == 0) next = atomicAdd(s.n_deferred + 6, 1);
+        __syncthreads();
+        const int ci = next;
+        if (ci >= nclus) break;
+        const int n_i = s.clus_n[ci], first_i = s.clus_first[ci], cell = s.clus_cell[ci];
+        const float4 gi = s.clus_geo[ci], hi = s.clus_ext[ci];
+        const double X0 = s.clus_x64[4 * ci], Y0 = s.clus_x64[4 * ci + 1], Z0 = s.clus_x64[4 * ci + 2];
+        if (threadIdx.x < W) ioff[threadIdx.x] = s.slot_off[ci * W + threadIdx.x];
+        // the candidates (see k_water_search)
+        const int oc0 = s.cell_nclus[cell], oc1 = min(s.cell_nclus[cell + 1], s.max_clusters);
+        const int a0 = oc0 + ((oc0 - ci) & 1), b0 = oc0 + ((oc0 - ci - 1) & 1);
+        const int len_a = (oc1 - a0 + 1) >> 1, len_b = b0 < oc1 ? (oc1 - b0 + 1) >> 1 : 0;
+        const int skip_a = (ci - a0) >> 1, nb = b0 < ci ? (ci - b0 + 1) >> 1 : 0;
+        const int n_ab = len_a - skip_a + nb, skip_ab = skip_a + len_b - nb;
+        const int lidx = 2 * cell + (ci & 1);
+        const int total = s.cell_ncand[lidx] - skip_ab;
+        const float4* __restrict__ cgeo = s.cand_geo + s.cell_cand[lidx];
+        const float4* __restrict__ cext = s.cand_ext + s.cell_cand[lidx];
+        // box tests, 128 candidates a round
+        int nraw = 0;
+        for (int v0 = 0, par = 0; v0 < total; v0 += kSearchWarps * 32, par ^= 1) {
+            const int v = v0 + threadIdx.x;
+            bool surv = false;
+            int jc = 0;
+            float rj = 0.f;
+            if (v < total) {
+                const int pos = v + (v < n_ab ? skip_a : skip_ab);
+                const float4 gj = cgeo[pos], hj = cext[pos];
+                jc = min(max(__float_as_int(hj.w), 0), nclus - 1);
+                if (FILTER && box_wide(P, hj)) jc |= kWide;
+                rj = gj.w;
+                surv = boxes_near(P, B.rcl, gi, hi, gj, hj);
+            }
+            const unsigned b = __ballot_sync(0xffffffffu, surv);
+            if (lane == 0) wcnt[par][w] = __popc(b);
+            __syncthreads();
+            int before = 0, round = 0;
+#pragma unroll
+            for (int k = 0; k < kSearchWarps; ++k) {
+                if (k < w) before += wcnt[par][k];
+                round += wcnt[par][k];
+            }
+            const int p = nraw + before + __popc(b & below);
+            if (surv && p < kBlockSurvivors) {
+                q_jc[p] = jc;
+                q_sp[p] = rj;
+            }
+            nraw += round;
+        }
+        if (nraw > kBlockSurvivors) {  // cannot be (kBlockClusters); never written past, and never silent
+            if (threadIdx.x == 0) atomicOr(&s.err[0], ERR_WLIST_OVERFLOW);
+            nraw = kBlockSurvivors;
+        }
+        __syncthreads();
+        // classification: this warp's batches, grouped up to 32 survivors
+        const int nbatch = (nraw + 31) >> 5;
+        const bool wide_i = box_wide(P, hi);
+        int np = 0;
+        for (int b = w;; b += kSearchWarps) {
+            const bool end = b >= nbatch;
+            const int q = 32 * b + lane;
+            bool keep = !end && q < nraw;
+            int bj = keep ? q_jc[q] : 0;
+            const float bsp = keep ? q_sp[q] : 0.f;
+            if (FILTER && __any_sync(0xffffffffu, keep && (wide_i || (bj & kWide)))) {
+                bj &= ~kWide;
+                if (keep) keep = boxes_near(P, B.rcl, s.clus_tgeo[ci], s.clus_text[ci], s.clus_tgeo[bj], s.clus_text[bj]);
+            }
+            const unsigned kept = __ballot_sync(0xffffffffu, keep);
+            const int nk = __popc(kept);
+            if (np > 0 && (end || np + nk > 32)) {
+                const int jc = lane < np ? p_jc[w][lane] : 0, my_batch = lane < np ? p_batch[w][lane] : -1;
+                SearchMask<W> ms, ml;
+                classify_survivor<W>(s, P, B, ci, n_i, first_i, X0, Y0, Z0, gi.w, ioff, lane < np, jc,
+                                     lane < np ? p_sp[w][lane] : 0.f, ms, ml);
+                const int last = __shfl_sync(0xffffffffu, my_batch, np - 1);
+                for (int bb = __shfl_sync(0xffffffffu, my_batch, 0); bb <= last; bb += kSearchWarps) {
+                    const bool mine = my_batch == bb;
+                    if (!__any_sync(0xffffffffu, mine)) continue;
+                    int cs = 0, cl = 0;
+#pragma unroll
+                    for (int m = 0; m < W; ++m) {
+                        const uint32_t slot = static_cast<uint32_t>(jc * W + m);
+                        const unsigned row_s = mine ? unsigned(ms >> (m * W)) & kRow : 0u;
+                        const unsigned row_l = mine ? unsigned(ml >> (m * W)) & kRow : 0u;
+                        const unsigned bs = __ballot_sync(0xffffffffu, row_s != 0u);
+                        const unsigned bl = __ballot_sync(0xffffffffu, row_l != 0u);
+                        if (row_s) ent_s[bb][cs + __popc(bs & below)] = (slot << 8) | row_s;
+                        if (row_l) ent_l[bb][cl + __popc(bl & below)] = (slot << 8) | row_l;
+                        cs += __popc(bs);
+                        cl += __popc(bl);
+                    }
+                    if (lane == 0) {
+                        n_s[bb] = cs;
+                        n_l[bb] = cl;
+                    }
+                }
+                np = 0;
+                __syncwarp();
+            }
+            if (end) break;
+            if (keep) {
+                const int p = np + __popc(kept & below);
+                p_jc[w][p] = bj;
+                p_sp[w][p] = bsp;
+                p_batch[w][p] = b;
+            }
+            if (nk == 0 && lane == 0) n_s[b] = n_l[b] = 0;
+            np += nk;
+            __syncwarp();
+        }
+        __syncthreads();
+        // places: entry rank in batch order; the first kEntBuf ranks are sorted by
+        // popcount (most bits first, stable), later ones follow as they come
+        uint32_t* outs = s.wl_s + static_cast<size_t>(ci) * P.wcap;
+        uint32_t* outl = s.wl_l + static_cast<size_t>(ci) * P.wcap;
+        int rank_s = lane < nbatch ? n_s[lane] : 0, rank_l = lane < nbatch ? n_l[lane] : 0;
+        const int own_s = rank_s, own_l = rank_l;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int ys = __shfl_up_sync(0xffffffffu, rank_s, o), yl = __shfl_up_sync(0xffffffffu, rank_l, o);
+            if (lane >= o) {
+                rank_s += ys;
+                rank_l += yl;
+            }
+        }
+        const int all_s = __shfl_sync(0xffffffffu, rank_s, 31), all_l = __shfl_sync(0xffffffffu, rank_l, 31);
+        rank_s -= own_s;
+        rank_l -= own_l;
+        auto class_masks = [&](const uint32_t* buf, int e, bool in, unsigned (&m)[4]) {  // 4, 3, 2, 1 bits
+            const int k = in ? __popc(buf[e] & 0xffu) - 1 : 0;
+            const unsigned bv = __ballot_sync(0xffffffffu, in);
+            const unsigned x0 = __ballot_sync(0xffffffffu, in && (k & 1)), x1 = __ballot_sync(0xffffffffu, in && (k & 2));
+            m[0] = x0 & x1;
+            m[1] = x1 & ~x0;
+            m[2] = x0 & ~x1;
+            m[3] = bv & ~(x0 | x1);
+            return 3 - k;
+        };
+        for (int b = w; b < nbatch; b += kSearchWarps)
+#pragma unroll
+            for (int l = 0; l < 2; ++l) {
+                const int n = l ? n_l[b] : n_s[b], r0 = __shfl_sync(0xffffffffu, l ? rank_l : rank_s, b);
+                uint32_t h = 0;
+                for (int c = 0; c < n; c += 32) {
+                    unsigned m[4];
+                    class_masks(l ? ent_l[b] : ent_s[b], c + lane, c + lane < n && r0 + c + lane < kEntBuf, m);
+                    h += __popc(m[0]) | (__popc(m[1]) << 8) | (__popc(m[2]) << 16) | (uint32_t(__popc(m[3])) << 24);
+                }
+                if (lane == 0) (l ? hist_l : hist_s)[b] = h;
+            }
+        __syncthreads();
+#pragma unroll
+        for (int l = 0; l < 2; ++l) {
+            const uint32_t h = lane < nbatch ? (l ? hist_l : hist_s)[lane] : 0u;
+            int pre[4], base = 0;  // lane b: entries of its class before batch b's, in output order
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int own = int((h >> (8 * k)) & 0xffu);
+                int x = own;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (lane >= o) x += y;
+                }
+                const int sum = __shfl_sync(0xffffffffu, x, 31);
+                pre[k] = base + x - own;
+                base += sum;
+            }
+            uint32_t* __restrict__ out = l ? outl : outs;
+            for (int b = w; b < nbatch; b += kSearchWarps) {
+                const uint32_t* buf = l ? ent_l[b] : ent_s[b];
+                const int n = l ? n_l[b] : n_s[b], r0 = __shfl_sync(0xffffffffu, l ? rank_l : rank_s, b);
+                int at[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) at[k] = __shfl_sync(0xffffffffu, pre[k], b);
+                for (int c = 0; c < n; c += 32) {
+                    const int e = c + lane;
+                    const bool in = e < n && r0 + e < kEntBuf;
+                    unsigned m[4];
+                    const int cls = class_masks(buf, e, in, m);
+                    const unsigned mine = cls == 0 ? m[0] : cls == 1 ? m[1] : cls == 2 ? m[2] : m[3];
+                    const int b0k = cls == 0 ? at[0] : cls == 1 ? at[1] : cls == 2 ? at[2] : at[3];
+                    const int p = in ? b0k + __popc(mine & below) : r0 + e;
+                    if (e < n && p < P.wcap) out[p] = buf[e];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) at[k] += __popc(m[k]);
+                }
+            }
+        }
+        if (threadIdx.x == 0) {
+            if (all_s > P.wcap || all_l > P.wcap) atomicOr(&s.err[0], ERR_WLIST_OVERFLOW);
+            s.wn_s[ci] = min(all_s, P.wcap);
+            s.wn_l[ci] = min(all_l, P.wcap);
+        }
     }
 }
 
@@ -1251,6 +1530,8 @@ namespace gnb {
 }  // namespace gnb
 
 namespace gnb {
+template __global__ void k_water_search_block<false>(const SysDev*, const SearchParams);
+template __global__ void k_water_search_block<true>(const SysDev*, const SearchParams);
 template __global__ void k_water_search<4, false, false>(const SysDev*, const SearchParams);
 template __global__ void k_water_search<4, false, true>(const SysDev*, const SearchParams);
 template __global__ void k_water_search<4, true, false>(const SysDev*, const SearchParams);

@@ -7,7 +7,7 @@ import oracle_binding as ob
 from gromos_nb import generators
 from gromos_nb.nonbonded import Forcefield
 from gromos_nb.system import System
-from test_gpu_parity import compare_eval, sorted_pairs
+from test_gpu_parity import check_pairlist, compare_eval, sorted_pairs
 
 pytestmark = pytest.mark.gpu
 
@@ -37,3 +37,16 @@ def test_lists_of_clusters_in_several_images(waters, rcutp, rcutl, layout, width
         for got, want in zip(ff.pairlist_lists(), ref):
             assert np.array_equal(sorted_pairs(got), sorted_pairs(want))
         ff.close()
+
+
+# one block per cluster: fewer candidates than a round, several rounds and batches, lists beyond the 480
+# entries that are sorted (1.9 nm), the last sizes of the kernel and the first without it (1,472 clusters)
+@pytest.mark.parametrize("waters,rcutp,rcutl", [(1, 0.9, 0.9), (5, 0.8, 0.9), (130, 0.8, 0.9), (700, 1.2, 1.4),
+                                                (4000, 1.9, 1.9), (4000, 0.8, 1.9), (5776, 0.8, 1.0),
+                                                (5900, 0.8, 1.0)])
+def test_search_by_blocks(waters, rcutp, rcutl):
+    s = generators.spc_water_system(waters, max(generators.box_for_waters(waters), 2.0 * rcutl + 0.01), 8,
+                                    rcutp=rcutp, rcutl=rcutl)
+    check_pairlist(s)
+    if waters > 100:  # a handful of waters lie outside each other's cutoff: no forces to compare
+        compare_eval(s, steps=2, move=0.001)
