@@ -1113,12 +1113,11 @@ gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events, bool fin
     // graph each event node adds its own latency to the step, so a graph holds
     // just the first and last (the step's total device time)
     const bool stage = record_events && !in_capture;
-    // Programmatic launches where nothing is recorded between the kernels and no
-    // other member shares the chip by a graph: a boundary between two small
-    // kernels costs its drain and launch latency otherwise, and the solute kernels
-    // run beside the water kernel (MD step of 1,000 waters 57 -> 50 us, of 3,000 with
-    // 200 ions 100 -> 70).
-    pdl = prm.kernel == GR_KERNEL_FIXED && !record_events && !in_capture;
+    // Programmatic launches where nothing is recorded between the kernels and the
+    // members of a batch leave room: a boundary between two small kernels costs its
+    // drain and launch latency otherwise, and the solute kernels run beside the water
+    // kernel (MD step of 1,000 waters 57 -> 50 us, of 3,000 with 200 ions 100 -> 70).
+    pdl = prm.kernel == GR_KERNEL_FIXED && !record_events && !(in_capture && crowded);
     if (stage) last_staged = true;
     if (stage) {
         evk_valid = prm.kernel == GR_KERNEL_FIXED && NCG > NSCG;

@@ -4,7 +4,7 @@ import pytest
 
 import oracle_binding as ob
 from gromos_nb import generators
-from gromos_nb.nonbonded import Forcefield
+from gromos_nb.nonbonded import Batch, Forcefield
 
 pytestmark = pytest.mark.gpu
 
@@ -79,3 +79,26 @@ def test_tiled_step_of_a_large_system():
     assert abs(st["e_kin"] - so["e_kin"]) <= 1e-5 * so["e_kin"] and st["settle_failures"] == 0
     ff.close()
     ref.close()
+
+
+# members of a batch below and above 16 clusters per SM (2,368): the recorded steps start their kernels
+# while the predecessors end and search by blocks, or do neither
+@pytest.mark.parametrize("members,waters", [(2, 700), (3, 3300)])
+def test_batch_steps_equal_standalone_steps(members, waters):
+    s = generators.solvated_solute_system(waters, 30, seed=15, single_atom_cgs=True)
+    s.params.rcutp, s.params.rcutl = 0.8, 1.0
+    alone = start(s)
+    alone.md_run(7)
+    want = alone.md_state()
+    alone.close()
+    b = Batch()
+    ffs = [start(s) for _ in range(members)]
+    for ff in ffs:
+        b.add(ff)
+    b.md_run(7)
+    for ff in ffs:
+        got = ff.md_state()
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    b.close()
+    for ff in ffs:
+        ff.close()
