@@ -231,6 +231,13 @@ void NbSystem::release() {
     d_sys = nullptr;
     sent_valid = false;
     if (any) cudaStreamSynchronize(mem_stream);  // the blocks are back in the pool before the stream goes
+    // (every fork was joined into the stream just synchronised)
+    if (ev_fork) cudaEventDestroy(ev_fork);
+    if (ev_join) cudaEventDestroy(ev_join);
+    if (side) cudaStreamDestroy(side);
+    ev_fork = ev_join = nullptr;
+    side = nullptr;
+    forked = side_waits = main_waits = false;
     std::memset(&h, 0, sizeof(h));
     d_cg_key = nullptr;
     for (auto& e : ev)
@@ -879,9 +886,56 @@ cudaError_t NbSystem::launch(void (*kernel)(P...), dim3 grid, unsigned threads, 
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = pdl ? 1 : 0;
+    // (a kernel after an event of the other stream has two predecessors: a plain launch)
+    bool& waits = s == side ? side_waits : main_waits;
+    cfg.numAttrs = pdl && !waits ? 1 : 0;
+    waits = false;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
+
+// The side stream.  Solute kernels and the FP64 terms need nothing of the water
+// kernels (all of them add to fixed-point sums), so where the kernels are
+// launched back to back (pdl) they run beside these: fork() orders the side
+// stream after everything enqueued on s, join() orders s after the side stream.
+// A MD step of 3,000 waters with 200 ions takes 66 us this way, 81 one kernel
+// after the other; 16 frames of 3,000 waters 3.2 and 4.1 ms.  Not in the recorded
+// steps of a batch, whose members already run side by side: their graphs
+// would cost more to record and launch than the branches give (six served jobs
+// 19.4 ms with them, 18.1 without).
+cudaError_t NbSystem::ensure_side() {
+    if (side) return cudaSuccess;
+    cudaError_t e = cudaSuccess;
+    if (!ev_fork) e = cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming);
+    if (e == cudaSuccess && !ev_join) e = cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+    if (e != cudaSuccess) side = nullptr;
+    return e;
+}
+
+cudaError_t NbSystem::fork(cudaStream_t s) {
+    cudaError_t e = cudaEventRecord(ev_fork, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(side, ev_fork, 0);
+    forked = side_waits = e == cudaSuccess;
+    return e;
+}
+
+cudaError_t NbSystem::join(cudaStream_t s) {
+    if (!forked) return cudaSuccess;
+    forked = false;
+    cudaError_t e = cudaEventRecord(ev_join, side);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, ev_join, 0);
+    main_waits = e == cudaSuccess;
+    return e;
+}
+
+namespace {
+// Joins on every way out of a function that forks.
+struct JoinAtEnd {
+    NbSystem& S;
+    cudaStream_t s;
+    ~JoinAtEnd() { S.join(s); }
+};
+}  // namespace
 
 gr_status NbSystem::push_descriptor(cudaStream_t s) {
     // Only what changed travels: the copy is an operation of its own between two
@@ -960,6 +1014,8 @@ gr_status NbSystem::build_pairlist(cudaStream_t s, bool sync) {
         return GR_ERR_STATE;
     }
     regrow_count = 0;
+    const bool beside = pdl && !in_capture && NCG > NSCG && NSCG > 0 && side;  // the solute search beside the water search
+    JoinAtEnd join_at_end{*this, s};
     if (relist) {  // list storage sized afresh from the requested capacity
         wcap_alloc = 0;
         wcap_want = 0;
@@ -973,6 +1029,7 @@ gr_status NbSystem::build_pairlist(cudaStream_t s, bool sync) {
         snapshot = MdSnapshot{};  // taken once (a retry builds the same positions)
         GR_CUDA(launch(k_scatter, blocks_for(NCG, 256), 256, 0, s, d_sys, d_cg_key));
         GR_CUDA(launch(k_cell_sort, h.n_cells, 256, 0, s, d_sys));
+        if (beside) GR_CUDA(fork(s));
         GR_CUDA(launch(k_cluster_setup, h.n_cells, 128, 0, s, d_sys));
         if (NCG > NSCG) {
             GR_CUDA(launch(k_cell_candidates, dim3(h.n_cells, 2), 256, 0, s, d_sys));
@@ -1030,13 +1087,14 @@ gr_status NbSystem::build_pairlist(cudaStream_t s, bool sync) {
             }
 #undef GR_WATER_SEARCH
         }
-        if (NSCG > 0)
-            GR_CUDA(launch(k_solute_search, NSCG, kSoluteSearchWarps * 32, 0, s, d_sys, pdl && NCG > NSCG));
+        const cudaStream_t ss = beside ? side : s;
+        if (NSCG > 0) GR_CUDA(launch(k_solute_search, NSCG, kSoluteSearchWarps * 32, 0, ss, d_sys));
         if (n_pert > 0 && NSCG > 0) {
-            GR_CUDA(cudaMemsetAsync(h.n_pert_pairs, 0, sizeof(int), s));
-            GR_CUDA(launch(k_pert_pairs, blocks_for((long long)NSCG * h.scap, 256), 256, 0, s, d_sys));
+            GR_CUDA(cudaMemsetAsync(h.n_pert_pairs, 0, sizeof(int), ss));
+            GR_CUDA(launch(k_pert_pairs, blocks_for((long long)NSCG * h.scap, 256), 256, 0, ss, d_sys));
         }
         GR_CUDA(cudaGetLastError());
+        GR_CUDA(join(s));
         if (!sync) {
             // overflow flags are read back asynchronously and resolved by the next
             // call that synchronises (resolve_pending)
@@ -1122,9 +1180,10 @@ gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events, bool fin
     const bool stage = record_events && !in_capture;
     // Programmatic launches where nothing is recorded between the kernels and the
     // members of a batch leave room: a boundary between two small kernels costs its
-    // drain and launch latency otherwise, and the solute kernels run beside the water
-    // kernel (MD step of 1,000 waters 57 -> 50 us, of 3,000 with 200 ions 100 -> 70).
+    // drain and launch latency otherwise (MD step of 1,000 waters 57 -> 50 us), and the
+    // solute kernels run beside the water kernels.
     pdl = prm.kernel == GR_KERNEL_FIXED && !record_events && !(in_capture && crowded);
+    if (pdl && NCG > NSCG && NSA + h.n_ex_pairs + h.n_14_pairs > 0 && !in_capture) GR_CUDA(ensure_side());
     if (stage) last_staged = true;
     if (stage) {
         evk_valid = prm.kernel == GR_KERNEL_FIXED && NCG > NSCG;
@@ -1168,8 +1227,24 @@ gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events, bool fin
     bool do_long = h.twin && (rebuild || !lr_computed);
     const int sm = sm_count();
     const size_t shg = size_t(2 * G * G) * sizeof(unsigned long long);
+    const int nterm = NSA + h.n_ex_pairs + h.n_14_pairs;
+    // solute kernels and FP64 terms beside the water kernels
+    const bool beside = pdl && !in_capture && NCG > NSCG && nterm > 0 && side;
+    const cudaStream_t ss = beside ? side : s;
+    JoinAtEnd join_at_end{*this, s};
+    auto clear_long = [&]() -> gr_status {
+        GR_CUDA(cudaMemsetAsync(h.f_long, 0, size_t(N) * 3 * sizeof(long long), s));
+        GR_CUDA(cudaMemsetAsync(h.acc_long, 0, size_t(NA) * sizeof(long long), s));
+        if (NCG > NSCG)
+            GR_CUDA(cudaMemsetAsync(h.fs_long, 0, size_t(h.max_clusters) * W * 9 * sizeof(long long), s));
+        return GR_OK;
+    };
     if (prm.kernel == GR_KERNEL_FIXED) {
         WaterParams wp;
+        if (beside) {
+            if (do_long && (st = clear_long())) return st;
+            GR_CUDA(fork(s));
+        }
         if (NCG > NSCG) {
             wp = water_params();
             if (!prepped) GR_CUDA(launch(k_water_prep, blocks_for(NCG - NSCG, 128), 128, 0, s, d_sys));
@@ -1180,22 +1255,18 @@ gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events, bool fin
         // solute work items: (CG, chunk of list entries), 4 warps per block
         const unsigned sgrid = std::max(1u, std::min(blocks_for((long long)NSCG * ((h.scap - 1) / solute_chunk(h.twin != 0) + 1), 4),
                                                      unsigned(sm * 8)));
-        const bool beside = pdl && NCG > NSCG;
         auto* solute_s = max_cg == 1 ? k_solute_force<false, 1> : max_cg <= 4 ? k_solute_force<false, 4> : k_solute_force<false, 8>;
         auto* solute_l = max_cg == 1 ? k_solute_force<true, 1> : max_cg <= 4 ? k_solute_force<true, 4> : k_solute_force<true, 8>;
-        if (NSCG > 0) GR_CUDA(launch(solute_s, sgrid, 128, shg, s, d_sys, beside));
+        if (NSCG > 0) GR_CUDA(launch(solute_s, sgrid, 128, shg, ss, d_sys));
         if (stage) GR_CUDA(record_event(ev[2], s));
         if (do_long) {
-            GR_CUDA(cudaMemsetAsync(h.f_long, 0, size_t(N) * 3 * sizeof(long long), s));
-            GR_CUDA(cudaMemsetAsync(h.acc_long, 0, size_t(NA) * sizeof(long long), s));
-            if (NCG > NSCG)
-                GR_CUDA(cudaMemsetAsync(h.fs_long, 0, size_t(h.max_clusters) * W * 9 * sizeof(long long), s));
+            if (!beside && (st = clear_long())) return st;
             if (NCG > NSCG) {
                 if (stage) GR_CUDA(record_event(evk[2], s));
                 if ((st = launch_water(s, wp, true))) return st;
                 if (stage) GR_CUDA(record_event(evk[3], s));
             }
-            if (NSCG > 0) GR_CUDA(launch(solute_l, sgrid, 128, shg, s, d_sys, beside));
+            if (NSCG > 0) GR_CUDA(launch(solute_l, sgrid, 128, shg, ss, d_sys));
             lr_computed = true;
             if (stage && NCG > NSCG) evk_long = true;
         }
@@ -1218,20 +1289,17 @@ gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events, bool fin
     }
     if (stage) GR_CUDA(record_event(ev[3], s));
     const size_t sha = size_t(NA) * sizeof(unsigned long long);
-    // the FP64 terms also run beside the water kernel (the one right before them
-    // and the solute kernel) when nothing but kernels was enqueued since
-    const bool after_water = pdl && prm.kernel == GR_KERNEL_FIXED && NCG > NSCG;
     // one thread per term, in small blocks: the few terms of a solute spread over SMs
-    const int nterm = NSA + h.n_ex_pairs + h.n_14_pairs;
     if (nterm > 0) {
         const int bt = nterm <= 64 * sm ? 64 : 128;
-        GR_CUDA(launch(k_excluded_14, blocks_for(nterm, bt), bt, sha, s, d_sys, after_water));
+        GR_CUDA(launch(k_excluded_14, blocks_for(nterm, bt), bt, sha, ss, d_sys));
     }
     if (n_pert > 0) {
         const int term_blocks = int(blocks_for(std::max(NSA, h.n_pp), 128));
         const unsigned pair_blocks = std::min(blocks_for(std::max(pcap_alloc, 1), 128), unsigned(sm * 4));
-        GR_CUDA(launch(k_pert, term_blocks + pair_blocks, 128, sha, s, d_sys, term_blocks, after_water));
+        GR_CUDA(launch(k_pert, term_blocks + pair_blocks, 128, sha, ss, d_sys, term_blocks));
     }
+    GR_CUDA(join(s));
     if (finalize) {
         GR_CUDA(launch(k_finalize, blocks_for(std::max<long long>(3LL * N, NA), 256), 256, 0, s, d_sys,
                        prm.kernel == GR_KERNEL_PLAIN));

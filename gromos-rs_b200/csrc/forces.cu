@@ -229,8 +229,8 @@ struct SoluteWarp {
 };
 
 template <bool LONG, int MAXA>
-__global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__ sys, int beside) {
-    if (!beside) pdl_wait();
+__global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__ sys) {
+    pdl_wait();
     pdl_trigger();
     const SysDev& s = sys[blockIdx.y];
     const int lane = threadIdx.x & 31;
@@ -457,7 +457,6 @@ __global__ void __launch_bounds__(128) k_solute_force(const SysDev* __restrict__
 #pragma unroll
     for (int v = 0; v < 9; ++v) idx[v] = 2 * G * G + v;
     block_flush<9>(acc, dst, idx);
-    if (beside) pdl_wait();
 }
 
 // ---------------------------------------------------------------------------
@@ -571,8 +570,8 @@ __device__ __forceinline__ void shared_add(unsigned long long* sh, int idx, doub
 // multi-atom CGs and 11 us for 200 ions (ncu).  Here every value is taken to
 // fixed point by its thread and the warp's integers are summed by shuffles (the
 // same totals), one shared add per warp: 7.2 and 4.6 us.
-__global__ void k_excluded_14(const SysDev* __restrict__ sys, int beside) {
-    if (!beside) pdl_wait();
+__global__ void k_excluded_14(const SysDev* __restrict__ sys) {
+    pdl_wait();
     pdl_trigger();
     const SysDev& s = sys[blockIdx.y];
     const int G = s.n_egroups;
@@ -646,7 +645,6 @@ __global__ void k_excluded_14(const SysDev* __restrict__ sys, int beside) {
     __syncthreads();
     for (int v = threadIdx.x; v < NA; v += blockDim.x)
         if (sh[v]) atomicAdd(reinterpret_cast<unsigned long long*>(s.acc_short + v), sh[v]);
-    if (beside) pdl_wait();
 }
 
 // perturbed_lj_crf_interaction (perturbed.rs:124-266), FP64.
@@ -932,8 +930,8 @@ __device__ __forceinline__ void pert_terms(const SysDev& s, unsigned long long* 
 
 // All perturbation corrections in one launch: the first term_blocks blocks
 // take the per-atom terms, the others the listed pairs.
-__global__ void __launch_bounds__(128) k_pert(const SysDev* __restrict__ sys, int term_blocks, int beside) {
-    if (!beside) pdl_wait();
+__global__ void __launch_bounds__(128) k_pert(const SysDev* __restrict__ sys, int term_blocks) {
+    pdl_wait();
     pdl_trigger();
     const SysDev& s = sys[blockIdx.y];
     const int NA = acc_size(s.n_egroups);
@@ -947,7 +945,6 @@ __global__ void __launch_bounds__(128) k_pert(const SysDev* __restrict__ sys, in
     __syncthreads();
     for (int v = threadIdx.x; v < NA; v += blockDim.x)
         if (sh[v]) atomicAdd(reinterpret_cast<unsigned long long*>(s.acc_short + v), sh[v]);
-    if (beside) pdl_wait();
 }
 
 // Fixed point -> FP64 results.  plain != 0 adds the FP32 baseline buffers.
@@ -1035,12 +1032,12 @@ __global__ void k_finalize_plain_energies(const SysDev* __restrict__ sys) {
 }
 
 // Explicit instantiations used by the host runtime.
-template __global__ void k_solute_force<false, 8>(const SysDev*, int);
-template __global__ void k_solute_force<true, 8>(const SysDev*, int);
-template __global__ void k_solute_force<false, 4>(const SysDev*, int);
-template __global__ void k_solute_force<true, 4>(const SysDev*, int);
-template __global__ void k_solute_force<false, 1>(const SysDev*, int);
-template __global__ void k_solute_force<true, 1>(const SysDev*, int);
+template __global__ void k_solute_force<false, 8>(const SysDev*);
+template __global__ void k_solute_force<true, 8>(const SysDev*);
+template __global__ void k_solute_force<false, 4>(const SysDev*);
+template __global__ void k_solute_force<true, 4>(const SysDev*);
+template __global__ void k_solute_force<false, 1>(const SysDev*);
+template __global__ void k_solute_force<true, 1>(const SysDev*);
 
 }  // namespace gnb
 

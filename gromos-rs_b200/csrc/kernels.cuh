@@ -14,7 +14,7 @@ template <int W, bool POPSORT, bool FILTER>
 __global__ void k_water_search(const SysDev* __restrict__ sys, const SearchParams P);
 template <bool FILTER>
 __global__ void k_water_search_block(const SysDev* __restrict__ sys, const SearchParams P);
-__global__ void k_solute_search(const SysDev* __restrict__ sys, int beside);
+__global__ void k_solute_search(const SysDev* __restrict__ sys);
 __global__ void k_pert_pairs(const SysDev* __restrict__ sys);
 __global__ void k_expand_cgpairs(const SysDev* __restrict__ sys, int long_range);
 
@@ -28,11 +28,11 @@ __global__ void k_water_deferred(const SysDev* __restrict__ sys, const WaterPara
 template <int W, bool LJ00, bool LONG, bool PK>
 __global__ void k_water_force_it(const SysDev* __restrict__ sys, const WaterParams wp, const WaterScaled ws);
 template <bool LONG, int MAXA>
-__global__ void k_solute_force(const SysDev* __restrict__ sys, int beside);
+__global__ void k_solute_force(const SysDev* __restrict__ sys);
 __global__ void k_pos32(const SysDev* __restrict__ sys);
 __global__ void k_plain_force(const SysDev* __restrict__ sys, int long_range);
-__global__ void k_excluded_14(const SysDev* __restrict__ sys, int beside);
-__global__ void k_pert(const SysDev* __restrict__ sys, int term_blocks, int beside);
+__global__ void k_excluded_14(const SysDev* __restrict__ sys);
+__global__ void k_pert(const SysDev* __restrict__ sys, int term_blocks);
 __global__ void k_finalize(const SysDev* __restrict__ sys, int plain);
 __global__ void k_finalize_plain_energies(const SysDev* __restrict__ sys);
 __global__ void k_ffma_peak(float* out, int iters, float a, float b);

@@ -235,11 +235,10 @@ __device__ __forceinline__ void red_add(long long* addr, long long v) {
 // predecessors have completed and their writes are visible; pdl_trigger() lets
 // the successor start once every block has called it (or ended).  Without the
 // attribute both do nothing.  Every kernel launched so calls pdl_wait before it
-// touches memory and then pdl_trigger -- except the ones that only add to
-// fixed-point sums beside the water kernel (`beside` below), which wait at
-// their end: they start when every block of the kernel before them has passed
-// its own wait, so what they read is complete, and their end still means that
-// everything before them has ended.
+// touches memory and then pdl_trigger: a grid sees its predecessors' writes
+// only through its own wait, not through one of another grid.  Kernels that run
+// beside the water kernels are therefore on a stream of their own, forked and
+// joined by events (NbSystem::fork).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

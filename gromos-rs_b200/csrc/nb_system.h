@@ -40,6 +40,9 @@ class NbSystem {
     gr_status energy_buffer();
     gr_status pair_counts(cudaStream_t s, long long* n_short, long long* n_long);
     gr_status push_descriptor(cudaStream_t s);
+    cudaError_t ensure_side();
+    cudaError_t fork(cudaStream_t s);
+    cudaError_t join(cudaStream_t s);
     cudaError_t dev_malloc(void** p, size_t n);
     void dev_free(void* p);
     cudaStream_t mem_stream = nullptr;  // the context's stream: pool allocations and releases are ordered on it
@@ -139,6 +142,11 @@ class NbSystem {
     cudaEvent_t ev_step = nullptr;
     bool step_check = false;
     bool pdl = false;         // this evaluation's kernels start while their predecessors end (see eval)
+    // The side stream: kernels that run beside the water kernels (see fork).
+    cudaStream_t side = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    bool forked = false;      // side work that `join` has not yet ordered before the main stream
+    bool side_waits = false, main_waits = false;  // the stream's next kernel follows an event of the other stream
     bool in_capture = false;  // recording a CUDA graph: the device descriptor is already current
     bool crowded = false;     // ... a batch's, whose members fill the chip between them
     bool last_staged = false; // the last timed evaluation recorded its stage events (kernel by kernel)

@@ -1306,19 +1306,18 @@ __device__ __forceinline__ unsigned long long excl_mask_warp(const SysDev& s, in
 // Exclusion masks are only looked up for the CGs that share an excluded or
 // 1-4 pair with this one (cgx, from the topology), after the sweep, one
 // warp per mask.  The kernel needs nothing of the water search and runs beside
-// it (nb_common.cuh, pdl_wait).
+// it, on the side stream (NbSystem::fork).
 constexpr int kSoluteSearchWarps = 8;
 constexpr int kMaskQueue = 64;
 
-__global__ void __launch_bounds__(kSoluteSearchWarps * 32) k_solute_search(const SysDev* __restrict__ sys, int beside) {
-    if (!beside) pdl_wait();
+__global__ void __launch_bounds__(kSoluteSearchWarps * 32) k_solute_search(const SysDev* __restrict__ sys) {
+    pdl_wait();
     pdl_trigger();
     const SysDev& s = sys[blockIdx.y];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int ci = blockIdx.x;
     if (s.cg_off[ci + 1] - s.cg_off[ci] > kMaxCGAtoms) {
         if (threadIdx.x == 0) atomicOr(&s.err[0], ERR_CG_TOO_LARGE);
-        if (beside) pdl_wait();
         return;
     }
     __shared__ int seg_lo[27], seg_pre[28];
@@ -1447,7 +1446,6 @@ __global__ void __launch_bounds__(kSoluteSearchWarps * 32) k_solute_search(const
         atomicMax(&s.sn_max[0], cnt_s);
         atomicMax(&s.sn_max[1], cnt_l);
     }
-    if (beside) pdl_wait();
 }
 
 // Explicit list of atom pairs that the FEP correction visits: pairs of the

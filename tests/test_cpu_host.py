@@ -253,3 +253,22 @@ def test_reference_arm_json_line_and_nonzero_ranks():
     other = subprocess.run(cmd, capture_output=True, text=True, timeout=120, check=True,
                            env=dict(env, RANK="1", WORLD_SIZE="2", LOCAL_RANK="1"))
     assert other.stdout.strip() == ""
+
+
+def test_kernels_wait_before_they_touch_memory():
+    """A kernel that lets its successor start early (pdl_trigger) has waited for its own predecessors
+    first: their writes are visible to a grid only through its own griddepcontrol.wait."""
+    import re
+
+    seen = 0
+    for name in sorted(os.listdir(_lib.SRC_DIR)):
+        with open(os.path.join(_lib.SRC_DIR, name)) as fh:
+            text = fh.read()
+        for m in re.finditer(r"__global__\s+void[^;{]*?(\w+)\(const SysDev\*[^;{]*\)\s*\{", text):
+            body = text[m.end():text.index("\n}", m.end())]
+            if "pdl_trigger()" in body:
+                seen += 1
+                first = [line.strip() for line in body.strip().splitlines()[:2]]
+                assert first == ["pdl_wait();", "pdl_trigger();"], (name, m.group(1), first)
+                assert body.count("pdl_wait()") == 1, (name, m.group(1))
+    assert seen >= 16
