@@ -346,10 +346,13 @@ class Forcefield:
 
     def close(self) -> None:
         if getattr(self, "_h", None):
-            batch = getattr(self, "_batch", None)
-            batch = batch() if batch is not None else None
-            if batch is not None:  # a batch member leaves its batch first
-                batch.remove(self)
+            place = getattr(self, "_place", None)
+            if place is not None:  # a batch member leaves its batch first
+                batch = place.batch()
+                if batch is not None:
+                    batch.remove(self)
+                else:
+                    place.remove(self)
             check(self._L.gr_ctx_destroy(self._h))
             self._h = None
 
@@ -366,6 +369,22 @@ def _autotune_dict(r) -> Dict:
     return {"water_layout": r.water_layout, "cluster_size": r.cluster_size, "candidates": cands}
 
 
+class _BatchPlace:
+    """The library's batch as both a Batch and its members hold it, without a cycle between them.
+
+    A member that is finalized with its batch (both in one garbage cycle: weak references are
+    cleared before the finalizers run, in either order) still leaves the library's batch here.
+    """
+
+    def __init__(self, lib, handle, batch: "Batch"):
+        self._L, self.handle, self.batch = lib, handle, weakref.ref(batch)
+
+    def remove(self, ff: "Forcefield") -> None:
+        if self.handle:
+            check(self._L.gr_batch_remove(self.handle, ff.handle))
+        ff._place = None
+
+
 class Batch:
     """Members (Forcefield objects) stepped together: one CUDA graph launch per MD step.
 
@@ -380,17 +399,18 @@ class Batch:
         h = C.c_void_p()
         check(self._L.gr_batch_create(device, C.byref(h)))
         self._h = h
+        self._place = _BatchPlace(self._L, h, self)
         self.members: List["Forcefield"] = []
 
     def add(self, ff: "Forcefield") -> None:
         check(self._L.gr_batch_add(self._h, ff.handle))
         self.members.append(ff)
-        ff._batch = weakref.ref(self)  # no cycle: a dropped batch and its members go at once
+        ff._place = self._place
 
     def remove(self, ff: "Forcefield") -> None:
         check(self._L.gr_batch_remove(self._h, ff.handle))
         self.members.remove(ff)
-        ff._batch = None
+        ff._place = None
 
     def __len__(self) -> int:
         return len(self.members)
@@ -449,9 +469,9 @@ class Batch:
     def close(self) -> None:
         if getattr(self, "_h", None):
             self._L.gr_batch_destroy(self._h)
-            self._h = None
+            self._h = self._place.handle = None
             for ff in self.members:
-                ff._batch = None
+                ff._place = None
             self.members = []
 
     def __del__(self):
