@@ -546,7 +546,7 @@ gr_status NbSystem::md_step_launch(cudaStream_t s, bool fuse_prep) {
     // records come from this kernel
     md.prep_next = fuse_prep && md_settle && NCG > NSCG && h.wrec && !in_capture && built &&
                    steps_since_update < prm.nsnb;
-    prepped_next = prep_in_acc = md.prep_next != 0;
+    if (!in_capture) prepped_next = prep_in_acc = md.prep_next != 0;
     const int n_units = md_settle ? NSA + (N - NSA) / 3 : N;
     // a unit is one long FP64 chain: small blocks spread few units over more SMs
     const unsigned bt = n_units <= 128 * sm_count() ? 64 : 128;

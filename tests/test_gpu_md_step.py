@@ -45,7 +45,7 @@ def test_forces_and_energies_of_the_last_step(k, settle, steps):
 
 def test_records_written_ahead_do_not_reach_another_evaluation():
     """The step kernel writes the next step's water records; an evaluation of other positions, a graph
-    replay and a batch must not count their energies twice."""
+    replay and a batch's steps must not count their energies twice."""
     s = systems()[0]
     want = Forcefield(s).apply(s.pos)
     for graph in (False, True):
@@ -56,6 +56,40 @@ def test_records_written_ahead_do_not_reach_another_evaluation():
         got = ff.apply(s.pos, force_rebuild=True, graph=graph)
         assert got["e_crf"] == want["e_crf"] and np.array_equal(got["forces"], want["forces"])
         ff.close()
+    for capacity in (0, 40):  # 40: the batch's rebuild overflows, and the member runs the step on its own
+        ff, b = start(s), Batch()
+        ff.md_run(2)
+        x = ff.md_state()[0]
+        b.add(ff)
+        if capacity:
+            ff.set_params(list_capacity=capacity)
+        b.md_run(1)
+        got, want = ff.result(), Forcefield(s).apply(x)
+        assert got["e_crf"] == want["e_crf"] and np.array_equal(got["forces"], want["forces"])
+        assert (ff.md_stats()["rollbacks"] > 0) == (capacity > 0)
+        b.close()
+        ff.close()
+
+
+def test_records_written_ahead_are_those_of_the_members_last_own_step():
+    """A member's own steps between those of its batch: the records that they wrote ahead are of positions
+    that the batch's steps leave behind."""
+    s = systems()[0]
+    state = []
+    for fresh in (False, True):
+        ff, b = start(s), Batch()
+        b.add(ff)
+        b.md_run(5)
+        ff.md_run(2)
+        b.md_run(3)  # the same recorded steps
+        if fresh:
+            ff.positions_device_ptr()  # the caller may write the positions: no record is kept
+        ff.md_run(1)
+        state.append((ff.result()["forces"], *ff.md_state()))
+        b.close()
+        ff.close()
+    for got, want in zip(*state):
+        assert np.array_equal(got, want)
 
 
 def test_tiled_step_of_a_large_system():
