@@ -718,7 +718,7 @@ gr_status NbSystem::set_params(const gr_nb_params* p) {
 }
 
 gr_status NbSystem::set_box(const double box[3]) {
-    prepped_next = false;
+    state_changed();
     if (prm.boundary == 1 && (!(box[0] > 0) || !(box[1] > 0) || !(box[2] > 0))) {
         set_error("gr_set_box: rectangular box edges must be positive");
         return GR_ERR_INVALID;
@@ -1312,6 +1312,14 @@ gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events, bool fin
     return GR_OK;
 }
 
+// Positions, velocities, bath or box were changed outside md_run: records
+// written ahead are not of these positions, and a rollback must not go back to
+// a period start before the change.
+void NbSystem::state_changed() {
+    prepped_next = false;
+    md_psnap_valid = false;
+}
+
 void NbSystem::drop_graphs() {
     for (auto& g : g_step) {
         if (g) cudaGraphExecDestroy(g);
@@ -1787,7 +1795,7 @@ gr_status gr_positions_upload(gr_ctx* ctx, const double* xyz) {
         set_error("gr_positions_upload: no system or null positions");
         return GR_ERR_STATE;
     }
-    ctx->sys.prepped_next = false;
+    ctx->sys.state_changed();
     cudaError_t e = cudaMemcpyAsync(ctx->sys.h.pos, xyz, size_t(ctx->sys.N) * 3 * sizeof(double),
                                     cudaMemcpyHostToDevice, ctx->stream);
     if (e != cudaSuccess) {
@@ -1805,7 +1813,7 @@ gr_status gr_positions_device(gr_ctx* ctx, double** dev_xyz) {
         return GR_ERR_STATE;
     }
     *dev_xyz = ctx->sys.h.pos;
-    ctx->sys.prepped_next = false;  // the caller may write the coordinates
+    ctx->sys.state_changed();  // the caller may write the coordinates
     ctx->sys.pos_set = true;
     return GR_OK;
 }

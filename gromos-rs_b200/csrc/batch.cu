@@ -423,7 +423,7 @@ gr_status gr_batch_md_run(gr_batch* b, int32_t n_steps) {
     if ((st = batch_prepare(b, true))) return st;
     for (auto& mb : b->m) {  // the graphs write their own water records
         NbSystem& S = mb.ctx->sys;
-        S.prepped_next = false;
+        S.state_changed();
         if (!S.prep_in_acc) continue;
         if ((st = S.drop_prep(mb.ctx->stream))) return st;
         GR_CUDA(cudaStreamSynchronize(mb.ctx->stream));

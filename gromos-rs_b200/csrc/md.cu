@@ -731,6 +731,7 @@ gr_status gr_md_set_temperature(gr_ctx* ctx, double t0, int32_t rescale_velociti
         set_error("gr_md_set_temperature: t0 must be positive");
         return GR_ERR_INVALID;
     }
+    S.md_psnap_valid = false;  // a replay of earlier steps would see the new bath and unscaled velocities
     // the bath temperature lives in device memory (k_md_step reads it every
     // step): recorded step graphs stay valid, and the write is ordered after
     // the steps already enqueued on this context's stream

@@ -36,6 +36,7 @@ class NbSystem {
     gr_status drop_prep(cudaStream_t s);
     gr_status eval_graph(cudaStream_t s, int flags);
     void drop_graphs();
+    void state_changed();
     gr_status download(cudaStream_t s, gr_result* out);
     gr_status energy_buffer();
     gr_status pair_counts(cudaStream_t s, long long* n_short, long long* n_long);

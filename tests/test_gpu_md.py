@@ -15,7 +15,7 @@ import pytest
 
 import oracle_binding as ob
 from gromos_nb import generators as g
-from gromos_nb.nonbonded import Forcefield
+from gromos_nb.nonbonded import Batch, Forcefield
 
 pytestmark = pytest.mark.gpu
 
@@ -147,6 +147,43 @@ def test_md_rollback_mid_period_keeps_the_schedule():
     (xb, vb), sb = out[1]
     assert sa["rollbacks"] == 0 and sb["rollbacks"] >= 1
     assert np.array_equal(xa, xb) and np.array_equal(va, vb)
+
+
+# positions given by the caller, velocities scaled to another temperature, steps taken in a batch
+@pytest.mark.parametrize("act", ["upload", "temperature", "batch"])
+def test_md_rollback_keeps_what_happened_since_the_period_began(act):
+    """A rollback goes back no further than the last change of the state from outside md_run.  The
+    rollback rebuilds the lists where it starts again, up to three steps off the other run's schedule:
+    molecules that cross a cutoff in between move velocities by some 1e-3 and positions by 1e-5 nm, where
+    a lost change moves them by 0.1 and 0.007 nm at least."""
+    s = g.spc_water_system(1200, box=g.box_for_waters(1200), seed=33, rcutp=0.8, rcutl=1.2, nsnb=4)
+    m = g.masses(s)
+    v = g.maxwell_velocities(m, 300.0, 8)
+    out = []
+    for tiny in (False, True):
+        ff = Forcefield(s)
+        ff.upload_positions(s.pos)
+        ff.md_init(m, v, dt=0.002, settle=True, dist_oh=0.1, dist_hh=g.SPC_DHH)
+        ff.md_run(2)
+        if act == "upload":
+            ff.upload_positions(ff.md_state()[0] + 0.2)
+        elif act == "temperature":
+            ff.md_set_temperature(450.0)
+        else:
+            b = Batch()
+            b.add(ff)
+            b.md_run(6)  # two steps into a period, as the member's own run before
+            b.remove(ff)
+            b.close()
+        if tiny:
+            ff.set_params(list_capacity=16)
+        st = ff.md_run(5)
+        out.append((ff.md_state(), st))
+        ff.close()
+    (xa, va), sa = out[0]
+    (xb, vb), sb = out[1]
+    assert sa["rollbacks"] == 0 and sb["rollbacks"] >= 1
+    assert np.abs(xa - xb).max() <= 1e-3 and np.linalg.norm(va - vb) <= 0.02 * np.linalg.norm(va)
 
 
 def test_md_trajectory_files(tmp_path):
