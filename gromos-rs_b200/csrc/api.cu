@@ -17,6 +17,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <unordered_map>
 #include <utility>
 #include <vector>
 
@@ -1998,24 +1999,68 @@ gr_status gr_forces_eval(gr_ctx* ctx, int32_t flags, gr_result* out) {
 // Page-locked host memory for result buffers: a download into it is one DMA
 // transfer, where one into pageable memory is staged by the driver and faults
 // in every fresh page on the way.
+//
+// The first CUDA call of a thread makes a context on the thread's current
+// device (GPU 0 unless set), so an allocation for a context is made on that
+// context's device, and each block is released on the device it was made on.
+namespace {
+struct HostBlocks {
+    std::mutex mu;
+    std::unordered_map<void*, int> device;
+};
+HostBlocks& host_blocks() {
+    static HostBlocks* b = new HostBlocks;  // never destroyed: arrays may be released at exit
+    return *b;
+}
+}  // namespace
+
 gr_status gr_host_alloc(size_t bytes, void** out) {
     if (!out || bytes == 0) {
         set_error("gr_host_alloc: null out or no bytes");
         return GR_ERR_INVALID;
     }
     *out = nullptr;
-    const cudaError_t e = cudaHostAlloc(out, bytes, cudaHostAllocPortable);
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaHostAlloc(out, bytes, cudaHostAllocPortable);
     if (e != cudaSuccess) {
         cudaGetLastError();
         *out = nullptr;
         set_error(std::string("gr_host_alloc: ") + cudaGetErrorString(e));
         return e == cudaErrorMemoryAllocation ? GR_ERR_OOM : GR_ERR_CUDA;
     }
+    try {
+        HostBlocks& B = host_blocks();
+        std::lock_guard<std::mutex> lock(B.mu);
+        B.device[*out] = dev;
+    } catch (...) {  // no exception leaves a C entry
+        cudaFreeHost(*out);
+        *out = nullptr;
+        set_error("gr_host_alloc: out of host memory");
+        return GR_ERR_OOM;
+    }
     return GR_OK;
 }
 
+gr_status gr_ctx_host_alloc(gr_ctx* ctx, size_t bytes, void** out) {
+    CTX_GUARD(ctx);
+    return gr_host_alloc(bytes, out);
+}
+
 gr_status gr_host_free(void* p) {
-    if (p) GR_CUDA(cudaFreeHost(p));
+    if (!p) return GR_OK;
+    int dev = -1;
+    {
+        HostBlocks& B = host_blocks();
+        std::lock_guard<std::mutex> lock(B.mu);
+        auto it = B.device.find(p);
+        if (it != B.device.end()) {
+            dev = it->second;
+            B.device.erase(it);
+        }
+    }
+    if (dev >= 0) GR_CUDA(cudaSetDevice(dev));
+    GR_CUDA(cudaFreeHost(p));
     return GR_OK;
 }
 

@@ -132,6 +132,7 @@ _SIGNATURES = {
     "gr_forces_device": (C.c_int32, [C.c_void_p, C.POINTER(C.c_void_p)]),
     "gr_result_download": (C.c_int32, [C.c_void_p, C.POINTER(GrResult)]),
     "gr_host_alloc": (C.c_int32, [C.c_size_t, C.POINTER(C.c_void_p)]),
+    "gr_ctx_host_alloc": (C.c_int32, [C.c_void_p, C.c_size_t, C.POINTER(C.c_void_p)]),
     "gr_host_free": (C.c_int32, [C.c_void_p]),
     "gr_last_timings": (C.c_int32, [C.c_void_p, C.POINTER(C.c_float)]),
     "gr_last_kernel_timings": (C.c_int32, [C.c_void_p, C.POINTER(C.c_float)]),

@@ -62,8 +62,9 @@ def _pop(size: int):
     return place
 
 
-def _take(size: int):
-    """A block of `size` bytes, or None when the limit is reached."""
+def _take(size: int, ctx):
+    """A block of `size` bytes, or None when the limit is reached.  A new arena is allocated on the
+    device of the context handle `ctx`."""
     global _held
     n = max(1, min(ARENA // size, 64))
     with _lock:
@@ -78,7 +79,7 @@ def _take(size: int):
             return None
         _held += n * size
     p = C.c_void_p()
-    if _lib.lib().gr_host_alloc(n * size, C.byref(p)) != _lib.GR_OK:
+    if _lib.lib().gr_ctx_host_alloc(ctx, n * size, C.byref(p)) != _lib.GR_OK:
         with _lock:
             _held -= n * size
         return None
@@ -89,12 +90,12 @@ def _take(size: int):
         return _pop(size)
 
 
-def empty(shape) -> np.ndarray:
-    """An uninitialised C-contiguous float64 array for a download to fill."""
+def empty(shape, ctx) -> np.ndarray:
+    """An uninitialised C-contiguous float64 array for a download from the context `ctx` to fill."""
     n = 8 * int(np.prod(shape))
     if n >= SMALLEST:
         size = -(-n // 4096) * 4096
-        place = _take(size)
+        place = _take(size, ctx)
         if place is not None:
             return np.asarray(_Block(place, size, shape))
     return np.empty(shape)

@@ -178,7 +178,7 @@ class Forcefield:
                 raise ValueError("out must be a C-contiguous float64 (n_atoms, 3) array")
             f = out
         else:
-            f = hostmem.empty((self.n_atoms, 3)) if download_forces else None
+            f = hostmem.empty((self.n_atoms, 3), self._h) if download_forces else None
         glj = np.zeros((self.G, self.G))
         gcrf = np.zeros((self.G, self.G))
         r = _lib.GrResult()
@@ -282,7 +282,7 @@ class Forcefield:
 
     def result(self) -> Dict:
         """Results of the last evaluation (e.g. after a batch evaluation), without evaluating."""
-        f = hostmem.empty((self.n_atoms, 3))
+        f = hostmem.empty((self.n_atoms, 3), self._h)
         glj = np.zeros((self.G, self.G))
         gcrf = np.zeros((self.G, self.G))
         r = _lib.GrResult()
@@ -319,8 +319,8 @@ class Forcefield:
         return self._h
 
     def md_state(self):
-        x = hostmem.empty((self.n_atoms, 3))
-        v = hostmem.empty((self.n_atoms, 3))
+        x = hostmem.empty((self.n_atoms, 3), self._h)
+        v = hostmem.empty((self.n_atoms, 3), self._h)
         check(self._L.gr_md_download(self._h, _p(x, C.c_double), _p(v, C.c_double)))
         return x, v
 

@@ -202,7 +202,8 @@ gr_status gr_last_kernel_timings(gr_ctx* ctx, float ms[3]);
 /* Page-locked host memory.  Results downloaded into it (gr_result.forces,
  * gr_md_download) arrive by one DMA transfer, about three times as fast as into
  * pageable memory that is already mapped and far more into fresh pages. */
-gr_status gr_host_alloc(size_t bytes, void** out);
+gr_status gr_host_alloc(size_t bytes, void** out);  /* on the calling thread's current device */
+gr_status gr_ctx_host_alloc(gr_ctx* ctx, size_t bytes, void** out);  /* on the context's device */
 gr_status gr_host_free(void* p);
 
 /* ---- measurement utilities (no counterpart in gromos-rs) ---------------- */

@@ -8,11 +8,15 @@ import pytest
 from gromos_nb import hostmem
 
 
+CTX = object()  # a context's handle
+
+
 class FakeLib:
     def __init__(self):
         self.live = {}
 
-    def gr_host_alloc(self, n, out):
+    def gr_ctx_host_alloc(self, ctx, n, out):
+        assert ctx is CTX         # never without the context whose device is meant
         buf = C.create_string_buffer(int(n))
         p = C.addressof(buf)
         self.live[p] = (buf, int(n))
@@ -41,27 +45,27 @@ def lib(monkeypatch):
 
 
 def test_memory_is_reused_after_every_view_is_gone(lib):
-    a = hostmem.empty((5000, 3))
+    a = hostmem.empty((5000, 3), CTX)
     a[:] = 7.0
     at, view = a.ctypes.data, a[10:]
     del a
-    b = hostmem.empty((5000, 3))
+    b = hostmem.empty((5000, 3), CTX)
     assert b.ctypes.data != at and (view == 7.0).all()   # the view still owns the block
     del view
-    c = hostmem.empty((5000, 3))
+    c = hostmem.empty((5000, 3), CTX)
     assert c.ctypes.data == at and c.flags.c_contiguous and c.flags.writeable and c.dtype == np.float64
     assert len(lib.live) == 1                             # one arena for the three
 
 
 def test_limit_and_release(lib, monkeypatch):
     monkeypatch.setattr(hostmem, "LIMIT", 20 << 20)
-    keep = [hostmem.empty((1 << 20,)) for _ in range(4)]  # 8 MB each: the first two fit
+    keep = [hostmem.empty((1 << 20,), CTX) for _ in range(4)]  # 8 MB each: the first two fit
     assert lib.bytes() <= 20 << 20 and hostmem._held == lib.bytes()
     for k, x in enumerate(keep):
         x[:] = k                                          # the others are ordinary arrays
     assert [x[0] for x in keep] == [0, 1, 2, 3]
     del keep, x
-    y = hostmem.empty((1000, 3))                          # another size: idle arenas make room
+    y = hostmem.empty((1000, 3), CTX)                          # another size: idle arenas make room
     assert lib.bytes() <= 20 << 20
     hostmem.release()
     assert len(lib.live) == 1                             # the arena of y stays
@@ -71,7 +75,7 @@ def test_limit_and_release(lib, monkeypatch):
 
 
 def test_small_arrays_are_ordinary(lib):
-    hostmem.empty((10, 3))[:] = 1.0
+    hostmem.empty((10, 3), CTX)[:] = 1.0
     assert not lib.live
 
 
@@ -80,7 +84,7 @@ def test_threads_never_share_a_block(lib):
 
     def work(tag):
         for _ in range(300):
-            a, b = hostmem.empty((2000, 3)), hostmem.empty((2000, 3))
+            a, b = hostmem.empty((2000, 3), CTX), hostmem.empty((2000, 3), CTX)
             a[:], b[:] = tag, -tag
             if (a != tag).any() or (b != -tag).any():
                 bad.append(tag)
@@ -89,3 +93,15 @@ def test_threads_never_share_a_block(lib):
     [t.start() for t in ts]
     [t.join() for t in ts]
     assert not bad
+
+
+def test_a_forcefields_arrays_are_allocated_on_its_device(lib):
+    from gromos_nb.nonbonded import Forcefield
+
+    for name in ("gr_md_download", "gr_result_download", "gr_forces_eval"):
+        setattr(lib, name, lambda *a: 0)
+    ff = Forcefield.__new__(Forcefield)
+    ff._L, ff._h, ff.n_atoms, ff.G = lib, CTX, 3000, 1
+    kept = [ff.md_state(), ff.result()["forces"], ff.apply()["forces"]]
+    assert len(lib.live) == 1 and kept
+    ff._h = None
