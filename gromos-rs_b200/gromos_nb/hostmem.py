@@ -7,12 +7,17 @@ took 1.4 ms, of which the transfer is 0.1.  :func:`empty` returns arrays whose
 memory is page-locked and goes back to a pool when the array (and every view
 of it) is gone.  Live and pooled blocks together stay within
 :data:`LIMIT` bytes; beyond that, and for small arrays, it returns ordinary
-arrays.  Safe with several threads: a block has one owner at a time.
+arrays.  Memory that no array uses is given back when it has been idle for
+:data:`IDLE_S` seconds (looked at on the next call here and when a context is
+closed), all of it when the process has no open context left, and whenever
+:func:`release` is called.  Safe with several threads: a block has one owner at
+a time.
 """
 from __future__ import annotations
 
 import ctypes as C
 import threading
+import time
 from collections import deque
 from typing import Dict, List
 
@@ -23,12 +28,15 @@ from . import _lib
 LIMIT = 512 << 20          # bytes of page-locked memory held at most, in use or pooled
 SMALLEST = 8 << 10        # smaller arrays gain nothing
 
+IDLE_S = 10.0              # seconds that memory without an array is kept for the next one
 ARENA = 8 << 20            # blocks of one size are cut from arenas of about this many bytes
 
 _lock = threading.Lock()
 _free: Dict[int, List[tuple]] = {}  # block size -> (address, arena)
 _held = 0                           # bytes of all arenas
-_returned: deque = deque()          # (block size, (address, arena)) of arrays that are gone
+_open: set = set()                  # handles of the contexts that may want arrays
+_looked = 0.0                       # when idle arenas were last looked for
+_returned: deque = deque()          # (block size, (address, arena), when) of arrays that are gone
 
 
 class _Arena:
@@ -36,6 +44,7 @@ class _Arena:
 
     def __init__(self, address: int, size: int, blocks: int):
         self.address, self.size, self.blocks, self.idle = address, size, blocks, 0
+        self.since = 0.0   # when its last array went
 
 
 class _Block:
@@ -46,14 +55,17 @@ class _Block:
         self.__array_interface__ = {"data": (place[0], False), "shape": tuple(shape), "typestr": "<f8", "version": 3}
 
     def __del__(self):
-        _returned.append((self._size, self._place))  # no lock: this may run inside any allocation
+        _returned.append((self._size, self._place, time.monotonic()))  # no lock: this may run inside any allocation
+        if not _open:
+            _give_back(0.0)
 
 
 def _drain() -> None:
     while _returned:
-        size, place = _returned.popleft()
+        size, place, when = _returned.popleft()
         _free.setdefault(size, []).append(place)
         place[1].idle += 1
+        place[1].since = when
 
 
 def _pop(size: int):
@@ -67,6 +79,8 @@ def _take(size: int, ctx):
     device of the context handle `ctx`."""
     global _held
     n = max(1, min(ARENA // size, 64))
+    if time.monotonic() - _looked > 0.1 * IDLE_S:
+        _give_back(IDLE_S)
     with _lock:
         _drain()
         if _free.get(size):
@@ -101,14 +115,47 @@ def empty(shape, ctx) -> np.ndarray:
     return np.empty(shape)
 
 
-def release() -> None:
-    """Give back the arenas that no array uses."""
-    global _held
-    with _lock:
-        _drain()
-        idle = {p[1] for places in _free.values() for p in places if p[1].idle == p[1].blocks}
+def _idle(age: float) -> list:
+    """Takes the arenas that no array has used for `age` seconds out of the pool (the caller holds the lock)."""
+    global _held, _looked
+    _drain()
+    _looked = now = time.monotonic()
+    idle = {p[1] for places in _free.values() for p in places
+            if p[1].idle == p[1].blocks and now - p[1].since >= age}
+    if idle:
         for size in list(_free):
             _free[size] = [p for p in _free[size] if p[1] not in idle]
         _held -= sum(a.size for a in idle)
+    return list(idle)
+
+
+def _give_back(age: float) -> None:
+    """Frees the arenas idle for `age` seconds, unless the pool is in use at this moment (this runs in
+    finalizers too, which may come in the middle of any of these functions)."""
+    if not _lock.acquire(blocking=False):
+        return
+    try:
+        idle = _idle(age)
+    finally:
+        _lock.release()
     for a in idle:
         _lib.lib().gr_host_free(a.address)
+
+
+def release() -> None:
+    """Give back the arenas that no array uses."""
+    with _lock:
+        idle = _idle(0.0)
+    for a in idle:
+        _lib.lib().gr_host_free(a.address)
+
+
+def opened(ctx) -> None:
+    """The context `ctx` was opened."""
+    _open.add(ctx)
+
+
+def closed(ctx) -> None:
+    """The context `ctx` was closed; with the last one go all idle arenas."""
+    _open.discard(ctx)
+    _give_back(IDLE_S if _open else 0.0)

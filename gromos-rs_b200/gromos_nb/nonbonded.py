@@ -132,6 +132,7 @@ class Forcefield:
         h = C.c_void_p()
         check(L.gr_ctx_create(device, C.byref(h)))
         self._h = h
+        hostmem.opened(h.value)
         self._topo = _TopologyStruct(system.topo)
         check(L.gr_system_upload(h, C.byref(self._topo.struct)))
         self._params = make_params(system.params, kernel, cluster_size, water_layout, list_capacity)
@@ -353,8 +354,10 @@ class Forcefield:
                     batch.remove(self)
                 else:
                     place.remove(self)
+            handle = self._h.value
             check(self._L.gr_ctx_destroy(self._h))
             self._h = None
+            hostmem.closed(handle)
 
     def __del__(self):
         try:

@@ -105,3 +105,27 @@ def test_a_forcefields_arrays_are_allocated_on_its_device(lib):
     kept = [ff.md_state(), ff.result()["forces"], ff.apply()["forces"]]
     assert len(lib.live) == 1 and kept
     ff._h = None
+
+
+def test_idle_memory_is_given_back(lib, monkeypatch):
+    now = [0.0]
+    monkeypatch.setattr(hostmem.time, "monotonic", lambda: now[0])
+    monkeypatch.setattr(hostmem, "_looked", 0.0)
+    hostmem.opened(1)
+    hostmem.opened(2)
+    a, b = hostmem.empty((5000, 3), CTX), hostmem.empty((1 << 20,), CTX)
+    del a
+    now[0] = hostmem.IDLE_S - 1.0
+    c = hostmem.empty((1000, 3), CTX)
+    assert len(lib.live) == 3                  # kept for the next array of its size
+    now[0] += 2.0
+    hostmem.empty((1000, 3), CTX)
+    assert len(lib.live) == 2                  # idle for too long: only b's and c's arenas
+    del b
+    hostmem.closed(1)
+    assert len(lib.live) == 2
+    hostmem.closed(2)                          # the last context: what no array uses
+    assert len(lib.live) == 1 and hostmem._held == lib.bytes()
+    c[:] = 1.0
+    del c                                      # and the rest with its array
+    assert not lib.live and hostmem._held == 0

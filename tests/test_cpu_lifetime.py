@@ -1,4 +1,5 @@
 """CPU: batches and their members let go of the library's objects in any order, over a fake library."""
+import ctypes as C
 import gc
 
 import pytest
@@ -20,11 +21,11 @@ class FakeLib:
         return _lib.GR_OK
 
     def gr_batch_add(self, b, c):
-        self.batch[b.value].add(c)
+        self.batch[b.value].add(c.value)
         return _lib.GR_OK
 
     def gr_batch_remove(self, b, c):
-        self.batch[b.value].remove(c)
+        self.batch[b.value].remove(c.value)
         return _lib.GR_OK
 
     def gr_batch_destroy(self, b):
@@ -32,9 +33,9 @@ class FakeLib:
         return _lib.GR_OK
 
     def gr_ctx_destroy(self, c):
-        if any(c in m for m in self.batch.values()):
+        if any(c.value in m for m in self.batch.values()):
             return _lib.GR_ERR_STATE
-        self.ctx.remove(c)
+        self.ctx.remove(c.value)
         return _lib.GR_OK
 
     def gr_last_error(self):
@@ -42,8 +43,8 @@ class FakeLib:
 
     def member(self):
         ff = Forcefield.__new__(Forcefield)
-        ff._L, ff._h = self, -1 - len(self.ctx)
-        self.ctx.add(ff._h)
+        ff._L, ff._h = self, C.c_void_p(1 + len(self.ctx))
+        self.ctx.add(ff._h.value)
         return ff
 
 
