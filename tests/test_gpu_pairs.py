@@ -83,3 +83,46 @@ def test_pair_loop(n_pairs, order, offset, periodic):
     assert abs(el - lj_ref) <= 2e-5 * max(abs(lj_ref), abs(crf_ref))
     assert abs(ec - crf_ref) <= 2e-5 * max(abs(lj_ref), abs(crf_ref))
     assert np.abs(v.cpu().numpy().reshape(3, 3) - v_ref).max() <= 2e-5 * np.abs(v_ref).max()
+
+
+def loop_on_host(x, pairs, c12, box=None, q=None):
+    from gromos_nb.nonbonded import lj_crf_innerloop
+
+    n = len(x)
+    return lj_crf_innerloop(x, np.zeros(n) if q is None else q, np.zeros(n, dtype=np.uint32), pairs,
+                            np.array([[[0.0, c12]]]), CRFParameters.new(1.4, 1.0, 61.0, 0.0), box)
+
+
+def test_rounding_of_one_pair():
+    """Every operation of a pair rounds once, as FP32 division and square root do: the error of r^-14 x
+    of separate pairs, whose r^2 is exact, is that of the same operations in numpy."""
+    rng = np.random.default_rng(9)
+    n = 4000
+    d = rng.integers(32, 128, (n, 3)) / 256.0          # 16 bits hold each square, 18 their sum
+    x = np.zeros((2 * n, 3), dtype=np.float32)
+    x[::2] = d
+    pairs = np.arange(2 * n, dtype=np.uint32).reshape(-1, 2)
+    f, e_lj, _, _ = loop_on_host(x, pairs, 1e-6)
+    r2 = (d * d).sum(1)
+    want = 12e-6 * r2 ** -7.0 * d[:, 0]
+    s = r2.astype(np.float32)
+    i2 = np.float32(1) / s
+    i6 = i2 * i2 * i2
+    same = np.float32(12) * np.float32(1e-6) * i6 * i6 * i2 * d[:, 0].astype(np.float32)
+
+    def rms(v):
+        return np.sqrt((((v - want) / want) ** 2).mean())
+
+    # 1.3: contracted operations round at other places; a reciprocal square root squared gives 2.3
+    assert rms(f[::2, 0]) <= 1.3 * rms(same) and rms(f[1::2, 0] * -1.0) <= 1.3 * rms(same)
+
+
+# edges for which 1.5 edges times the rounded reciprocal is below 1.5
+@pytest.mark.parametrize("edge", [3.38, 3.62, 3.83])
+def test_pairs_half_an_edge_apart(edge):
+    """The image is round(x / edge), ties to even: -1.5 edges become 0.5."""
+    edge = np.float32(edge)
+    x = np.array([[0.0, 0.1, 0.0], [np.float32(1.5) * edge, 0.4, 0.2]], dtype=np.float32)
+    assert float(x[1, 0]) == 1.5 * float(edge)
+    f, _, _, _ = loop_on_host(x, np.array([[0, 1]], dtype=np.uint32), 1e-6, np.array([float(edge)] * 3))
+    assert f[0, 0] > 0.0 > f[1, 0]
