@@ -567,9 +567,9 @@ __device__ __forceinline__ void shared_add(unsigned long long* sh, int idx, doub
 // from the topology).  The terms are few and their cost is latency: a thread
 // per atom that walked its exclusion list and added eleven values to shared
 // 64-bit words that its whole block adds to took 28 us for 200 atoms in
-// multi-atom CGs and 11 us for 200 ions (ncu).  Here every value is taken to
-// fixed point by its thread and the warp's integers are summed by shuffles (the
-// same totals), one shared add per warp: 7.2 and 4.6 us.
+// multi-atom CGs and 11 us for 200 ions (ncu).  Here a warp sums its values by
+// shuffles, in FP64 and per group slot, and takes each sum to fixed point once:
+// one shared add and one rounding per warp, 7.2 and 4.6 us.
 __global__ void k_excluded_14(const SysDev* __restrict__ sys) {
     pdl_wait();
     pdl_trigger();
@@ -583,13 +583,13 @@ __global__ void k_excluded_14(const SysDev* __restrict__ sys) {
     const int nsa = s.n_solute_atoms, nex = s.n_ex_pairs, nterm = nsa + nex + s.n_14_pairs;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     int sl = -1;
-    long long el = 0, ec = 0;
+    double el = 0.0, ec = 0.0;
     double v6[6] = {0, 0, 0, 0, 0, 0};  // xx, xy, xz, yy, yz, zz
     if (t < nsa) {
         const double qi = s.charge[t];
         const int gi = s.egroup[t];
         sl = group_slot(G, gi, gi);
-        ec = to_fixed_d(-0.5 * qi * qi * s.fpe * s.crf_cut, kEnergyScale);
+        ec = -0.5 * qi * qi * s.fpe * s.crf_cut;
     } else if (t < nterm) {
         const int2 ij = s.term_pairs[t - nsa];
         const int i = ij.x, j = ij.y;
@@ -604,18 +604,18 @@ __global__ void k_excluded_14(const SysDev* __restrict__ sys) {
         if (t < nsa + nex) {
             sl = group_slot(G, gi, gj);
             if (i < nsa) {
-                ec = to_fixed_d(q * (-s.crf_2cut3i * r2 - s.crf_cut), kEnergyScale);
+                ec = q * (-s.crf_2cut3i * r2 - s.crf_cut);
                 fs = q * s.crf_cut3i;
             } else {
-                ec = to_fixed_d(-qi * qj * s.fpe * s.crf_2cut3i * r2, kEnergyScale);
+                ec = -qi * qj * s.fpe * s.crf_2cut3i * r2;
             }
         } else if (!(r2 < 1e-10)) {
             sl = group_slot(G, gi, gj);
             const double* lj = s.lj64 + 4 * (s.iac[i] * s.n_types + s.iac[j]);
             const double cs6 = lj[2], cs12 = lj[3];
             const double ir2 = 1.0 / r2, ir6 = ir2 * ir2 * ir2, ir = sqrt(ir2);
-            el = to_fixed_d((cs12 * ir6 - cs6) * ir6, kEnergyScale);
-            ec = to_fixed_d(q * (ir - s.crf_2cut3i * r2 - s.crf_cut), kEnergyScale);
+            el = (cs12 * ir6 - cs6) * ir6;
+            ec = q * (ir - s.crf_2cut3i * r2 - s.crf_cut);
             fs = (12.0 * cs12 * ir6 - 6.0 * cs6) * ir6 * ir2 + q * (ir * ir2 + s.crf_cut3i);
         }
         if (fs != 0.0) {
@@ -630,11 +630,21 @@ __global__ void k_excluded_14(const SysDev* __restrict__ sys) {
             v6[5] = rz * fz;
         }
     }
-    warp_add_energies(sh, G, sl, el, ec);
+    unsigned left = __ballot_sync(0xffffffffu, sl >= 0);
+    while (left) {  // one round per group slot among the lanes
+        const int lead = __shfl_sync(0xffffffffu, sl, __ffs(left) - 1);
+        const bool mine = sl == lead;
+        const double l = warp_sum_d(mine ? el : 0.0), c = warp_sum_d(mine ? ec : 0.0);
+        if ((threadIdx.x & 31) == 0) {
+            shared_add(sh, lead, l);
+            shared_add(sh, G * G + lead, c);
+        }
+        left &= ~__ballot_sync(0xffffffffu, mine);
+    }
     if (__any_sync(0xffffffffu, t >= nsa && t < nterm)) {
 #pragma unroll
         for (int u = 0; u < 6; ++u) {
-            const long long v = warp_sum_ll(to_fixed_d(v6[u], kEnergyScale));
+            const long long v = to_fixed_d(warp_sum_d(v6[u]), kEnergyScale);
             if ((threadIdx.x & 31) == 0 && v) {
                 const int a = u < 3 ? 0 : u < 5 ? 1 : 2, b = u < 3 ? u : u < 5 ? u - 2 : 2;
                 atomicAdd(&sh[vb + 3 * a + b], static_cast<unsigned long long>(v));

@@ -4,8 +4,10 @@ import dataclasses
 import numpy as np
 import pytest
 
+import oracle_binding as ob
 from gromos_nb import generators
-from gromos_nb.system import csr_from_lists
+from gromos_nb.nonbonded import Forcefield
+from gromos_nb.system import NonbondedParams, System, Topology, csr_from_lists
 from test_gpu_parity import check_pairlist, compare_eval
 
 pytestmark = pytest.mark.gpu
@@ -46,3 +48,31 @@ def test_solute_lists_with_exclusions_between_groups(waters, solute, links, o14,
     s = linked_solute(waters, solute, 31 + waters, links, o14, hub, single=single)
     check_pairlist(s)
     compare_eval(s, steps=2, move=0.001)
+
+
+def test_excluded_terms_round_once_per_warp():
+    """125 copies of an eight-atom group out of each other's reach, two energy groups: only self and
+    excluded terms, whose sums in FP64 are taken to units of 2^-24 once per warp (and group pair)."""
+    n, size = 125, 8
+    rng = np.random.default_rng(5)
+    shape, q = rng.uniform(-0.2, 0.2, (size, 3)), rng.normal(0.0, 0.4, size)
+    at = np.stack(np.meshgrid(*[np.arange(5)] * 3, indexing="ij"), -1).reshape(-1, 1, 3) * 3.0 + 1.5
+    eo, ex = csr_from_lists([[b for b in range(a - a % size, a - a % size + size) if b != a]
+                             for a in range(n * size)], n * size)
+    topo = Topology(n_solute_atoms=n * size, n_solute_cg=n,
+                    cg_offsets=np.arange(0, n * size + 1, size), charge=np.tile(q, n),
+                    iac=np.zeros(n * size, dtype=int), lj=np.zeros((1, 1, 4)), excl_off=eo, excl=ex,
+                    o14_off=np.zeros(n * size + 1, dtype=int), o14=np.zeros(0, dtype=int),
+                    egroup=np.tile([0, 1], n * size // 2), n_egroups=2)
+    p = NonbondedParams(rcutp=1.0, rcutl=1.0, epsrf=61.0)
+    s = System(topo=topo, pos=(shape + at).reshape(-1, 3), box=np.full(3, 15.0), params=p)
+    ff = Forcefield(s)
+    got = ff.apply(s.pos)
+    ff.close()
+    want = ob.OracleForcefield(s).apply(s.pos)
+    warps = -(-n * (size + size * (size - 1) // 2) // 32)
+    half = 2.0 ** -25
+    assert np.abs(got["egroup_crf"] - want["egroup_crf"]).max() <= warps * half
+    assert np.abs(got["virial"] - want["virial"]).max() <= warps * half
+    # the terms of the copies are equal, so roundings of single terms add up: typically beyond this too
+    assert abs(got["e_crf"] - want["e_crf"]) <= 3.0 * half * np.sqrt(3.0 * warps)
