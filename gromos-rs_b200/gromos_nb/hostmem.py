@@ -54,10 +54,13 @@ class _Block:
         self._place, self._size = place, size
         self.__array_interface__ = {"data": (place[0], False), "shape": tuple(shape), "typestr": "<f8", "version": 3}
 
-    def __del__(self):
-        _returned.append((self._size, self._place, time.monotonic()))  # no lock: this may run inside any allocation
-        if not _open:
-            _give_back(0.0)
+    def __del__(self, returned=_returned, clock=time):
+        returned.append((self._size, self._place, clock.monotonic()))  # no lock: this may run inside any allocation
+        try:
+            if not _open:
+                _give_back(0.0)
+        except Exception:      # the interpreter exits: this module's names may be gone
+            pass
 
 
 def _drain() -> None:

@@ -1,5 +1,6 @@
 """CPU: the pool of page-locked result arrays, over a fake of the library's allocation calls."""
 import ctypes as C
+import sys
 import threading
 
 import numpy as np
@@ -129,3 +130,16 @@ def test_idle_memory_is_given_back(lib, monkeypatch):
     c[:] = 1.0
     del c                                      # and the rest with its array
     assert not lib.live and hostmem._held == 0
+
+
+def test_arrays_may_outlive_the_module(lib, monkeypatch):
+    """At the interpreter's exit a module's names are cleared while arrays still live: no message."""
+    said = []
+    monkeypatch.setattr(sys, "unraisablehook", lambda u: said.append(u.exc_value))
+    a = hostmem.empty((5000, 3), CTX)
+    names = [n for n in vars(hostmem) if not n.startswith("__")]
+    with monkeypatch.context() as m:
+        for n in names:
+            m.setattr(hostmem, n, None)
+        del a
+    assert not said
