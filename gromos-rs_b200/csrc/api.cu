@@ -1512,16 +1512,19 @@ gr_status NbSystem::launch_water(cudaStream_t s, const WaterParams& wp, bool lr)
         const long long need = (static_cast<long long>(h.max_clusters) + kWaterWarps - 1) / kWaterWarps;
         return unsigned(std::max<long long>(1, std::min<long long>(wave, need)));
     };
+#define GR_WATER_IT1(WW, LJ, LL, PK, IM)                                                                 \
+    do {                                                                                                 \
+        GR_CUDA(occupancy(k_water_force_it<WW, LJ, LL, PK, IM>, 128, smem, &occ));                       \
+        GR_CUDA(launch(k_water_force_it<WW, LJ, LL, PK, IM>, water_grid(sm * occ), 128, smem, s, d_sys, wp, ws)); \
+    } while (0)
 #define GR_WATER_IT(WW, LJ, LL)                                                                          \
     do {                                                                                                 \
         const size_t smem = water_it_smem<WW>();                                                         \
         int occ = 1;                                                                                     \
-        if (layout == 4) {                                                                               \
-            GR_CUDA(occupancy(k_water_force_it<WW, LJ, LL, true>, 128, smem, &occ));                     \
-            GR_CUDA(launch(k_water_force_it<WW, LJ, LL, true>, water_grid(sm * occ), 128, smem, s, d_sys, wp, ws)); \
+        if (LL && narrow) {                                                                              \
+            if (layout == 4) GR_WATER_IT1(WW, LJ, LL, true, LL); else GR_WATER_IT1(WW, LJ, LL, false, LL); \
         } else {                                                                                         \
-            GR_CUDA(occupancy(k_water_force_it<WW, LJ, LL, false>, 128, smem, &occ));                    \
-            GR_CUDA(launch(k_water_force_it<WW, LJ, LL, false>, water_grid(sm * occ), 128, smem, s, d_sys, wp, ws)); \
+            if (layout == 4) GR_WATER_IT1(WW, LJ, LL, true, false); else GR_WATER_IT1(WW, LJ, LL, false, false); \
         }                                                                                                \
     } while (0)
 #define GR_WATER_SHARED(LJ, LL)                                                                          \
@@ -1531,6 +1534,14 @@ gr_status NbSystem::launch_water(cudaStream_t s, const WaterParams& wp, bool lr)
         GR_CUDA(launch(k_water_force<LJ, LL>, water_grid(sm * occ), 128, 0, s, d_sys, wp));             \
     } while (0)
     const WaterScaled ws = water_scaled(wp);
+    // Long-range pairs near half a box edge: a first-atom vector reaches the cutoff
+    // at the last rebuild plus what the molecules moved since, and the kernel keeps
+    // twice a molecule's extent away from the edge, 0.2 nm.  Wider boxes than this
+    // take the kernel without the in-place images, whose code costs there too
+    // (30,000 waters, long-range kernel: 121.9 us with it, 117.7 without); a pair that is
+    // near an edge all the same is deferred.
+    const bool narrow = h.boundary == 1 &&
+                        std::min({h.box[0], h.box[1], h.box[2]}) * 0.5 < prm.rcutl + prm.skin + 0.3;
     if (layout == 3 && !lr) {
         const WaterScaled& pp = ws;
         const size_t smem = water_ps_smem();
@@ -1566,6 +1577,7 @@ gr_status NbSystem::launch_water(cudaStream_t s, const WaterParams& wp, bool lr)
         }
     }
 #undef GR_WATER_IT
+#undef GR_WATER_IT1
 #undef GR_WATER_SHARED
     if (layout == 1) {  // the bit-iterating kernel handles its deferred pairs itself
         if (lj00) {

@@ -949,7 +949,7 @@ __device__ __forceinline__ void packed_column_sums(const float4* __restrict__ fi
 // read from shared memory by bit index; i-forces accumulate in a lane-private
 // shared-memory row (no atomics, so the result does not depend on the order
 // of lanes) and the rows are summed once per cluster.
-template <int W, bool LJ00, bool LONG, bool PK>
+template <int W, bool LJ00, bool LONG, bool PK, bool IMAGED>
 __global__ void __launch_bounds__(128, 3)
     k_water_force_it(const SysDev* __restrict__ sys, const WaterParams wp, const WaterScaled pp) {
     pdl_wait();
@@ -1141,7 +1141,7 @@ __global__ void __launch_bounds__(128, 3)
                         r0y += shy;
                         r0z += shz;
                         if (!(fabsf(r0x) < limx && fabsf(r0y) < limy && fabsf(r0z) < limz)) {
-                            if (LONG && water_pair_imaged<LJ00>(sp + k * 3, jbuf[wid][jb] + 3 * lane, Dx, Dy, Dz,
+                            if (IMAGED && water_pair_imaged<LJ00>(sp + k * 3, jbuf[wid][jb] + 3 * lane, Dx, Dy, Dz,
                                                                 myrow + k * 3, gx, gy, gz, ecrf, elj, v0s, v1s, v2s,
                                                                 v3s, v4s, v5s, wp, pp)) {
                                 ++n_wp;
@@ -1372,20 +1372,28 @@ template __global__ void k_water_force<false, true>(const SysDev*, const WaterPa
 }  // namespace gnb
 
 namespace gnb {
-template __global__ void k_water_force_it<4, true, false, false>(const SysDev*, const WaterParams, const WaterScaled);
-template __global__ void k_water_force_it<4, true, true, false>(const SysDev*, const WaterParams, const WaterScaled);
-template __global__ void k_water_force_it<4, false, false, false>(const SysDev*, const WaterParams, const WaterScaled);
-template __global__ void k_water_force_it<4, false, true, false>(const SysDev*, const WaterParams, const WaterScaled);
-template __global__ void k_water_force_it<8, true, false, false>(const SysDev*, const WaterParams, const WaterScaled);
-template __global__ void k_water_force_it<8, true, true, false>(const SysDev*, const WaterParams, const WaterScaled);
-template __global__ void k_water_force_it<8, false, false, false>(const SysDev*, const WaterParams, const WaterScaled);
-template __global__ void k_water_force_it<8, false, true, false>(const SysDev*, const WaterParams, const WaterScaled);
-template __global__ void k_water_force_it<4, true, false, true>(const SysDev*, const WaterParams, const WaterScaled);
-template __global__ void k_water_force_it<4, true, true, true>(const SysDev*, const WaterParams, const WaterScaled);
-template __global__ void k_water_force_it<4, false, false, true>(const SysDev*, const WaterParams, const WaterScaled);
-template __global__ void k_water_force_it<4, false, true, true>(const SysDev*, const WaterParams, const WaterScaled);
-template __global__ void k_water_force_it<8, true, false, true>(const SysDev*, const WaterParams, const WaterScaled);
-template __global__ void k_water_force_it<8, true, true, true>(const SysDev*, const WaterParams, const WaterScaled);
-template __global__ void k_water_force_it<8, false, false, true>(const SysDev*, const WaterParams, const WaterScaled);
-template __global__ void k_water_force_it<8, false, true, true>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<4, true, false, false, false>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<4, true, true, false, false>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<4, true, true, false, true>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<4, false, false, false, false>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<4, false, true, false, false>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<4, false, true, false, true>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<8, true, false, false, false>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<8, true, true, false, false>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<8, true, true, false, true>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<8, false, false, false, false>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<8, false, true, false, false>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<8, false, true, false, true>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<4, true, false, true, false>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<4, true, true, true, false>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<4, true, true, true, true>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<4, false, false, true, false>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<4, false, true, true, false>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<4, false, true, true, true>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<8, true, false, true, false>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<8, true, true, true, false>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<8, true, true, true, true>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<8, false, false, true, false>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<8, false, true, true, false>(const SysDev*, const WaterParams, const WaterScaled);
+template __global__ void k_water_force_it<8, false, true, true, true>(const SysDev*, const WaterParams, const WaterScaled);
 }  // namespace gnb
