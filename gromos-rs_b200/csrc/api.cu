@@ -603,7 +603,7 @@ gr_status NbSystem::upload(const gr_topology* t) {
     if ((st = alloc(&h.f_out, size_t(N) * 3))) return st;
     if ((st = alloc(&h.e_out, size_t(acc_size(G))))) return st;
     if ((st = alloc(&h.err, 4))) return st;
-    if ((st = alloc(&h.n_deferred, 9))) return st;  // see SysDev
+    if ((st = alloc(&h.n_deferred, 8))) return st;  // see SysDev
     if ((st = alloc(&h.max_delta, 1))) return st;
     GR_CUDA(cudaMemset(h.err, 0, 4 * sizeof(int)));
     GR_CUDA(cudaMemset(h.f_long, 0, size_t(N) * 3 * sizeof(long long)));
@@ -959,6 +959,7 @@ gr_status NbSystem::check_errors(cudaStream_t s, bool* retry) {
     GR_CUDA(cudaMemcpyAsync(err, h.err, sizeof(err), cudaMemcpyDeviceToHost, s));
     GR_CUDA(cudaStreamSynchronize(s));
     *retry = false;
+    several_images = err[1] != 0;
     if (err[0] == 0) return GR_OK;
     GR_CUDA(cudaMemset(h.err, 0, 4 * sizeof(int)));
     if (err[0] & ERR_CELL_TOO_DENSE) {
@@ -989,6 +990,7 @@ gr_status NbSystem::resolve_pending(bool* overflowed) {
     if (!pending_check) return GR_OK;
     GR_CUDA(cudaEventSynchronize(ev_err));
     pending_check = false;
+    several_images = err_host[1] != 0;
     if (err_host[0] == 0) return GR_OK;
     const int e = err_host[0];
     GR_CUDA(cudaMemset(h.err, 0, 4 * sizeof(int)));
@@ -1044,7 +1046,13 @@ gr_status NbSystem::build_pairlist(cudaStream_t s, bool sync) {
                 P.wide[k] = 0.25f * h.boxf[k];
             }
             // members in different images: only a periodic system has them (k_water_search)
-            const bool filter = h.boundary == 1 && std::min({h.gdim[0], h.gdim[1], h.gdim[2]}) >= 3;
+            const bool images = h.boundary == 1 && std::min({h.gdim[0], h.gdim[1], h.gdim[2]}) >= 3;
+            // The search with the image filter where there are such clusters: a box that is
+            // not shifted against its molecules has none, and there the filter costs (build
+            // of 30,000 waters 154 us with it, 135 without).  Either form gives the same lists,
+            // so the last build's answer decides.  A batch's recorded steps outlive that
+            // answer: they hold both forms, one of which ends at once, or the filter.
+            const bool filter = images && (batch_capture || several_images);
             P.c2s = h.c2s;
             P.c2l = h.c2l;
             P.boundary = h.boundary;
@@ -1064,7 +1072,7 @@ gr_status NbSystem::build_pairlist(cudaStream_t s, bool sync) {
     } while (0)
             if (layout == 1) {
                 if (filter) GR_WATER_SEARCH(4, false, true); else GR_WATER_SEARCH(4, false, false);
-            } else if (W == 4 && !(in_capture && crowded) && h.max_clusters <= kBlockClusters) {
+            } else if (W == 4 && !(batch_capture && crowded) && h.max_clusters <= kBlockClusters) {
                 int occ = 1;
                 if (filter) {
                     GR_CUDA(occupancy(k_water_search_block<true>, kSearchWarps * 32, 0, &occ));
@@ -1076,12 +1084,8 @@ gr_status NbSystem::build_pairlist(cudaStream_t s, bool sync) {
                                    0, s, d_sys, P));
                 }
             } else if (W == 4) {
-                // both forms, one of which ends at once: whether a cluster is wide is known
-                // on the device only, and where none is, as in a box that is not shifted,
-                // the filter costs (build of 30,000 waters 154 us with it, 135 this way;
-                // both bodies in one kernel 142, and 1% of a shifted box's steps lost)
-                P.by_width = filter;
-                GR_WATER_SEARCH(4, true, false);
+                P.by_width = batch_capture && filter;
+                if (!filter || P.by_width) GR_WATER_SEARCH(4, true, false);
                 if (filter) GR_WATER_SEARCH(4, true, true);
             } else {
                 if (filter) GR_WATER_SEARCH(8, true, true); else GR_WATER_SEARCH(8, true, false);
@@ -1183,7 +1187,7 @@ gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events, bool fin
     // members of a batch leave room: a boundary between two small kernels costs its
     // drain and launch latency otherwise (MD step of 1,000 waters 57 -> 50 us), and the
     // solute kernels run beside the water kernels.
-    pdl = prm.kernel == GR_KERNEL_FIXED && !record_events && !(in_capture && crowded);
+    pdl = prm.kernel == GR_KERNEL_FIXED && !record_events && !(batch_capture && crowded);
     if (pdl && NCG > NSCG && NSA + h.n_ex_pairs + h.n_14_pairs > 0 && !in_capture) GR_CUDA(ensure_side());
     if (stage) last_staged = true;
     if (stage) {
@@ -1359,6 +1363,7 @@ gr_status NbSystem::eval_graph(cudaStream_t s, int flags) {
     bool overflowed = false;
     if ((st = resolve_pending(&overflowed))) return st;
     if (overflowed) lr_computed = false;
+    if (several_images && !g_several) g_gen = -1;  // recorded again, with the image filter
     const bool rebuild = !built || steps_since_update >= prm.nsnb || (flags & GR_EVAL_FORCE_REBUILD);
     const bool do_long = h.twin && (rebuild || !lr_computed);
     if (!ever_built || !warm || prm.kernel != GR_KERNEL_FIXED || (!rebuild && do_long)) {
@@ -1383,7 +1388,7 @@ gr_status NbSystem::eval_graph(cudaStream_t s, int flags) {
         const bool built0 = built, lr0 = lr_computed;
         const long long l0 = launches;
         in_capture = true;
-        crowded = false;
+        g_several = several_images;
         for (int v = 0; v < 2 && !st; ++v) {
             steps_since_update = v ? prm.nsnb : 1;
             built = true;

@@ -157,7 +157,7 @@ gr_status batch_capture_graphs(gr_batch* b) {
     long long clusters = 0;
     for (auto& mb : b->m) clusters += mb.ctx->sys.h.max_clusters;
     for (auto& mb : b->m) {
-        mb.ctx->sys.in_capture = true;
+        mb.ctx->sys.in_capture = mb.ctx->sys.batch_capture = true;
         mb.ctx->sys.crowded = clusters > 16LL * mb.ctx->sys.sm_count();
     }
     std::vector<long long> launches0(n);  // recording is not launching: restored below
@@ -217,7 +217,7 @@ gr_status batch_capture_graphs(gr_batch* b) {
         b->g_launches[p] = l1 - l0 + 1;  // + the flag gather
         if (st || e != cudaSuccess) {
             for (int i = 0; i < n; ++i) b->m[i].ctx->sys.launches = launches0[i];
-            for (auto& mb : b->m) mb.ctx->sys.in_capture = false;
+            for (auto& mb : b->m) mb.ctx->sys.in_capture = mb.ctx->sys.batch_capture = false;
             b->drop_graphs();
             if (!st) {
                 set_error(std::string("gr_batch: graph capture failed: ") + cudaGetErrorString(e));
@@ -229,7 +229,7 @@ gr_status batch_capture_graphs(gr_batch* b) {
     b->gens.resize(n);
     for (int i = 0; i < n; ++i) {
         NbSystem& S = b->m[i].ctx->sys;
-        S.in_capture = false;
+        S.in_capture = S.batch_capture = false;
         S.pending_check = false;
         S.launches = launches0[i];
         b->gens[i] = S.alloc_gen;

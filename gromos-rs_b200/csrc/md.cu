@@ -661,6 +661,7 @@ gr_status NbSystem::md_run(cudaStream_t s, int n_steps, gr_md_stats* out) {
                 GR_CUDA(cudaEventSynchronize(ev_md));
                 const int* e = reinterpret_cast<const int*>(md_err_host);
                 pending_check = false;  // a rebuild at the block's last step: its flags are in e[0] too
+                several_images = e[1] != 0;
                 if (e[0]) {
                     const int f = e[0];
                     GR_CUDA(cudaMemset(h.err, 0, 4 * sizeof(int)));

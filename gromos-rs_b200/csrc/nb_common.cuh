@@ -152,7 +152,7 @@ struct SysDev {
     long long* fs_short;       // [max_clusters*W*9] water forces per slot (fixed 2^32)
     long long* fs_long;        // same, long-range cache
     int* deferred;             // [2 * 2 * defer_cap] (i slot, j slot): short, then long
-    int* n_deferred;           // [9]: deferred pairs, water-kernel work counters, finished blocks (short, long each), search counters [2], wide clusters
+    int* n_deferred;           // [8]: deferred pairs, water-kernel work counters, finished blocks (short, long each), search counters [2]
     float* max_delta;          // [1] largest |offset| component of a water atom from its first atom (this step)
     int defer_cap;
     // ---- plain-kernel data
@@ -172,7 +172,7 @@ struct SysDev {
     long long* acc_long;       // same layout (long-range cache)
     double* f_out;             // n_atoms*3 final forces
     double* e_out;             // [2*G*G + 9 + 1] final energies/virial/dhdl
-    int* err;                  // [4] error flags, counters
+    int* err;                  // [4] error flags; the last build found a cluster in several images (box_wide)
 };
 
 // The MD state that a pairlist build copies aside for a rollback (null pos: none).

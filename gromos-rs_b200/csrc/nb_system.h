@@ -149,7 +149,10 @@ class NbSystem {
     bool forked = false;      // side work that `join` has not yet ordered before the main stream
     bool side_waits = false, main_waits = false;  // the stream's next kernel follows an event of the other stream
     bool in_capture = false;  // recording a CUDA graph: the device descriptor is already current
-    bool crowded = false;     // ... a batch's, whose members fill the chip between them
+    bool batch_capture = false;  // ... a batch's
+    bool crowded = false;     // ... whose members fill the chip between them
+    bool several_images = false;  // the last build read back had a cluster with members in several periodic images
+    bool g_several = false;       // ... and so the recorded evaluation graphs search with the image filter
     bool last_staged = false; // the last timed evaluation recorded its stage events (kernel by kernel)
     bool prep_in_acc = false; // the accumulators hold the energies of water records written by the last MD step
     bool prepped_next = false; // the last MD step wrote this evaluation's water records (k_water_prep skipped)

@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(256) k_cell_sort(const SysDev* __restrict__ sy
         if (threadIdx.x == 0) {
             s.n_deferred[6] = 0;  // the water search's cluster counter
             s.n_deferred[7] = 0;  // the candidate lists' allocation counter
-            s.n_deferred[8] = 0;  // set by k_cluster_setup when a cluster is wide
+            s.err[1] = 0;         // set by k_cluster_setup when a cluster is wide
             if (total > s.max_clusters) {
                 atomicOr(&s.err[0], ERR_WLIST_OVERFLOW);
                 total = s.max_clusters;
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(256) k_cluster_setup(const SysDev* __restrict_
                                              float(0.5 * (hz - lz)) * (1.f + 1e-6f) + 1e-6f, 0.f);
                 s.clus_ext[k] = e;
                 if (e.x > 0.25f * s.boxf[0] || e.y > 0.25f * s.boxf[1] || e.z > 0.25f * s.boxf[2])
-                    s.n_deferred[8] = 1;  // (box_wide; any thread's store will do)
+                    s.err[1] = 1;  // (box_wide; any thread's store will do)
                 s.clus_tgeo[k] = make_float4(float(x0 + 0.5 * (double(tl.x) + double(th.x))),
                                              float(y0 + 0.5 * (double(tl.y) + double(th.y))),
                                              float(z0 + 0.5 * (double(tl.z) + double(th.z))), 0.f);
@@ -817,7 +817,7 @@ __global__ void __launch_bounds__(kSearchWarps * 32, W == 4 ? 8 : 4) k_water_sea
     pdl_wait();
     pdl_trigger();
     const SysDev& s = sys[blockIdx.y];
-    if (P.by_width && (s.n_deferred[8] != 0) != FILTER) return;  // the other form's turn
+    if (P.by_width && (s.err[1] != 0) != FILTER) return;  // the other form's turn
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     __shared__ uint32_t ebuf_s[kSearchWarps][kEntBuf], ebuf_l[kSearchWarps][kEntBuf];
     __shared__ int q_jc[kSearchWarps][64];          // surviving j-clusters, candidate order

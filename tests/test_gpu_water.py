@@ -50,3 +50,25 @@ def test_search_by_blocks(waters, rcutp, rcutl):
     check_pairlist(s)
     if waters > 100:  # a handful of waters lie outside each other's cutoff: no forces to compare
         compare_eval(s, steps=2, move=0.001)
+
+
+# the search's form follows what the build before found: systems below and above 1,472 clusters, width 8,
+# layout 1
+@pytest.mark.parametrize("waters,layout,width", [(3000, 0, 0), (6500, 0, 0), (6500, 0, 8), (3000, 1, 0)])
+def test_search_after_builds_with_and_without_several_images(waters, layout, width):
+    s = generators.spc_water_system(waters, generators.box_for_waters(waters), 7, rcutp=0.8, rcutl=1.2)
+    shifted = s.pos + np.array([0.37, -0.21, 0.5]) * s.box[0]
+    ff = Forcefield(s, water_layout=layout, cluster_size=width)
+    ref = [ob.pairlist(System(s.topo, x, s.box, s.params), algorithm=2) for x in (s.pos, shifted)]
+    for k in (0, 1, 1, 0, 0):
+        ff.upload_positions((s.pos, shifted)[k])
+        ff.build_pairlist()
+        for got, want in zip(ff.pairlist_lists(), ref[k]):
+            assert np.array_equal(sorted_pairs(got), sorted_pairs(want))
+    # recorded steps, before and after the first clusters in several images
+    graph = Forcefield(s, water_layout=layout, cluster_size=width)
+    for x in (s.pos, s.pos, s.pos, shifted, shifted, s.pos, shifted):
+        a, b = ff.apply(x, force_rebuild=True), graph.apply(x, force_rebuild=True, graph=True)
+        assert np.array_equal(a["forces"], b["forces"]) and a["e_crf"] == b["e_crf"]
+    ff.close()
+    graph.close()
