@@ -724,6 +724,8 @@ gr_status NbSystem::set_box(const double box[3]) {
         set_error("gr_set_box: rectangular box edges must be positive");
         return GR_ERR_INVALID;
     }
+    // recorded steps hold the box (kernel parameters, grid of the cell kernels): they are stale
+    if (box_set && (box[0] != h.box[0] || box[1] != h.box[1] || box[2] != h.box[2])) ++alloc_gen;
     for (int k = 0; k < 3; ++k) {
         h.box[k] = box[k];
         h.inv_box[k] = prm.boundary == 1 ? 1.0 / box[k] : 0.0;

@@ -406,3 +406,37 @@ def test_null_output_arguments_are_rejected():
     r = ff.apply(s.pos)                          # the context is still usable
     assert np.isfinite(r["e_lj"])
     ff.close()
+
+
+@pytest.mark.parametrize("waters", [900, 1100])  # the new box has more cells; as many
+def test_recorded_steps_follow_a_new_box(waters):
+    """A box set after steps were recorded (evaluation graphs, a batch's steps) is the box of the next ones."""
+    from gromos_nb.nonbonded import Batch
+
+    s = generators.spc_water_system(waters, generators.box_for_waters(waters), 23, rcutp=0.8, rcutl=1.0)
+    box = s.box * np.array([1.01, 1.0, 1.02])
+    plain, graph = Forcefield(s), Forcefield(s)
+    for _ in range(4):
+        graph.apply(s.pos, graph=True)
+    plain.set_box(box)
+    graph.set_box(box)
+    want, got = plain.apply(s.pos), graph.apply(s.pos, force_rebuild=True, graph=True)
+    assert np.array_equal(got["forces"], want["forces"]) and got["e_crf"] == want["e_crf"]
+    state = []
+    m = generators.masses(s)
+    for batch in (False, True):
+        ff, b = Forcefield(s), Batch()
+        ff.upload_positions(s.pos)
+        ff.md_init(m, generators.maxwell_velocities(m, 300.0, 4), dist_hh=generators.SPC_DHH)
+        if batch:
+            b.add(ff)
+        run = b.md_run if batch else ff.md_run
+        run(5)
+        ff.set_box(box)
+        run(5)
+        state.append(ff.md_state())
+        b.close()
+        ff.close()
+    assert np.array_equal(state[0][0], state[1][0]) and np.array_equal(state[0][1], state[1][1])
+    plain.close()
+    graph.close()
