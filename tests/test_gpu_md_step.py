@@ -95,7 +95,10 @@ def test_records_written_ahead_are_those_of_the_members_last_own_step():
 def test_tiled_step_of_a_large_system():
     """More than 128 units per SM take the tiled step kernel: a last tile that is not full, solute atoms
     before the molecules, steps inside a pairlist period and across its end."""
-    s = generators.solvated_solute_system(19411, 7, seed=14, single_atom_cgs=True)
+    import torch
+
+    waters = 128 * torch.cuda.get_device_properties(0).multi_processor_count + 467
+    s = generators.solvated_solute_system(waters, 7, seed=14, single_atom_cgs=True)
     s.params.rcutp, s.params.rcutl = 0.8, 1.0
     m = generators.masses(s)
     v = generators.maxwell_velocities(m, 300.0, 3)

@@ -76,3 +76,27 @@ def test_excluded_terms_round_once_per_warp():
     assert np.abs(got["virial"] - want["virial"]).max() <= warps * half
     # the terms of the copies are equal, so roundings of single terms add up: typically beyond this too
     assert abs(got["e_crf"] - want["e_crf"]) <= 3.0 * half * np.sqrt(3.0 * warps)
+
+
+# solvent molecules of two kinds: the solute's entries go atom by atom with the atoms' own charges and
+# types.  (Solvent pairs take the first molecule's parameters; the reference's topology knows one solvent
+# only.  Its solvent loop of the short range does the same, that of the long range does not, so a twin
+# range is compared on the solute's atoms.)
+@pytest.mark.parametrize("waters,solute,single,rcutp", [(700, 30, True, 0.8), (700, 30, False, 0.8),
+                                                        (600, 40, False, 1.2)])
+def test_solvent_of_two_kinds(waters, solute, single, rcutp):
+    s = generators.solvated_solute_system(waters, solute, seed=41, single_atom_cgs=single)
+    s.params.rcutp, s.params.rcutl = rcutp, 1.2
+    t = s.topo
+    charge, iac = t.charge.copy(), t.iac.copy()
+    odd = (t.n_solute_atoms + 3 * np.arange(1, waters, 2))[:, None] + np.arange(3)
+    charge[odd] *= 0.8
+    iac[odd[:, 0]] = iac[0]
+    s.topo = dataclasses.replace(t, charge=charge, iac=iac)
+    ff = Forcefield(s)
+    got, want = ff.apply(s.pos)["forces"], ob.OracleForcefield(s).apply(s.pos)["forces"]
+    ff.close()
+    n = t.n_solute_atoms
+    assert np.linalg.norm(got[:n] - want[:n]) <= 1e-5 * np.linalg.norm(want[:n])
+    if rcutp == s.params.rcutl:
+        compare_eval(s, steps=2, move=0.001)
