@@ -2241,9 +2241,12 @@ extern "C" gr_status gr_lj_crf_innerloop(const float* positions, const float* ch
         set_error(std::string("gr_lj_crf_innerloop: ") + cudaGetErrorString(e));
         st = GR_ERR_CUDA;
     };
+    // (the pool keeps what it is given back, so the block of a long list, whose copy takes
+    // far longer than an allocation, is one of its own)
+    const bool pooled = total <= (size_t(64) << 20);
     cudaMemPool_t pool = nullptr;
-    cudaError_t e = device_pool(&pool);
-    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&block), total, pool, 0);
+    cudaError_t e = pooled ? device_pool(&pool) : cudaMalloc(&block, total);
+    if (pooled && e == cudaSuccess) e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&block), total, pool, 0);
     if (e != cudaSuccess) {
         cudaGetLastError();
         fail(e);
@@ -2280,7 +2283,10 @@ extern "C" gr_status gr_lj_crf_innerloop(const float* positions, const float* ch
         }
     }
     cudaStreamSynchronize(0);  // also after an error: nothing may still read the caller's arrays
-    cudaFreeAsync(block, 0);
+    if (pooled)
+        cudaFreeAsync(block, 0);
+    else
+        cudaFree(block);
     return st;
 }
 

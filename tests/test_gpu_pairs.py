@@ -126,3 +126,20 @@ def test_pairs_half_an_edge_apart(edge):
     assert float(x[1, 0]) == 1.5 * float(edge)
     f, _, _, _ = loop_on_host(x, np.array([[0, 1]], dtype=np.uint32), 1e-6, np.array([float(edge)] * 3))
     assert f[0, 0] > 0.0 > f[1, 0]
+
+
+def test_long_lists_leave_no_device_memory_behind():
+    """The library's pool keeps blocks for the next call, those of long lists (more than 64 MB) excepted."""
+    import torch
+
+    x, q, iac, pairs, lj = inputs(60000, "sorted")
+    crf = CRFParameters.new(1.4, 1.0, 61.0, 0.0)
+    from gromos_nb.nonbonded import lj_crf_innerloop
+
+    once = lj_crf_innerloop(x, q, iac, pairs, lj, crf, BOX)
+    free = torch.cuda.mem_get_info()[0]
+    many = lj_crf_innerloop(x, q, iac, np.tile(pairs, (150, 1)), lj, crf, BOX)  # 72 MB
+    assert torch.cuda.mem_get_info()[0] >= free - (8 << 20)
+    # 60,000 and 9,000,000 FP32 additions to the largest sums
+    assert np.abs(many[0] - 150.0 * once[0]).max() <= 1e-3 * np.abs(many[0]).max()
+    assert many[1] == pytest.approx(150.0 * once[1], rel=1e-5)
