@@ -7,7 +7,15 @@ took 1.4 ms, of which the transfer is 0.1.  :func:`empty` returns arrays whose
 memory is page-locked and goes back to a pool when the array (and every view
 of it) is gone.  Live and pooled blocks together stay within
 :data:`LIMIT` bytes; beyond that, and for small arrays, it returns ordinary
-arrays.  Memory that no array uses is given back when it has been idle for
+arrays.
+
+Page-locking takes longer than a pageable download saves (3 to 10 ms for 8 MB),
+so it has to pay: blocks come in size classes of at most a quarter more than
+asked for, which arrays of uneven systems share, and beyond a class's first two
+blocks only as many are made as arrays of the class have been dropped.  A
+program that keeps its results gets ordinary arrays.
+
+Memory that no array uses is given back when it has been idle for
 :data:`IDLE_S` seconds (looked at on the next call here and when a context is
 closed), all of it when the process has no open context left, and whenever
 :func:`release` is called.  Safe with several threads: a block has one owner at
@@ -29,18 +37,20 @@ LIMIT = 512 << 20          # bytes of page-locked memory held at most, in use or
 SMALLEST = 8 << 10        # smaller arrays gain nothing
 
 IDLE_S = 10.0              # seconds that memory without an array is kept for the next one
-ARENA = 8 << 20            # blocks of one size are cut from arenas of about this many bytes
+ARENA = 8 << 20            # blocks of one size are cut from arenas of at most about this many bytes
 
 _lock = threading.Lock()
 _free: Dict[int, List[tuple]] = {}  # block size -> (address, arena)
+_blocks: Dict[int, int] = {}        # block size -> blocks in all its arenas
+_dropped: Dict[int, int] = {}       # block size -> ordinary arrays of it that are gone, less the blocks made since
 _held = 0                           # bytes of all arenas
 _open: set = set()                  # handles of the contexts that may want arrays
 _looked = 0.0                       # when idle arenas were last looked for
-_returned: deque = deque()          # (block size, (address, arena), when) of arrays that are gone
+_returned: deque = deque()          # (block size, (address, arena) or None, when) of arrays that are gone
 
 
 class _Arena:
-    """One page-locked allocation cut into blocks of one size."""
+    """One page-locked allocation of `size` bytes cut into blocks of one size."""
 
     def __init__(self, address: int, size: int, blocks: int):
         self.address, self.size, self.blocks, self.idle = address, size, blocks, 0
@@ -48,11 +58,16 @@ class _Arena:
 
 
 class _Block:
-    """One page-locked block, the base of the array over it."""
+    """One page-locked block, or the ordinary memory in its place: the base of the array over it."""
 
-    def __init__(self, place: tuple, size: int, shape):
+    def __init__(self, place, size: int, shape):
         self._place, self._size = place, size
-        self.__array_interface__ = {"data": (place[0], False), "shape": tuple(shape), "typestr": "<f8", "version": 3}
+        if place is None:
+            self._memory = np.empty(shape)
+            self.__array_interface__ = self._memory.__array_interface__
+        else:
+            self.__array_interface__ = {"data": (place[0], False), "shape": tuple(shape), "typestr": "<f8",
+                                        "version": 3}
 
     def __del__(self, returned=_returned, clock=time):
         returned.append((self._size, self._place, clock.monotonic()))  # no lock: this may run inside any allocation
@@ -66,6 +81,9 @@ class _Block:
 def _drain() -> None:
     while _returned:
         size, place, when = _returned.popleft()
+        if place is None:
+            _dropped[size] = _dropped.get(size, 0) + 1
+            continue
         _free.setdefault(size, []).append(place)
         place[1].idle += 1
         place[1].since = when
@@ -77,28 +95,41 @@ def _pop(size: int):
     return place
 
 
+def _class(n: int) -> int:
+    """The block size for n bytes: whole pages, four sizes to a power of two."""
+    pages = -(-n // 4096)
+    step = 1 << max(0, pages.bit_length() - 3)
+    return -(-pages // step) * step * 4096
+
+
 def _take(size: int, ctx):
-    """A block of `size` bytes, or None when the limit is reached.  A new arena is allocated on the
-    device of the context handle `ctx`."""
+    """A block of `size` bytes, or None where an ordinary array does as well or the limit is reached.
+    A new arena is allocated on the device of the context handle `ctx`."""
     global _held
-    n = max(1, min(ARENA // size, 64))
     if time.monotonic() - _looked > 0.1 * IDLE_S:
         _give_back(IDLE_S)
     with _lock:
         _drain()
         if _free.get(size):
             return _pop(size)
+        made = _blocks.get(size, 0)
+        if made and not _dropped.get(size, 0):
+            return None
+        n = max(1, min(ARENA // size, 64, max(2, made)))
         full = _held + n * size > LIMIT
     if full:
-        release()          # idle arenas of other sizes make room
+        _give_back(1.0)    # arenas that the current results do not need make room
     with _lock:
         if _held + n * size > LIMIT:
             return None
         _held += n * size
+        _blocks[size] = _blocks.get(size, 0) + n
+        _dropped[size] = max(0, _dropped.get(size, 0) - n)
     p = C.c_void_p()
     if _lib.lib().gr_ctx_host_alloc(ctx, n * size, C.byref(p)) != _lib.GR_OK:
         with _lock:
             _held -= n * size
+            _blocks[size] -= n
         return None
     arena = _Arena(int(p.value), n * size, n)
     with _lock:
@@ -110,12 +141,10 @@ def _take(size: int, ctx):
 def empty(shape, ctx) -> np.ndarray:
     """An uninitialised C-contiguous float64 array for a download from the context `ctx` to fill."""
     n = 8 * int(np.prod(shape))
-    if n >= SMALLEST:
-        size = -(-n // 4096) * 4096
-        place = _take(size, ctx)
-        if place is not None:
-            return np.asarray(_Block(place, size, shape))
-    return np.empty(shape)
+    if n < SMALLEST:
+        return np.empty(shape)
+    size = _class(n)
+    return np.asarray(_Block(_take(size, ctx), size, shape))
 
 
 def _idle(age: float) -> list:
@@ -128,7 +157,9 @@ def _idle(age: float) -> list:
     if idle:
         for size in list(_free):
             _free[size] = [p for p in _free[size] if p[1] not in idle]
-        _held -= sum(a.size for a in idle)
+        for a in idle:
+            _held -= a.size
+            _blocks[a.size // a.blocks] -= a.blocks
     return list(idle)
 
 

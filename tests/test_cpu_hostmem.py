@@ -15,9 +15,11 @@ CTX = object()  # a context's handle
 class FakeLib:
     def __init__(self):
         self.live = {}
+        self.calls = 0
 
     def gr_ctx_host_alloc(self, ctx, n, out):
         assert ctx is CTX         # never without the context whose device is meant
+        self.calls += 1
         buf = C.create_string_buffer(int(n))
         p = C.addressof(buf)
         self.live[p] = (buf, int(n))
@@ -37,10 +39,14 @@ def lib(monkeypatch):
     fake = FakeLib()
     monkeypatch.setattr(hostmem._lib, "lib", lambda: fake)
     hostmem._free.clear()
+    hostmem._blocks.clear()
+    hostmem._dropped.clear()
     hostmem._returned.clear()
     hostmem._held = 0
     yield fake
     hostmem._free.clear()
+    hostmem._blocks.clear()
+    hostmem._dropped.clear()
     hostmem._returned.clear()
     hostmem._held = 0
 
@@ -143,3 +149,36 @@ def test_arrays_may_outlive_the_module(lib, monkeypatch):
             m.setattr(hostmem, n, None)
         del a
     assert not said
+
+
+def test_kept_results_are_not_page_locked(lib):
+    """Memory is page-locked for arrays that come and go, not for a list of results that grows."""
+    hostmem.opened(1)
+    kept = [(hostmem.empty((90000, 3), CTX), hostmem.empty((90000, 3), CTX)) for _ in range(40)]
+    assert lib.calls == 1 and kept
+    del kept
+    for _ in range(40):
+        hostmem.empty((90000, 3), CTX), hostmem.empty((90000, 3), CTX)
+    assert lib.calls <= 2
+    hostmem.closed(1)
+
+
+def test_uneven_sizes_share_their_memory(lib):
+    """The results of 256 uneven systems, dropped after every pass: page-locked a few times, then reused."""
+    hostmem.opened(1)
+    sizes = [3 * n for n in range(500, 8180, 30)]
+    calls = []
+    for _ in range(8):
+        results = [hostmem.empty((n, 3), CTX) for n in sizes for _ in range(2)]
+        assert all(a.flags.c_contiguous and a.shape == (n, 3) for a, n in zip(results[::2], sizes))
+        del results
+        calls.append(lib.calls)
+    assert calls[-1] == calls[3] and calls[-1] < 128
+    assert lib.bytes() <= 2.5 * sum(2 * 24 * n for n in sizes)
+    hostmem.closed(1)
+
+
+def test_block_sizes():
+    for n in (8192, 8193, 24000, 36000, 131072, 131073, 2160000, 123456789):
+        assert n <= hostmem._class(n) <= max(1.25 * n, n + 4095) and hostmem._class(n) % 4096 == 0
+        assert hostmem._class(hostmem._class(n)) == hostmem._class(n)
