@@ -901,10 +901,12 @@ cudaError_t NbSystem::launch(void (*kernel)(P...), dim3 grid, unsigned threads, 
 // launched back to back (pdl) they run beside these: fork() orders the side
 // stream after everything enqueued on s, join() orders s after the side stream.
 // A MD step of 3,000 waters with 200 ions takes 66 us this way, 81 one kernel
-// after the other; 16 frames of 3,000 waters 3.2 and 4.1 ms.  Not in the recorded
-// steps of a batch, whose members already run side by side: their graphs
-// would cost more to record and launch than the branches give (six served jobs
-// 19.4 ms with them, 18.1 without).
+// after the other; 16 frames of 3,000 waters 3.2 and 4.1 ms.  Not for the members of
+// a batch, which already run side by side: recorded steps would cost more to
+// record and launch than the branches give (six served jobs 19.4 ms with
+// them, 18.1 without), and a stream takes 0.1 ms to create.
+bool NbSystem::may_fork() const { return pdl && !in_capture && !batch_member && NCG > NSCG; }
+
 cudaError_t NbSystem::ensure_side() {
     if (side) return cudaSuccess;
     cudaError_t e = cudaSuccess;
@@ -1019,7 +1021,7 @@ gr_status NbSystem::build_pairlist(cudaStream_t s, bool sync) {
         return GR_ERR_STATE;
     }
     regrow_count = 0;
-    const bool beside = pdl && !in_capture && NCG > NSCG && NSCG > 0 && side;  // the solute search beside the water search
+    const bool beside = may_fork() && NSCG > 0 && side;  // the solute search beside the water search
     JoinAtEnd join_at_end{*this, s};
     if (relist) {  // list storage sized afresh from the requested capacity
         wcap_alloc = 0;
@@ -1190,7 +1192,7 @@ gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events, bool fin
     // drain and launch latency otherwise (MD step of 1,000 waters 57 -> 50 us), and the
     // solute kernels run beside the water kernels.
     pdl = prm.kernel == GR_KERNEL_FIXED && !record_events && !(batch_capture && crowded);
-    if (pdl && NCG > NSCG && NSA + h.n_ex_pairs + h.n_14_pairs > 0 && !in_capture) GR_CUDA(ensure_side());
+    if (may_fork() && NSA + h.n_ex_pairs + h.n_14_pairs > 0) GR_CUDA(ensure_side());
     if (stage) last_staged = true;
     if (stage) {
         evk_valid = prm.kernel == GR_KERNEL_FIXED && NCG > NSCG;
@@ -1236,7 +1238,7 @@ gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events, bool fin
     const size_t shg = size_t(2 * G * G) * sizeof(unsigned long long);
     const int nterm = NSA + h.n_ex_pairs + h.n_14_pairs;
     // solute kernels and FP64 terms beside the water kernels
-    const bool beside = pdl && !in_capture && NCG > NSCG && nterm > 0 && side;
+    const bool beside = may_fork() && nterm > 0 && side;
     const cudaStream_t ss = beside ? side : s;
     JoinAtEnd join_at_end{*this, s};
     auto clear_long = [&]() -> gr_status {

@@ -41,6 +41,7 @@ class NbSystem {
     gr_status energy_buffer();
     gr_status pair_counts(cudaStream_t s, long long* n_short, long long* n_long);
     gr_status push_descriptor(cudaStream_t s);
+    bool may_fork() const;
     cudaError_t ensure_side();
     cudaError_t fork(cudaStream_t s);
     cudaError_t join(cudaStream_t s);

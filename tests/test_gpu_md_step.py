@@ -145,24 +145,18 @@ def test_batch_steps_equal_standalone_steps(members, waters):
 @pytest.mark.parametrize("waters,solute,rcutp,kw", [(900, 30, 0.8, {"perturbed": True, "single_atom_cgs": True}),
                                                     (1200, 60, 0.8, {}), (900, 20, 1.0, {})])
 def test_solute_kernels_beside_the_water_kernels(waters, solute, rcutp, kw):
-    """Evaluations without timing events run the solute's kernels on a stream of their own: the same bits."""
+    """Steps without timing events run the solute's kernels on a stream of their own: the same bits."""
     s = generators.solvated_solute_system(waters, solute, seed=16, **kw)
     s.params.rcutp, s.params.rcutl, s.params.lam = rcutp, 1.0, 0.3
-    one, two, b = Forcefield(s), Forcefield(s), Batch()
-    two.upload_positions(s.pos)
-    b.add(two)
-    rng = np.random.default_rng(16)
-    for k in range(7):  # past the pairlist period
-        x = s.pos + rng.normal(0.0, 0.002, s.pos.shape)
-        want = one.apply(x)
-        if k == 0:  # the batch evaluates a new member once more, to size its lists
-            want = one.apply(x)
-        two.upload_positions(x)
-        b.eval()
-        got = two.result()
+    for steps in (0, 3, 5):  # the first step of a period, one inside, the first of the next
+        ff, ref = start(s), start(s)
+        ff.md_run(steps)
+        ref.md_run(steps)
+        want = ref.apply(ref.md_state()[0])
+        ff.md_run(1)
+        got = ff.result()
         assert np.array_equal(got["forces"], want["forces"]) and np.array_equal(got["virial"], want["virial"])
         for key in ("e_lj", "e_crf", "dhdl"):
             assert got[key] == want[key]
-    b.close()
-    one.close()
-    two.close()
+        ff.close()
+        ref.close()
