@@ -902,10 +902,11 @@ cudaError_t NbSystem::launch(void (*kernel)(P...), dim3 grid, unsigned threads, 
 // stream after everything enqueued on s, join() orders s after the side stream.
 // A MD step of 3,000 waters with 200 ions takes 66 us this way, 81 one kernel
 // after the other; 16 frames of 3,000 waters 3.2 and 4.1 ms.  Not for the members of
-// a batch, which already run side by side: recorded steps would cost more to
-// record and launch than the branches give (six served jobs 19.4 ms with
-// them, 18.1 without), and a stream takes 0.1 ms to create.
-bool NbSystem::may_fork() const { return pdl && !in_capture && !batch_member && NCG > NSCG; }
+// a batch, which already run side by side: branches in their recorded steps give
+// small batches 1.06-1.14x but cost more to record (six served jobs 17.9 ms
+// without them, 20.1 with; first passes 10-18% longer), and a stream takes 0.1 ms
+// to create.
+bool NbSystem::may_fork() const { return pdl && !batch_member && NCG > NSCG; }
 
 cudaError_t NbSystem::ensure_side() {
     if (side) return cudaSuccess;
@@ -1187,11 +1188,13 @@ gr_status NbSystem::eval(cudaStream_t s, int flags, bool record_events, bool fin
     // graph each event node adds its own latency to the step, so a graph holds
     // just the first and last (the step's total device time)
     const bool stage = record_events && !in_capture;
-    // Programmatic launches where nothing is recorded between the kernels and the
-    // members of a batch leave room: a boundary between two small kernels costs its
-    // drain and launch latency otherwise (MD step of 1,000 waters 57 -> 50 us), and the
-    // solute kernels run beside the water kernels.
-    pdl = prm.kernel == GR_KERNEL_FIXED && !record_events && !(batch_capture && crowded);
+    // Programmatic launches where no event is recorded between the kernels: a
+    // boundary between two small kernels costs its drain and launch latency otherwise
+    // (MD step of 1,000 waters 57 -> 50 us), and the solute kernels run beside the water
+    // kernels.  Not in the recorded steps of a batch: blocks that wait hold places that
+    // other members' kernels could use (10 steps of 3 x 1,351 waters 1,500 us
+    // without, 1,544 with; 8 x 1,500 waters lose 8%, 21 x 5,000 3%).
+    pdl = prm.kernel == GR_KERNEL_FIXED && !record_events && !in_capture;
     if (may_fork() && NSA + h.n_ex_pairs + h.n_14_pairs > 0) GR_CUDA(ensure_side());
     if (stage) last_staged = true;
     if (stage) {

@@ -148,12 +148,8 @@ gr_status batch_capture_graphs(gr_batch* b) {
     GR_CUDA(cudaMemcpy(b->d_errp, errp.data(), sizeof(int*) * n, cudaMemcpyHostToDevice));
     for (auto& mb : b->m) GR_CUDA(cudaStreamSynchronize(mb.ctx->stream));
     // Members that fill the chip between them (16 clusters per SM, about the warps that
-    // the water kernel keeps resident) take the water search with the least work and
-    // kernels that start when their predecessors have ended: blocks that wait hold
-    // places that other members' kernels could use (8 x 1,500 waters would lose 8% with
-    // programmatic launches, 21 x 5,000 3%).  Below that the shortest way from start to
-    // end counts: k_water_search_block and programmatic launches (10 steps of 3 x 1,351
-    // waters 1,432 -> 1,322 us, of 7 x 608 1,957 -> 1,907).
+    // the water kernel keeps resident) take the water search with the least work, others
+    // k_water_search_block, the shortest way from start to end.
     long long clusters = 0;
     for (auto& mb : b->m) clusters += mb.ctx->sys.h.max_clusters;
     for (auto& mb : b->m) {

@@ -569,7 +569,7 @@ __device__ __forceinline__ void shared_add(unsigned long long* sh, int idx, doub
 // 64-bit words that its whole block adds to took 28 us for 200 atoms in
 // multi-atom CGs and 11 us for 200 ions (ncu).  Here a warp sums its values by
 // shuffles, in FP64 and per group slot, and takes each sum to fixed point once:
-// one shared add and one rounding per warp, 7.2 and 4.6 us.
+// one shared add and one rounding per warp, 6.6 and 5.3 us.
 __global__ void k_excluded_14(const SysDev* __restrict__ sys) {
     pdl_wait();
     pdl_trigger();
@@ -1064,8 +1064,8 @@ namespace gnb {
 // components of a j-force are one 8-byte and one 4-byte reduction, whichever
 // way round the address allows.  Energies and the virial go to FP64 per warp
 // chunk and once per block to memory, where eleven FP64 atomics per warp went to
-// one cache line.  6.3 M pairs of 30,000 atoms: 622 us with one addition per pair
-// and component, 87 now (ncu).  The arithmetic hides behind the reductions:
+// one cache line.  6.3 M pairs of 30,000 atoms: 613 us with one addition per pair
+// and component, 83 now (ncu).  The arithmetic hides behind the reductions:
 // IEEE division and square root, which round once where a reciprocal square
 // root would give r^-6 2.3 times the rounding, cost nothing (92.5 us a call
 // either way), and the image is the reference's round(x / box).
