@@ -1068,7 +1068,7 @@ namespace gnb {
 // and component, 83 now (ncu).  The arithmetic hides behind the reductions:
 // IEEE division and square root, which round once where a reciprocal square
 // root would give r^-6 2.3 times the rounding, cost nothing (92.5 us a call
-// either way), and the image is the reference's round(x / box).
+// either way), and the image is the nearest integer to the quotient x / box itself.
 constexpr int kPairIters = 8;
 
 __device__ __forceinline__ void red_add3(float* p, float x, float y, float z) {
