@@ -117,15 +117,17 @@ def test_rounding_of_one_pair():
     assert rms(f[::2, 0]) <= 1.3 * rms(same) and rms(f[1::2, 0] * -1.0) <= 1.3 * rms(same)
 
 
-# edges for which 1.5 edges times the rounded reciprocal is below 1.5
-@pytest.mark.parametrize("edge", [3.38, 3.62, 3.83])
-def test_pairs_half_an_edge_apart(edge):
-    """The image is round(x / edge), ties to even: -1.5 edges become 0.5."""
+# 3.38, 3.62, 3.83: 1.5 edges times the rounded reciprocal is below 1.5
+@pytest.mark.parametrize("edge,apart,image", [(3.38, 1.5, -0.5), (3.62, 1.5, -0.5), (3.83, 1.5, -0.5), (3.25, 0.5, 0.5),
+                                              (3.25, 1.5, -0.5), (3.25, 2.5, 0.5), (2.9, 3.25, 0.25), (3.1, -1.75, 0.25)])
+def test_pairs_some_edges_apart(edge, apart, image):
+    """A component of `apart` edges is `image` edges: less the nearest whole number, ties to even."""
     edge = np.float32(edge)
-    x = np.array([[0.0, 0.1, 0.0], [np.float32(1.5) * edge, 0.4, 0.2]], dtype=np.float32)
-    assert float(x[1, 0]) == 1.5 * float(edge)
+    x = np.array([[np.float32(apart) * edge, 0.1, 0.0], [0.0, 0.4, 0.2]], dtype=np.float32)
+    assert float(x[0, 0]) == apart * float(edge) or abs(image) != 0.5
     f, _, _, _ = loop_on_host(x, np.array([[0, 1]], dtype=np.uint32), 1e-6, np.array([float(edge)] * 3))
-    assert f[0, 0] > 0.0 > f[1, 0]
+    d = np.array([image * float(edge), -0.3, -0.2])
+    assert np.allclose(f[0], 12e-6 * (d @ d) ** -7 * d, rtol=1e-5, atol=0.0) and np.array_equal(f[0], -f[1])
 
 
 def test_long_lists_leave_no_device_memory_behind():
