@@ -112,10 +112,10 @@ def _take(size: int, ctx):
         _drain()
         if _free.get(size):
             return _pop(size)
-        made = _blocks.get(size, 0)
-        if made and not _dropped.get(size, 0):
+        made, dropped = _blocks.get(size, 0), _dropped.get(size, 0)
+        if made and not dropped:
             return None
-        n = max(1, min(ARENA // size, 64, max(2, made)))
+        n = max(1, min(ARENA // size, 64, max(2, made, dropped)))  # few calls: each takes about a millisecond
         full = _held + n * size > LIMIT
     if full:
         _give_back(1.0)    # arenas that the current results do not need make room
